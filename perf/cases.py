@@ -196,11 +196,11 @@ def _kill_rates(kind, n, q2, d):
 
 @functools.lru_cache(maxsize=None)
 def _density(kind, n, q2, d):
-    """Of one unit of the line: positions the wheel of 2 ... 13 leaves, prime
-    tests past the first 32 pattern primes until one kills, survivors."""
+    """Of one unit of the line: positions a wheel of 2 ... 31 leaves, prime
+    tests past the first 38 primes until one kills, survivors."""
     q, r = _kill_rates(kind, n, q2, d)
     keep = np.cumprod(1.0 - r)
-    return keep[5], float(keep[37:].sum()), float(keep[-1])
+    return keep[10], float(keep[37:].sum()), float(keep[-1])
 
 
 def _spec(kind, n, q2, d, units, value_log10, depth):
