@@ -1,6 +1,6 @@
 // fk_classify.cuh -- base residues, chain classification and ordering.
 //
-// k_xq        X0 mod q for every (item, sieve prime): the per-launch
+// k_xq        X0 mod q, or its multiple, for every (item, sieve prime): the per-launch
 //             "(k_base mod q)" tables of the reference
 //             (euler-prime-runs/euler_gpu.py:1474-1477,
 //             primorial-ap/ap_gpu.py:586-593), computed on the device from
@@ -16,6 +16,7 @@
 //             host sort: counting scatter by item, then a bitonic sort of
 //             each item's segment.
 #pragma once
+#include "fk_sieve.cuh"
 #include "fk_sprp.cuh"
 #include "fk_types.h"
 
@@ -304,18 +305,15 @@ __global__ void k_dense(const DevItem* items, const u32* dense_idx,
   }
 }
 
-// X0 mod q for every (item, prime) of sieve items.
+// The base residues of every (item, prime) of sieve items.
 __global__ void k_xq(const DevEngine* engines, const DevItem* items,
                      const u32* sieve_idx, u32 nsieve, u32* xq) {
   for (u32 s = blockIdx.y; s < nsieve; s += gridDim.y) {
     const DevItem it = items[sieve_idx[s]];
     const DevEngine& e = engines[it.engine];
     for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < e.NP;
-         i += gridDim.x * blockDim.x) {
-      const PrimeRec pr = e.recs[i];
-      xq[it.xq_off + i] =
-          fk_bmod128(it.X0_lo, it.X0_hi, pr.q, pr.magic, e.c64[i]);
-    }
+         i += gridDim.x * blockDim.x)
+      xq[it.xq_off + i] = base_residue(e, it, i);
   }
 }
 

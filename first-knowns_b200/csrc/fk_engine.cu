@@ -274,6 +274,7 @@ static Cost engine_cost(const fk_engine* e, u32 NPm, u32 ns_sieve, u32 ns,
 // within it falls below `cut` (or after 4096 primes), so the ballot
 // compaction between rounds runs when about 1 - cut of the lanes have gone
 // idle; at most kMaxRounds rounds.
+static constexpr u32 kMaxWarpQueue = 513;  // above any queue: no rounds
 static constexpr double kDefaultRoundCut = 0.5;
 static std::vector<u32> compute_rounds(const fk_engine* e, double cut,
                                        u32 ns) {
@@ -439,45 +440,59 @@ static fk_status build_engine(fk_engine* e) {
       const u32 v = x * x + x;
       sbits[v >> 5] |= 1u << (v & 31);
     }
-    if (sbits.size() > 512)
+    if (sbits.size() > (size_t)kSbits)
       return set_err(FK_ERR_DOMAIN, "n too large for the Euler bitset test");
   }
   std::vector<PrimeRec> recs(NP);
-  std::vector<u32> c64(NP), lists;
-  std::vector<u64> hmask(NP, 0);
+  std::vector<TestRec> trec(NP);
+  std::vector<ListFilter> filt;
+  std::vector<u32> c64(NP), lists, boff, bits;
+  u32 ap_div = 0;
+  if (e->kind == KIND_AP)
+    for (u32 i = 0; i < NP; ++i) ap_div |= e->d % e->sieve[i] == 0;
+  if (e->kind == KIND_DICKSON || ap_div) filt.resize(NP);
   for (u32 i = 0; i < NP; ++i) {
     const u32 q = e->sieve[i];
     PrimeRec r;
     r.q = q;
+    r.pad = 0;
     r.magic = (u64)(((u128)1 << 64) / q);
-    r.aux = 0;
+    recs[i] = r;
     c64[i] = (u32)(((u128)1 << 64) % q);
-    const auto& f = e->forb[i];
-    bool use_list = false;
-    if (e->kind == KIND_DICKSON) use_list = true;
-    if (e->kind == KIND_EULER && q <= xxmax) use_list = true;
+    u64 a = 1;
+    if (e->kind == KIND_EULER) a = q - 1;
     if (e->kind == KIND_AP) {
       const u64 dq = (u64)(e->d % q);
-      r.aux = dq ? (u32)invmod(dq, q) : 0;
+      a = q - (dq ? invmod(dq, q) : 1);
+      if (!dq) filt[i].f0 = 1;
     }
-    if (use_list && i >= (u32)kNSMin) {
-      std::vector<u32> lf = f;
-      if (e->kind == KIND_DICKSON) {
-        // the roots come in pairs x, q - x: keep min(x, q - x) and a 64-bit
-        // filter of the kept values mod 64
-        lf.clear();
-        for (u32 x : f) lf.push_back(std::min(x, q - x));
-        std::sort(lf.begin(), lf.end());
-        lf.erase(std::unique(lf.begin(), lf.end()), lf.end());
-        for (u32 h : lf) hmask[i] |= 1ull << (h & 63);
-      }
-      if (lf.size() > 127) return set_err(FK_ERR_DOMAIN, "forbidden list too long");
-      if (lists.size() >= (1u << 24)) return set_err(FK_ERR_DOMAIN, "lists too large");
-      r.aux = 0x80000000u | ((u32)lf.size() << 24) | (u32)lists.size();
-      lists.insert(lists.end(), lf.begin(), lf.end());
+    trec[i] = redc_rec(q, a);
+    if (e->kind != KIND_DICKSON || i < (u32)kNSMin) continue;
+    // the roots come in pairs x, q - x: the smaller is listed
+    std::vector<u32> lf;
+    for (u32 f : e->forb[i]) lf.push_back(std::min(f, q - f));
+    std::sort(lf.begin(), lf.end());
+    lf.erase(std::unique(lf.begin(), lf.end()), lf.end());
+    if (lf.size() > 127) return set_err(FK_ERR_DOMAIN, "forbidden list too long");
+    if (lists.size() >= (1u << 24)) return set_err(FK_ERR_DOMAIN, "lists too large");
+    if (i < (u32)(kNSMax + kStaged)) {
+      boff.push_back((u32)bits.size());
+      bits.resize(bits.size() + q / 64 + 1, 0);
+      for (u32 h : lf) bits[boff.back() + (h >> 5)] |= 1u << (h & 31);
     }
-    recs[i] = r;
+    for (u32 h : lf) {
+      filt[i].f0 |= 1u << (h & 31);
+      filt[i].f1 |= 1u << ((h >> 5) & 31);
+      filt[i].f2 |= 1u << ((h >> 10) & 31);
+    }
+    lf.resize((lf.size() + 3) / 4 * 4, 0xFFFFFFFFu);
+    filt[i].list = ((u32)(lf.size() / 4) << 24) | (u32)(lists.size() / 4);
+    lists.insert(lists.end(), lf.begin(), lf.end());
   }
+  boff.push_back((u32)bits.size());
+  for (size_t i = 0; i + 1 < boff.size(); ++i)
+    if (boff[std::min(i + kStaged, boff.size() - 1)] - boff[i] > (u32)kStagedBits)
+      return set_err(FK_ERR_DOMAIN, "staged bitmaps too large");
   for (u32 i = kNSMax; i < NP; ++i)
     e->survival *= 1.0 - (double)e->forb[i].size() / e->sieve[i];
   // ---- compaction rounds: a round ends when survival within it halves ----
@@ -555,7 +570,18 @@ static fk_status build_engine(fk_engine* e) {
   if ((st = upload(e, recs, &d.recs))) return st;
   if ((st = upload(e, c64, &d.c64))) return st;
   if ((st = upload(e, lists, &d.lists))) return st;
-  if ((st = upload(e, hmask, &d.hmask))) return st;
+  d.ap_div = ap_div;
+  d.deep = 0;
+  for (;; ++d.deep) {
+    double left = 1.0;
+    for (u32 i = d.deep; i < std::min(d.deep + 128, NP); ++i)
+      left *= 1.0 - (double)e->forb[i].size() / e->sieve[i];
+    if (left >= 0.75) break;
+  }
+  if ((st = upload(e, boff, &d.boff))) return st;
+  if ((st = upload(e, bits, &d.bits))) return st;
+  if ((st = upload(e, trec, &d.trec))) return st;
+  if ((st = upload(e, filt, &d.filt))) return st;
   if ((st = upload(e, rounds, &d.rounds))) return st;
   if ((st = upload(e, sbits, &d.sbits))) return st;
   d.NPm = NPm;
@@ -904,8 +930,14 @@ static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
         di.Tc = (u32)tc;
         di.nchunk = (words + G * tc - 1) / (G * tc);
         const u64 chains = di.nchunk * L;      // one per group
-        const u64 per_task = (u64)b->tune.warp_tasks * (32 / G);
-        di.ntask = (chains + per_task - 1) / per_task;
+        const u64 blocks = (chains + 32 / G - 1) / (32 / G);
+        // blocks per CTA task: as many as leave every CTA about 16 tasks
+        // (the last ones' imbalance), at most kMaxTaskBlocks
+        const u64 ctas = (u64)b->nsm * b->tune.sieve_ctas_per_sm;
+        di.blocks = (u32)std::min<u64>(
+            std::max<u64>(blocks / (ctas * 16), b->tune.warp_tasks),
+            kMaxTaskBlocks);
+        di.ntask = (blocks + di.blocks - 1) / di.blocks;
       }
       Family& f = b->fam[fam_of(e->P0, mark)];
       di.task0 = f.prefix.back();
@@ -1026,7 +1058,6 @@ static fk_status enqueue(fk_batch* b, bool capturing = false) {
     a.task_ctr = b->d_task_ctr.p + f;
     a.warp_queue = b->tune.warp_queue;
     a.seg_per_task = b->tune.seg_per_task;
-    a.warp_tasks = b->tune.warp_tasks;
     const u64 grid = std::min<u64>(
         a.ntask, (u64)b->nsm * (F.mark ? b->tune.mark_ctas_per_sm
                                        : b->tune.sieve_ctas_per_sm));
@@ -1482,7 +1513,7 @@ fk_status fk_batch_set_tuning(fk_batch* b, const fk_tuning* t) {
     return set_err(FK_ERR_DOMAIN, "tuning value out of range");
   if (n.sieve_ctas_per_sm > 3 || n.mark_ctas_per_sm > 3 ||
       n.chains_per_sm < 64 || n.chains_per_sm > 65536 ||
-      n.warp_queue > (u32)kWq + 1 || n.seg_per_task > 64 ||
+      n.warp_queue > kMaxWarpQueue || n.seg_per_task > 64 ||
       n.classify_ctas_per_sm > 32 || n.mark_limit > 65536 ||
       n.warp_lane_words < 32 || n.group_lane_words < 8 ||
       !(n.mark_bias < 1e6f))

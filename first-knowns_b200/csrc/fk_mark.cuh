@@ -40,7 +40,7 @@ struct MarkSmem {
   u32 lsh[kNSMax];                    // the lane's index shift per prime
   u32 warp[kBlock / 32];
   u32 minv[kNSMax];
-  u32 sbits[512];
+  u32 sbits[kSbits + 1];
   u64 task;
   u32 item;
   u32 eng;
@@ -79,15 +79,17 @@ struct PatSeg<P0, NS, NS, WPT> {
 
 template <int KIND>
 __device__ __forceinline__ bool tail_alive(u64 v, const DevEngine& e,
-                                           const u32* __restrict__ xq,
+                                           const u32* __restrict__ kq,
                                            const u32* s_sbits, u64& ntest) {
+  const TestCtx c{e.trec, e.filt, kq, e.lists, s_sbits,
+                  e.n, e.xxmax, e.sbits_words, e.ap_div};
+  const u32 vl = (u32)v & ((1u << kRedcSplit) - 1u);
+  const u32 vh = (u32)(v >> kRedcSplit);
   for (u32 i = e.NPm; i < e.NP; ++i) {
-    const PrimeRec pr = e.recs[i];
-    u32 rr = fk_bmod(v, pr.q, pr.magic) + __ldg(xq + i);
-    rr = min(rr, rr - pr.q);
     ++ntest;
-    const u64 hm = KIND == KIND_DICKSON ? __ldg(e.hmask + i) : 0ull;
-    if (kill_test<KIND>(pr, rr, e.lists, s_sbits, e.xxmax, e.n, hm))
+    Prime<KIND> p;
+    p.load(c, i);
+    if (p.kills(c, vl, vh))
       return false;
   }
   return true;
@@ -140,8 +142,8 @@ __global__ void __launch_bounds__(kBlock, 3) k_mark(SieveArgs a) {
       if (!stage_patterns<P0, NS>(spat, eg, &S.mbar, &S.status, phase, a.ctr))
         return;
       for (u32 i = tid; i < (u32)NS; i += kBlock) S.minv[i] = eg.pat_minv[i];
-      for (u32 i = tid; i < eg.sbits_words && i < 512; i += kBlock)
-        S.sbits[i] = eg.sbits[i];
+      for (u32 i = tid; i <= eg.sbits_words; i += kBlock)
+        S.sbits[i] = i < eg.sbits_words ? eg.sbits[i] : 0u;
       __syncthreads();
       if (tid == 0) S.eng = eidx;
     }

@@ -108,16 +108,14 @@ __global__ void k_na_init(unsigned char* s, DevEngine eng, DevItem item,
   }
 }
 
-// X0 mod q for every sieve prime of the call's item, into the array.
+// The base residues of the call's item (base_residue), into the array.
 __global__ void k_na_xq(unsigned char* s) {
   const DevItem* it = reinterpret_cast<const DevItem*>(s + kOffItem);
   const DevEngine* e = reinterpret_cast<const DevEngine*>(s + kOffEngine);
   u32* xq = reinterpret_cast<u32*>(s + kOffXq);
   for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < e->NP;
-       i += gridDim.x * blockDim.x) {
-    const PrimeRec pr = e->recs[i];
-    xq[i] = fk_bmod128(it->X0_lo, it->X0_hi, pr.q, pr.magic, e->c64[i]);
-  }
+       i += gridDim.x * blockDim.x)
+    xq[i] = base_residue(*e, *it, i);
 }
 
 // The call's outcome once the sieve is done: 0 the survivors fit, 1 too
@@ -339,6 +337,7 @@ extern "C" fk_status fk_sieve_noalloc(fk_engine* e, const uint64_t lo[2],
   it.ntask = ntask;
   it.xq_off = 0;
   it.marked = 0;
+  it.blocks = kBlock / 32;  // ntask above counts kBlock chains per task
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   k_na_init<<<1, kBlock, 0, s>>>(base, v.dev, it, ntask);
   k_na_xq<<<64, kBlock, 0, s>>>(base);
@@ -357,7 +356,6 @@ extern "C" fk_status fk_sieve_noalloc(fk_engine* e, const uint64_t lo[2],
   a.task_ctr = at<unsigned long long>(base, kOffTaskCtr);
   a.warp_queue = kWarpMode;
   a.seg_per_task = kSegPerTask;
-  a.warp_tasks = kBlock / 32;  // ntask above counts kBlock chains per task
   const u32 grid = (u32)(ntask < (u64)nsm * 2 ? ntask : (u64)nsm * 2);
   // the engine's own descriptor is the default variant: kNS pattern primes
   ce = launch_sieve(v.P0, kNS, grid, s, a);

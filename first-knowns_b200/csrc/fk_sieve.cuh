@@ -5,10 +5,10 @@
 // Tc 64-period words per thread: either one thread per lane on Tc
 // consecutive words, or -- for long lanes -- one warp per lane, thread t
 // on words t, t + 32, ... (so a warp's pattern loads are 32 consecutive
-// table entries).  A CTA runs 256 threads' chains (a TASK), and a
-// persistent grid pulls tasks from a device counter, so thousands of
-// items of uneven length run in one launch.  Inside a task the warps claim
-// blocks of 32 threads' chains (warp tasks) from a shared counter.
+// table entries).  32 threads' chains are a BLOCK; a CTA task is a run of
+// one item's blocks, pulled from a device counter by a persistent grid, so
+// thousands of items of uneven length run in one launch, and inside a task
+// the warps claim blocks from a shared counter.
 //
 // S1 (pattern sieve).  For the NS pattern primes starting at prime index
 // P0 (NS = 24, 32 or 40: a template variant chosen per batch) --
@@ -22,17 +22,24 @@
 // gather primorial-ap/ap_gpu.py:204-313), re-indexed so that one table per
 // prime serves every lane of every wheel.
 //
-// S2 (compaction rounds).  S1 survivors go to a per-WARP shared-memory
-// queue (ballot/prefix compaction inside the warp, so the word loop has no
-// block-wide barrier).  When it fills, the warp drains it through rounds
-// over the remaining primes: every live candidate is tested against a
-// round's primes (Barrett residue plus the engine's kill test), then the
-// survivors are compacted with ballots so the next round starts with every
-// lane busy; a short queue instead goes one candidate per warp, the lanes
-// splitting the primes -- the reference's stage 1b / stage 2 rounds
-// (euler-prime-runs/euler_gpu.py:523-709, dickson-ladders/ladder_gpu.py:
-// 349-407) without a host-visible queue.  Final survivors are appended to
-// a global candidate list with warp-aggregated atomics.
+// S2 (compaction rounds).  S1 survivors go through per-thread columns to a
+// per-WARP shared-memory queue (no block-wide barrier in the word loop).
+// When it fills, the warp drains it: over the first primes one candidate
+// per lane, the survivors compacted with ballots between rounds; then one
+// prime per lane, every candidate against 32 or 128 primes at once (the
+// reference's stage 1b / stage 2 rounds, euler-prime-runs/euler_gpu.py:
+// 523-709, dickson-ladders/ladder_gpu.py:349-407, without a host-visible
+// queue).  A test is one Montgomery reduction (fk_redc.h) and the engine's
+// kill test on the scaled residue.  Final survivors are appended to a
+// global candidate list with warp-aggregated atomics.
+//
+// What bounds it, and what this shape measured (B200, kernel ms against
+// the 64-bit Barrett tests with a queue drained at every block's end): the
+// kernel issues instructions, so the tests' length is what counts -- 10
+// to 20 warp instructions a test against 58 -- then the pattern loads'
+// shared-memory wavefronts.  256 mixed intervals 204 -> 119 ms, the Dickson
+// window of 2^38 j 12.7 -> 7.8, the Euler n = 17 windows of 5e14 and 2e16
+// 42.2 -> 32.2 and 795 -> 627, the 13# line's quarter 19.3 -> 15.5.
 #pragma once
 #include "fk_arith.cuh"
 #include "fk_types.h"
@@ -40,7 +47,7 @@
 namespace fk {
 
 constexpr u32 kWaitSpins = 1u << 20;
-constexpr int kRoundUnroll = 2;  // primes per trip of the compaction rounds
+constexpr u32 kRoundUnroll = 4;  // primes per trip of the compaction rounds
 
 __device__ __forceinline__ u32 smem_u32(const void* p) {
   return (u32)__cvta_generic_to_shared(p);
@@ -70,54 +77,96 @@ __device__ __forceinline__ u32 block_scan(u32 v, u32* s_warp, u32* total) {
   return base + x - v;
 }
 
+// The base of every (item, prime) of sieve items: X0 mod q for the primes
+// sieved by pattern or mark, X0 * c1 mod q for those tested per candidate
+// (the rounds' from their first cut, the marking sieve's past NPm).
+__device__ __forceinline__ u32 base_residue(const DevEngine& e,
+                                            const DevItem& it, u32 i) {
+  const PrimeRec pr = e.recs[i];
+  const u32 x = fk_bmod128(it.X0_lo, it.X0_hi, pr.q, pr.magic, e.c64[i]);
+  const u32 first = it.marked ? e.NPm : e.rounds[0];
+  return i < first ? x : fk_mulmod(x, e.trec[i].c1, pr.q, pr.magic);
+}
+
 // ---- per-candidate kill tests ------------------------------------------
-// aux bit 31 set: explicit list, offset in bits 0..23, count in 24..30.
-__device__ __forceinline__ bool list_kill(u32 aux, u32 r,
+// What the tests read besides the prime's record, gathered per item (in
+// shared memory for the rounds, from the descriptor for the marking tail).
+struct TestCtx {
+  const TestRec* trec;
+  const ListFilter* filt;
+  const u32* kq;        // this item's X0 * c1 mod q
+  const u32* lists;
+  const u32* sbits;     // Euler: bitset of {x^2 + x : x < n}
+  u32 n, xxmax, xxwords, ap_div;
+};
+
+// Is residue r on the prime's list?  The three filter bits settle nearly
+// every residue off it; the list itself (groups of four, padded with ~0) is
+// read only behind them.
+__device__ __forceinline__ bool list_kill(const ListFilter& f, u32 r,
                                           const u32* __restrict__ lists) {
-  const u32 off = aux & 0x00FFFFFFu, cnt = (aux >> 24) & 0x7Fu;
+  if (!((f.f0 >> (r & 31)) & (f.f1 >> ((r >> 5) & 31)) &
+        (f.f2 >> ((r >> 10) & 31)) & 1u))
+    return false;
+  const uint4* l = reinterpret_cast<const uint4*>(lists) + (f.list & 0xFFFFFFu);
+  const u32 cnt = f.list >> 24;
   bool k = false;
-  for (u32 c = 0; c < cnt; ++c) k |= (__ldg(lists + off + c) == r);
+  for (u32 c = 0; c < cnt; ++c) {
+    const uint4 x = __ldg(l + c);
+    k |= (x.x == r) | (x.y == r) | (x.z == r) | (x.w == r);
+  }
   return k;
 }
 
+// Does prime i kill a value of scaled residue r (Euler, AP)?
 template <int KIND>
-__device__ __forceinline__ bool kill_test(const PrimeRec& pr, u32 r,
-                                          const u32* __restrict__ lists,
-                                          const u32* s_sbits, u32 xxmax,
-                                          u32 n, u64 hm) {
-  if (KIND == KIND_DICKSON) {
-    // the forbidden residues come in pairs r, q - r: h = min(r, q - r)
-    // must be on the half list, which a 64-bit filter of h mod 64
-    // screens first
-    const u32 h = min(r, pr.q - r);
-    if (!((hm >> (h & 63)) & 1ull)) return false;
-    return list_kill(pr.aux, h, lists);
+__device__ __forceinline__ bool kill_test(const TestCtx& c, u32 i,
+                                          const TestRec& t, u32 r) {
+  bool kill;
+  if (KIND == KIND_AP) {
+    kill = r < c.n;
+    if (c.ap_div && kill && c.filt[i].f0) kill = r == 0;
+  } else {
+    // r = -x is killed when it is one of the x^2 + x: the bitset's last
+    // word (xxwords) is zero
+    kill = (c.sbits[min(r >> 5, c.xxwords)] >> (r & 31)) & 1u;
+    // the primes up to max(x^2 + x): so are r + q, r + 2q, ...
+    if (t.q <= c.xxmax)
+      for (u32 s = r + t.q; s <= c.xxmax; s += t.q)
+        kill |= (c.sbits[s >> 5] >> (s & 31)) & 1u;
   }
-  if (pr.aux & 0x80000000u) return list_kill(pr.aux, r, lists);
-  if (KIND == KIND_EULER) {
-    // q > max(x^2+x): r is killed iff q - r (mod q) is one of the x^2+x.
-    if (r == 0) return true;
-    const u32 t = pr.q - r;
-    return t <= xxmax && ((s_sbits[t >> 5] >> (t & 31)) & 1u);
-  } else if (KIND == KIND_AP) {
-    // killed iff r + j*d == 0 (mod q) for some j < n, i.e.
-    // j = (q - r) * d^-1 mod q is below n; aux = d^-1 (0 when q | d).
-    if (r == 0) return true;
-    if (pr.aux == 0) return false;
-    // for q < 2^16 the product (q - r) * d^-1 < q^2 fits 32 bits: a
-    // 32-bit Barrett with floor(2^32 / q); deeper primes take 64 bits
-    u32 t;
-    if (pr.q < 65536u) {
-      const u32 x = (pr.q - r) * pr.aux;
-      t = x - __umulhi(x, (u32)(pr.magic >> 32)) * pr.q;
-      t = min(t, t - pr.q);
-    } else {
-      t = fk_mulmod(pr.q - r, pr.aux, pr.q, pr.magic);
-    }
-    return t < n;
-  }
-  return false;  // Dickson primes always carry a list
+  return kill;
 }
+
+__device__ __forceinline__ TestRec load_rec(const TestRec* p) {
+  const uint4 x = __ldg(reinterpret_cast<const uint4*>(p));
+  return TestRec{x.x, x.y, x.z, x.w};
+}
+
+__device__ __forceinline__ ListFilter load_filt(const ListFilter* p) {
+  const uint4 x = __ldg(reinterpret_cast<const uint4*>(p));
+  return ListFilter{x.x, x.y, x.z, x.w};
+}
+
+// One prime's data in registers.
+template <int KIND>
+struct Prime {
+  TestRec t;
+  ListFilter f;   // Dickson only
+  u32 k, i;
+  __device__ __forceinline__ void load(const TestCtx& c, u32 p) {
+    i = p;
+    t = load_rec(c.trec + p);
+    k = __ldg(c.kq + p);
+    if (KIND == KIND_DICKSON) f = load_filt(c.filt + p);
+  }
+  __device__ __forceinline__ bool kills(const TestCtx& c, u32 vl,
+                                        u32 vh) const {
+    const u32 r = redc_residue(t, k, vl, vh);
+    if (KIND == KIND_DICKSON) return list_kill(f, min(r, t.q - r), c.lists);
+    return kill_test<KIND>(c, i, t, r);
+  }
+};
 
 // ---- S1 helpers, unrolled over the compile-time pattern primes ----------
 // k[I] is the lane's current TABLE INDEX for pattern prime I (entry k =
@@ -232,9 +281,6 @@ struct SieveArgs {
   u32 warp_queue;     // compaction: warp queues below this go one
                       // candidate per warp
   u32 seg_per_task;   // marking: segments per task
-  u32 warp_tasks;     // pattern sieve: warp tasks per CTA task (8, 16 or
-                      // 32); a warp task is one warp's 32 threads' chains
-  u32 pad2;
 };
 
 // The entry of the item holding task t: the last i with task_prefix[i] <=
@@ -255,24 +301,36 @@ __device__ __forceinline__ u32 task_item(const SieveArgs& a, u64 t, u32 from) {
   return lo;
 }
 
-// Per-warp candidate queues: kQcap / 8 entries per warp, two buffers.
-constexpr u32 kWq = kQcap / (kBlock / 32);
+// Per-warp candidate queues of line offsets v = u * M + R.  A queue
+// outlives its warp's blocks and tasks: it is drained when it is full and
+// when the CTA moves to another item.  In front of it every thread has a
+// column of kColSlots codes (word of the chain << 6 | bit): pushing a
+// pattern survivor there takes a store and no vote, and a warp's columns
+// are turned into offsets a row at a time, when one is full or the block
+// ends.
+constexpr u32 kWarps = kBlock / 32;
+constexpr u32 kWq = 384;
+constexpr u32 kColSlots = 16;
 
 struct SieveSmem {
-  u32 qa[kQcap];
-  u32 qb[kQcap];
-  u64 chain_R[kBlock];
-  u64 chain_w0[kBlock];   // the thread's first word; word j is w0 + j*stride
-  u32 stride;             // 1, or 32 when a warp sweeps one lane
-  u32 wnext;              // the CTA task's next warp task
-  u32 warp[kBlock / 32];
+  u64 queue[kWarps * kWq];
+  unsigned short col[kWarps * kColSlots * 32];
+  // the first kStaged test primes: every drain starts on these, and a
+  // shared load answers in a tenth of the time of one from L2
+  TestRec srec[kStaged];
+  u32 skq[kStaged];
+  u32 sboff[kStaged];     // Dickson: the prime's first word in sbit
+  u32 sbit[kStagedBits];  // bit h: min(r, q - r) = h is killed
+  TestCtx ctx;            // the current item's tests
+  const u32* rounds;
+  u32 NP, kind, deep;
+  u32 wnext[2];           // next warp block of the current / next CTA task
+  u64 task[2];
+  u32 item[2];
   u32 minv[kNSMax];
-  u32 sbits[512];
-  u64 task;
-  u32 item;
+  u32 sbits[kSbits + 1];
   u32 eng;
   u32 status;
-  u32 pad;
   unsigned long long mbar;
 };
 
@@ -283,154 +341,168 @@ __host__ __device__ constexpr u32 pat_bytes() {
   return ((fk_pat_prefix(P0, NS) + 1) / 2) * 16;
 }
 
-// A queued candidate: the chain (thread of the CTA), the word within the
-// chain and the bit within the word.
-__device__ __forceinline__ u64 cand_value(const SieveSmem& S, u32 code,
-                                          u64 M) {
-  const u32 t = code >> 22;
-  const u64 u = 64ull * (S.chain_w0[t] +
-                         (u64)((code >> 6) & 0xFFFFu) * S.stride) +
-                (code & 63u);
-  return u * M + S.chain_R[t];
-}
-
-__device__ __forceinline__ void emit_cand(const SieveArgs& a, u64 v,
-                                          u32 gitem, u64 p) {
-  if (p < a.cand_cap) {
-    a.cand_key[p] = v;
-    a.cand_item[p] = gitem;
-  } else {
-    atomicOr(&a.ctr->overflow, 1u);
+// A warp's n candidates against the primes [at, end), 32 at a time: each
+// lane holds one prime, every candidate is tested against all of them at
+// once and the survivors are compacted in place; the next 32 primes' loads
+// are in flight meanwhile.  Returns the survivors' count.
+template <int KIND>
+__device__ __forceinline__ u32 drain_groups(u64* Q, u32 n, const TestCtx& c,
+                                            u32 at, u32 end, u32& ntest) {
+  const u32 lane = threadIdx.x & 31;
+  if (n == 0 || at >= end) return n;
+  Prime<KIND> p, next;
+  p.load(c, min(at + lane, end - 1));  // past the end: the last prime again
+  for (;;) {
+    at += 32;
+    next.load(c, min(at + lane, end - 1));
+    u32 out = 0;
+    for (u32 idx = 0; idx < n; idx += 2) {
+      const bool two = idx + 1 < n;
+      const u64 v = Q[idx], w = Q[two ? idx + 1 : idx];
+      const u32 vl = (u32)v & ((1u << kRedcSplit) - 1u);
+      const u32 vh = (u32)(v >> kRedcSplit);
+      const u32 wl = (u32)w & ((1u << kRedcSplit) - 1u);
+      const u32 wh = (u32)(w >> kRedcSplit);
+      const bool kv = p.kills(c, vl, vh), kw = p.kills(c, wl, wh);
+      const bool dv = __any_sync(0xffffffffu, kv);
+      const bool dw = __any_sync(0xffffffffu, kw) || !two;
+      if (!dv) {
+        if (lane == 0) Q[out] = v;  // out <= idx: read already
+        ++out;
+      }
+      if (!dw) {
+        if (lane == 0) Q[out] = w;
+        ++out;
+      }
+    }
+    ntest += n;
+    __syncwarp();
+    n = out;
+    if (at >= end || n == 0) return n;
+    p = next;
   }
 }
 
-// Drain one warp's queue (n candidates in qin; qout is the second buffer):
-// rounds over the per-candidate primes with ballot compaction, a short
-// queue one candidate per warp over every remaining prime, then the
-// survivors appended to the global list.  Warp-synchronous: every lane of
-// the warp calls it with the same n.
+// Drain one warp's queue of n candidates in place.  Over the first primes
+// past the pattern (the staged ones, which kill most): rounds with one
+// candidate per lane, the survivors compacted by ballot after each.  Once
+// fewer than a.warp_queue are left, or the staged primes are done, the
+// candidates share the warp instead: each lane holds one prime and every
+// candidate is tested against the warp's 32 primes at once, so no lane
+// idles behind a dead candidate and the records of 32 primes are loaded
+// (one group ahead) once for all of them.  The survivors go to the global
+// list.  Warp-synchronous: every lane calls it with the same n.  Returns
+// the lane's prime tests.  Not inlined: the pattern loop around it keeps
+// its NS table indexes in registers and runs between drains.
 template <int KIND>
-__device__ void warp_drain(u32* qin, u32* qout, u32 n, const SieveSmem& S,
-                           const DevEngine& e, const DevItem& it, u32 gitem,
-                           const SieveArgs& a, u32 wq_short, u32& ntest) {
+__device__ __noinline__ u32 warp_drain(u64* Q, u32 n, const SieveSmem& S,
+                                       u32 gitem, u32 wq_short, u64* cand_key,
+                                       u32* cand_item, u64 cand_cap,
+                                       DevCounters* ctr) {
   const u32 lane = threadIdx.x & 31;
   const u32 lt = (1u << lane) - 1u;
-  const u32* __restrict__ xq = a.xq + it.xq_off;
-  const u64 M = e.M;
-  for (u32 r = 0; r < e.nrounds && n > 0; ++r) {
-    const u32 i0 = __ldg(e.rounds + r), i1 = __ldg(e.rounds + r + 1);
-    if (n < wq_short) {
-      // one candidate per warp, the lanes splitting the primes 32 at a
-      // time and voting after each group (the reference's warp-per-
-      // candidate deep rounds, dickson-ladders/ladder_gpu.py:378-407)
-      for (u32 idx = 0; idx < n; ++idx) {
-        const u64 v = cand_value(S, qin[idx], M);
-        bool dead = false;
-        for (u32 b = i0; b < e.NP && !dead; b += 32) {
-          const u32 i = b + lane;
-          bool kill = false;
-          if (i < e.NP) {
-            const PrimeRec pr = e.recs[i];
-            u32 rr = fk_bmod(v, pr.q, pr.magic) + __ldg(xq + i);
-            rr = min(rr, rr - pr.q);
-            const u64 hm = KIND == KIND_DICKSON ? __ldg(e.hmask + i) : 0ull;
-            kill = kill_test<KIND>(pr, rr, e.lists, S.sbits, e.xxmax, e.n, hm);
-            ++ntest;
-          }
-          dead = __any_sync(0xffffffffu, kill);
-        }
-        if (!dead && lane == 0)
-          emit_cand(a, v, gitem, atomicAdd(&a.ctr->ncand, 1ull));
-      }
-      __syncwarp();
-      return;
-    }
+  const TestCtx c = S.ctx;
+  const u32 NP = S.NP, first = __ldg(S.rounds);
+  const u32 nstaged = min(kStaged, NP - first);
+  u32 ntest = 0, at = 0;
+  for (u32 r = 0; n >= wq_short && n > 0 && at < nstaged; ++r) {
+    // a round's cut, rounded up to whole trips (testing past it is no
+    // mistake, and past the last prime the tables repeat it)
+    const u32 i0 = at;
+    at = min((__ldg(S.rounds + r + 1) - first + kRoundUnroll - 1) /
+                 kRoundUnroll * kRoundUnroll, (u32)kStaged);
     u32 out = 0;
     for (u32 base = 0; base < n; base += 32) {
       const u32 idx = base + lane;
-      bool alive = false;
-      u32 code = 0;
-      if (idx < n) {
-        code = qin[idx];
-        const u64 v = cand_value(S, code, M);
-        alive = true;
-        u32 i = i0;
-        // kRoundUnroll primes per trip, every load issued before any test
-        // (a kill ends the round; tests past it in the trip are not counted)
-        for (; i + kRoundUnroll <= i1; i += kRoundUnroll) {
-          PrimeRec pr[kRoundUnroll];
-          u32 xo[kRoundUnroll];
-          u64 hm[kRoundUnroll];
+      bool alive = idx < n;
+      const u64 v = alive ? Q[idx] : 0;
+      const u32 vl = (u32)v & ((1u << kRedcSplit) - 1u);
+      const u32 vh = (u32)(v >> kRedcSplit);
+      // a dead lane idles until the chunk's last candidate dies
+      for (u32 i = i0; i < at && __any_sync(0xffffffffu, alive);
+           i += kRoundUnroll) {
+        if (alive) ntest += kRoundUnroll;
+        bool kill = false;
 #pragma unroll
-          for (int k = 0; k < kRoundUnroll; ++k) {
-            pr[k] = e.recs[i + k];
-            xo[k] = __ldg(xq + i + k);
-            hm[k] = KIND == KIND_DICKSON ? __ldg(e.hmask + i + k) : 0ull;
-          }
-          u32 kill = 0;
-#pragma unroll
-          for (int k = 0; k < kRoundUnroll; ++k) {
-            u32 rr = fk_bmod(v, pr[k].q, pr[k].magic) + xo[k];
-            rr = min(rr, rr - pr[k].q);
-            if (kill_test<KIND>(pr[k], rr, e.lists, S.sbits, e.xxmax, e.n,
-                                hm[k]))
-              kill |= 1u << k;
-          }
-          if (kill) {
-            i += __ffs((int)kill) - 1;
-            alive = false;
-            break;
+        for (u32 j = 0; j < kRoundUnroll; ++j) {
+          const TestRec t = S.srec[i + j];
+          const u32 q = redc_residue(t, S.skq[i + j], vl, vh);
+          if (KIND == KIND_DICKSON) {
+            const u32 h = min(q, t.q - q);
+            kill |= (S.sbit[S.sboff[i + j] + (h >> 5)] >> (h & 31)) & 1u;
+          } else {
+            kill |= kill_test<KIND>(c, first + i + j, t, q);
           }
         }
-        for (; alive && i < i1; ++i) {
-          const PrimeRec pr = e.recs[i];
-          u32 rr = fk_bmod(v, pr.q, pr.magic) + __ldg(xq + i);
-          rr = min(rr, rr - pr.q);
-          const u64 hm = KIND == KIND_DICKSON ? __ldg(e.hmask + i) : 0ull;
-          if (kill_test<KIND>(pr, rr, e.lists, S.sbits, e.xxmax, e.n, hm)) {
-            alive = false;
-            break;
-          }
-        }
-        ntest += (i - i0) + (alive ? 0 : 1);
+        alive = alive && !kill;
       }
       const u32 bal = __ballot_sync(0xffffffffu, alive);
-      if (alive) qout[out + __popc(bal & lt)] = code;
+      if (alive) Q[out + __popc(bal & lt)] = v;  // out <= base: read already
       out += __popc(bal);
     }
     __syncwarp();
-    u32* t = qin;
-    qin = qout;
-    qout = t;
     n = out;
   }
-  // emit survivors: one atomic per warp
+  at = min(first + at, NP);
+  const u32 deep = min(max(S.deep, at), NP);
+  n = drain_groups<KIND>(Q, n, c, at, deep, ntest);
+  // kDeep groups at a time: fewer votes and more loads in flight, once few
+  // candidates die among 128 primes
+  constexpr u32 kDeep = KIND == KIND_DICKSON ? 2 : 4;
+  at = deep;
+  for (; n > 0 && at + 32 * kDeep <= NP; at += 32 * kDeep) {
+    Prime<KIND> p[kDeep];
+#pragma unroll
+    for (u32 j = 0; j < kDeep; ++j) p[j].load(c, at + 32 * j + lane);
+    u32 out = 0;
+    for (u32 idx = 0; idx < n; ++idx) {
+      const u64 v = Q[idx];
+      const u32 vl = (u32)v & ((1u << kRedcSplit) - 1u);
+      const u32 vh = (u32)(v >> kRedcSplit);
+      bool kill = false;
+#pragma unroll
+      for (u32 j = 0; j < kDeep; ++j) kill |= p[j].kills(c, vl, vh);
+      if (!__any_sync(0xffffffffu, kill)) {
+        if (lane == 0) Q[out] = v;  // out <= idx: read already
+        ++out;
+      }
+    }
+    ntest += kDeep * n;
+    __syncwarp();
+    n = out;
+  }
+  n = drain_groups<KIND>(Q, n, c, at, NP, ntest);
+  // survivors: one atomic per warp
   if (n) {
     u64 base = 0;
-    if (lane == 0) base = atomicAdd(&a.ctr->ncand, (unsigned long long)n);
+    if (lane == 0) base = atomicAdd(&ctr->ncand, (unsigned long long)n);
     base = __shfl_sync(0xffffffffu, base, 0);
-    for (u32 idx = lane; idx < n; idx += 32)
-      emit_cand(a, cand_value(S, qin[idx], M), gitem, base + idx);
+    for (u32 idx = lane; idx < n; idx += 32) {
+      if (base + idx < cand_cap) {
+        cand_key[base + idx] = Q[idx];
+        cand_item[base + idx] = gitem;
+      } else {
+        atomicOr(&ctr->overflow, 1u);
+      }
+    }
   }
   __syncwarp();
+  return ntest;
 }
 
-__device__ __forceinline__ void drain_any(u32* qin, u32* qout, u32 n,
-                                          const SieveSmem& S,
-                                          const DevEngine& e,
-                                          const DevItem& it, u32 gitem,
-                                          const SieveArgs& a, u32 wq_short,
-                                          u32& ntest) {
-  switch (e.kind) {
+__device__ __forceinline__ u32 drain_any(u64* Q, u32 n, const SieveSmem& S,
+                                         u32 gitem, const SieveArgs& a) {
+  if (n == 0) return 0;
+  switch (S.kind) {
     case KIND_EULER:
-      warp_drain<KIND_EULER>(qin, qout, n, S, e, it, gitem, a, wq_short, ntest);
-      break;
+      return warp_drain<KIND_EULER>(Q, n, S, gitem, a.warp_queue, a.cand_key,
+                                    a.cand_item, a.cand_cap, a.ctr);
     case KIND_DICKSON:
-      warp_drain<KIND_DICKSON>(qin, qout, n, S, e, it, gitem, a, wq_short, ntest);
-      break;
+      return warp_drain<KIND_DICKSON>(Q, n, S, gitem, a.warp_queue, a.cand_key,
+                                      a.cand_item, a.cand_cap, a.ctr);
     default:
-      warp_drain<KIND_AP>(qin, qout, n, S, e, it, gitem, a, wq_short, ntest);
-      break;
+      return warp_drain<KIND_AP>(Q, n, S, gitem, a.warp_queue, a.cand_key,
+                                 a.cand_item, a.cand_cap, a.ctr);
   }
 }
 
@@ -486,134 +558,163 @@ __device__ __forceinline__ bool stage_patterns(u64* spat, const DevEngine& eg,
   return *status == 0;
 }
 
-// One block of 32 threads' chains (a warp task): thread wl of the warp
-// sweeps chain gw + (wl >> gsh) of the item, pushes its pattern survivors
-// into the warp's queue and drains it through the compaction rounds; the
-// queue is empty again on return.
+// Move a warp's columns (cn codes in this thread's) into its queue, which
+// holds qn entries and is drained when a row may not fit.  The thread's
+// chain: lane R, words w0, w0 + G, ...  Returns the queue's new length and
+// adds the lane's prime tests to ntest.  Not inlined, as warp_drain.
+static __device__ __noinline__ u32 flush_columns(const SieveSmem& S, u64* Q,
+                                          const unsigned short* C, u32 qn,
+                                          u32 cn, u64 R, u64 M, u32 w0, u32 G,
+                                          u32 gitem, const SieveArgs& a,
+                                          u32* ntest) {
+  const u32 wl = threadIdx.x & 31;
+  const u32 rows = __reduce_max_sync(0xffffffffu, cn);
+  for (u32 r = 0; r < rows; ++r) {
+    const u32 bal = __ballot_sync(0xffffffffu, r < cn);
+    if (qn + 32 > kWq) {
+      *ntest += drain_any(Q, qn, S, gitem, a);
+      qn = 0;
+    }
+    if (r < cn) {
+      const u32 code = C[32 * r];
+      const u64 u = 64ull * (w0 + (code >> 6) * G) + (code & 63u);
+      Q[qn + __popc(bal & ((1u << wl) - 1u))] = u * M + R;
+    }
+    qn += __popc(bal);
+  }
+  __syncwarp();
+  return qn;
+}
+
+// Push the set bits of one 32-bit half word into the thread's column while
+// it has room; the bits pushed are cleared.
+__device__ __forceinline__ void push_half(u32& x, u32 code, unsigned short* C,
+                                          u32& cn) {
+  while (x != 0 && cn < kColSlots) {
+    const u32 b = 31u - __clz((int)x);
+    x ^= 1u << b;
+    C[32 * cn] = (unsigned short)(code + b);
+    ++cn;
+  }
+}
+
+// One block of 32 threads' chains: thread wl of the warp sweeps chain
+// gw + (wl >> gsh) of the item and pushes its pattern survivors through its
+// column into the warp's queue (qn entries).
 template <int P0, int NS>
 __device__ __forceinline__ void sieve_block(
-    const u64* __restrict__ spat, SieveSmem& S, const SieveArgs& a,
-    const DevEngine& e, const DevItem& it, u32 gitem, u64 gw, u64 nchain,
-    u32 G, u32 gsh, u32 wq_short, u64 wfull, u32& ntest, u32& nword) {
-  const int tid = threadIdx.x;
-  const u32 wl = tid & 31, wid = tid >> 5;
-  const u64 U = it.U;
-  const u32 stride = G;
-  u32* wq = S.qa + wid * kWq;
-  u32* wq2 = S.qb + wid * kWq;
+    const u64* __restrict__ spat, SieveSmem& S, u64* Q, u32& qn,
+    const SieveArgs& a, const DevEngine& e, const DevItem& it, u32 gitem,
+    u64 gw, u64 nchain, u32& ntest, u32& nword) {
+  const u32 wl = threadIdx.x & 31;
+  const u32 G = it.lane_threads;
+  const u32 gsh = G == 32 ? 5u : (G == 8 ? 3u : 0u);
+  const u32 Tc = it.Tc, L = e.L;
+  const u64 U = it.U, M = e.M;
   // ---- this thread's chain -----------------------------------------
   const u64 g = gw + (wl >> gsh);
   const bool active = g < nchain;
-  const u64 chunk = active ? g / e.L : 0;
-  const u32 lane = active ? (u32)(g % e.L) : 0;
+  u32 chunk = 0, lane = 0;   // chunks per lane: below 2^30 words
+  if (active) {
+    if (nchain <= 0xFFFFFFFFull) {
+      chunk = (u32)g / L;
+      lane = (u32)g - chunk * L;
+    } else {
+      chunk = (u32)(g / L);
+      lane = (u32)(g % L);
+    }
+  }
   const u64 R = active ? e.lanes[lane] : 0;
-  const u64 w0 = chunk * (u64)G * it.Tc + (wl & (G - 1));
-  S.chain_R[tid] = R;
-  S.chain_w0[tid] = w0;
+  const u32 w0 = chunk * (G * Tc) + (wl & (G - 1));
+  const u32* xq = a.xq + it.xq_off;
   u32 rho[NS];
   if (G == 32) {
     // the whole warp sweeps one lane: thread I works out prime I's base
     // index once and the warp shares it (instead of every thread
     // computing all NS of them)
-    shared_setup<P0, NS, 32>(rho, e, a.xq + it.xq_off, S.minv, R,
-                             chunk * 32ull * it.Tc, wl);
+    shared_setup<P0, NS, 32>(rho, e, xq, S.minv, R, chunk * 32ull * Tc, wl);
   } else if (G == 8) {
     // the same within each group of eight threads sweeping one lane
-    shared_setup<P0, NS, 8>(rho, e, a.xq + it.xq_off, S.minv, R,
-                            chunk * 8ull * it.Tc, wl & 7u);
+    shared_setup<P0, NS, 8>(rho, e, xq, S.minv, R, chunk * 8ull * Tc, wl & 7u);
   } else {
-    Pat<P0, 0, NS>::setup(rho, R, 64ull * w0, a.xq + it.xq_off, S.minv);
+    Pat<P0, 0, NS>::setup(rho, R, 64ull * w0, xq, S.minv);
   }
-  u32 qn = 0;
-  if (active) {
-    // the chain's words in range: j < Tc with w0 + j*stride < ceil(U/64)
-    const u64 wend = (U + 63) >> 6;
-    if (w0 < wend)
-      nword += (u32)min((u64)it.Tc, (wend - w0 + stride - 1) / stride);
-  }
-  __syncwarp();
-  for (u32 wi = 0; wi < it.Tc; wi += 2) {
+  unsigned short* C = S.col + (threadIdx.x >> 5) * (kColSlots * 32) + wl;
+  u32 cn = 0;
+  // words in range: below wend; words from 1 to wfull - 1 lie whole inside
+  // the item, so only the first word (lo_off) and the last (hi_last, U)
+  // need a validity mask
+  const u32 wend = (u32)((U + 63) >> 6);
+  const u32 wfull = U ? (u32)((U - 1) >> 6) : 0;
+  if (active && w0 < wend) nword += min(Tc, (wend - w0 + G - 1) / G);
+  for (u32 wi = 0; wi < Tc; wi += 2) {
     // two words of the chain: j = wi and wi + 1
-    u64 sv[2] = {0, 0};
-    if (active) {
-      u64 acc[4] = {0, 0, 0, 0};
-      if (G == 32)
-        Pat<P0, 0, NS>::template word2<32>(spat, rho, acc);
-      else if (G == 8)
-        Pat<P0, 0, NS>::template word2<8>(spat, rho, acc);
-      else
-        Pat<P0, 0, NS>::template word2<1>(spat, rho, acc);
+    u64 acc[4] = {0, 0, 0, 0};
+    if (G == 32)
+      Pat<P0, 0, NS>::template word2<32>(spat, rho, acc);
+    else if (G == 8)
+      Pat<P0, 0, NS>::template word2<8>(spat, rho, acc);
+    else
+      Pat<P0, 0, NS>::template word2<1>(spat, rho, acc);
+    u64 sv[2];
 #pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const u64 w = w0 + (u64)(wi + k) * stride;
-        const u64 s = ~(acc[k * 2] | acc[k * 2 + 1]);
-        if (w != 0 && w < wfull && wi + k < it.Tc) {
-          sv[k] = s;  // an interior word: every period is in range
-          continue;
-        }
-        if (wi + k >= it.Tc || 64ull * w >= U) continue;
+    for (int k = 0; k < 2; ++k) {
+      const u32 w = w0 + (wi + k) * G;
+      u64 s = ~(acc[k * 2] | acc[k * 2 + 1]);
+      if (!active || wi + k >= Tc || w >= wend) {
+        s = 0;
+      } else if (w == 0 || w >= wfull) {
         const u64 left = U - 64ull * w;
-        u64 valid = left >= 64 ? ~0ull : ((1ull << left) - 1ull);
-        if (w == 0 && R < it.lo_off) valid &= ~1ull;
-        if (left <= 64 && R >= it.hi_last) valid &= ~(1ull << (left - 1));
-        sv[k] = s & valid;
+        if (left < 64) s &= (1ull << left) - 1ull;
+        if (w == 0 && R < it.lo_off) s &= ~1ull;
+        if (left <= 64 && R >= it.hi_last) s &= ~(1ull << (left - 1));
       }
+      sv[k] = s;
     }
-    // push the survivors into the warp's queue; drain first when they
-    // do not fit, and when one step alone overfills an empty queue
-    // push the prefix that fits and drain again (every pass pushes or
-    // drains, so it ends)
+    // into the columns; a full one empties the warp's
+    u32 x[4] = {(u32)sv[0], (u32)(sv[0] >> 32), (u32)sv[1],
+                (u32)(sv[1] >> 32)};
     for (;;) {
-      const u32 c = __popcll(sv[0]) + __popcll(sv[1]);
-      const u32 tot = __reduce_add_sync(0xffffffffu, c);
-      if (tot == 0) break;
-      if (qn + tot > kWq && qn > 0) {
-        drain_any(wq, wq2, qn, S, e, it, gitem, a, wq_short, ntest);
-        qn = 0;
-        continue;
-      }
-      // exclusive prefix of c over the warp
-      u32 x = c;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const u32 y = __shfl_up_sync(0xffffffffu, x, o);
-        if (wl >= (u32)o) x += y;
-      }
-      u32 pos = qn + x - c;
-      const u32 end = min(qn + tot, (u32)kWq);
+      for (int k = 0; k < 4; ++k) push_half(x[k], (wi << 6) + 32 * k, C, cn);
+      if (!__any_sync(0xffffffffu, (x[0] | x[1] | x[2] | x[3]) != 0)) break;
+      // the table indexes wait out the flush in local memory: live across
+      // the call they would be spilled in the word loop instead
+      volatile u32 keep[NS];
 #pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        while (sv[k] && pos < end) {
-          const int b = __ffsll((long long)sv[k]) - 1;
-          sv[k] &= sv[k] - 1;
-          wq[pos++] = ((u32)tid << 22) | ((wi + k) << 6) | (u32)b;
-        }
-      }
-      __syncwarp();
-      if (qn + tot <= (u32)kWq) {
-        qn += tot;
-        break;
-      }
-      drain_any(wq, wq2, kWq, S, e, it, gitem, a, wq_short, ntest);
-      qn = 0;
+      for (int i = 0; i < NS; ++i) keep[i] = rho[i];
+      qn = flush_columns(S, Q, C, qn, cn, R, M, w0, G, gitem, a, &ntest);
+      cn = 0;
+#pragma unroll
+      for (int i = 0; i < NS; ++i) rho[i] = keep[i];
     }
   }
-  // every queued code refers to this warp task's chains: drain them
-  // before the warp's threads take the next task's chains
-  drain_any(wq, wq2, qn, S, e, it, gitem, a, wq_short, ntest);
+  // the codes refer to this block's chains
+  qn = flush_columns(S, Q, C, qn, cn, R, M, w0, G, gitem, a, &ntest);
+}
+
+// Claim the CTA's next task into slot p: its number and its item (entry of
+// the family's list).
+__device__ __forceinline__ void claim_task(const SieveArgs& a, SieveSmem& S,
+                                           u32 p, u32 from) {
+  const u64 t = atomicAdd(a.task_ctr, 1ull);
+  S.task[p] = t;
+  S.wnext[p] = 0;
+  S.item[p] = t < a.ntask ? task_item(a, t, from) : 0u;
 }
 
 // NS: the pattern primes this variant stages (the engine descriptor's NS
-// and round cuts must match it).  DYN: the CTA's warps claim blocks of
-// chains from a shared counter (a.warp_tasks blocks per task); without it
-// each warp takes exactly its own block (a.warp_tasks = 8), which holds
-// fewer registers across the word loop.
-template <int P0, int NS, bool DYN>
-__global__ void __launch_bounds__(kBlock, 3) k_sieve(SieveArgs a) {
+// and round cuts must match it).  A CTA task is it.blocks blocks of 32
+// threads' chains, claimed by the warps from the CTA's counter, so a warp
+// held up by a queue drain takes fewer of them; the next task is claimed
+// while this one runs, so a task costs one barrier.
+template <int P0, int NS>
+__global__ void __launch_bounds__(kBlock, 3)
+    k_sieve(const __grid_constant__ SieveArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   u64* spat = reinterpret_cast<u64*>(smem_raw);
   SieveSmem& S = *reinterpret_cast<SieveSmem*>(smem_raw + pat_bytes<P0, NS>());
-  const int tid = threadIdx.x;
+  const u32 tid = threadIdx.x, wl = tid & 31, wid = tid >> 5;
   if (tid == 0) {
     S.eng = 0xFFFFFFFFu;
     const u32 mb = smem_u32(&S.mbar);
@@ -621,92 +722,91 @@ __global__ void __launch_bounds__(kBlock, 3) k_sieve(SieveArgs a) {
                  : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    claim_task(a, S, 0, 0);
   }
   __syncthreads();
   u32 phase = 0;
-
-  for (;;) {
-    if (tid == 0) {
-      const u64 t = atomicAdd(a.task_ctr, 1ull);
-      S.task = t;
-      S.wnext = 0;
-      if (t < a.ntask) {
-        // binary search: last entry with task_prefix[i] <= t
-        u32 lo = 0, hi = a.nitems;
-        while (hi - lo > 1) {
-          const u32 mid = (lo + hi) >> 1;
-          if (a.task_prefix[mid] <= t) lo = mid; else hi = mid;
-        }
-        S.item = lo;
-        S.stride = a.items[a.item_index[lo]].lane_threads;
-      }
-    }
-    __syncthreads();
-    const u64 task = S.task;
-    if (task >= a.ntask) break;
-    const u32 gitem = a.item_index[S.item];
-    const DevItem it = a.items[gitem];
-    const u32 eidx = it.engine;
-    const DevEngine& eg = a.engines[eidx];
-    // ---- engine switch: stage its pattern table into shared memory ----
-    if (S.eng != eidx) {
-      if (!stage_patterns<P0, NS>(spat, eg, &S.mbar, &S.status, phase, a.ctr))
-        return;
-      for (u32 i = tid; i < (u32)NS; i += kBlock) S.minv[i] = eg.pat_minv[i];
-      for (u32 i = tid; i < eg.sbits_words && i < 512; i += kBlock)
-        S.sbits[i] = eg.sbits[i];
-      __syncthreads();
-      if (tid == 0) S.eng = eidx;
-    }
-    const DevEngine e = eg;
-    // ---- warp tasks ------------------------------------------------------
-    // A CTA task is a.warp_tasks blocks of 32 threads' chains; each warp
-    // claims blocks from the CTA's counter until none is left, so a warp
-    // held up by a long queue drain takes fewer of them and the barrier
-    // that ends the CTA task comes once per a.warp_tasks blocks.
-    // G = lane_threads threads sweep one lane: thread t of the group takes
-    // words t, t + G, ... of a G * Tc word block, so a group's pattern
-    // loads are G consecutive table entries (G = 1: one lane per thread,
-    // Tc consecutive words; 8: four lanes per warp; 32: one per warp)
-    const u32 G = it.lane_threads;
-    const u32 gsh = G == 32 ? 5u : (G == 8 ? 3u : 0u);
-    const u32 wl = tid & 31, wid = tid >> 5;
-    const u64 nchain = it.nchunk * e.L;
-    const u64 wt0 = (task - a.task_prefix[S.item]) * (u64)a.warp_tasks;
-    const u32 cpw = 32u >> gsh;  // chains per warp task
-    const u32 wq_short = a.warp_queue;
-    // words below wfull end before the item's last period, so only the
-    // first word (lo_off) and the last (hi_last, U) need a validity mask
-    const u64 wfull = it.U ? (it.U - 1) >> 6 : 0;
-    u32 ntest = 0, nword = 0;  // this CTA task's counts
-    if (DYN) {
-      for (;;) {
-        u32 wt = 0;
-        if (wl == 0) wt = atomicAdd(&S.wnext, 1u);
-        wt = __shfl_sync(0xffffffffu, wt, 0);
-        if (wt >= a.warp_tasks) break;
-        const u64 gw = (wt0 + wt) * cpw;     // the warp task's first chain
-        if (gw >= nchain) break;             // and every later one's too
-        sieve_block<P0, NS>(spat, S, a, e, it, gitem, gw, nchain, G, gsh,
-                            wq_short, wfull, ntest, nword);
-      }
-    } else {
-      // this warp's own block (a block past the item's chains runs with
-      // every thread inactive and emits nothing)
-      sieve_block<P0, NS>(spat, S, a, e, it, gitem, (wt0 + wid) * cpw,
-                          nchain, G, gsh, wq_short, wfull, ntest, nword);
-    }
-    u64 nt = ntest, nw = nword;  // warp sums in 64 bits
+  u64* Q = S.queue + wid * kWq;
+  u32 qn = 0, gitem = 0xFFFFFFFFu;
+  u32 ntest = 0, nword = 0;  // since the last report
+  for (u32 p = 0;; p ^= 1u) {
+    const u64 task = S.task[p];
+    const u32 entry = S.item[p];
+    const bool done = task >= a.ntask;
+    const u32 next = done ? 0xFFFFFFFFu : a.item_index[entry];
+    if (done || next != gitem) {
+      // another item, or the end (a CTA may find every task claimed before
+      // its first): drain this one's queue and report
+      ntest += drain_any(Q, qn, S, gitem, a);
+      qn = 0;
+      u64 nt = ntest, nw = nword;  // warp sums in 64 bits
+      ntest = nword = 0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      nt += __shfl_down_sync(0xffffffffu, nt, o);
-      nw += __shfl_down_sync(0xffffffffu, nw, o);
+      for (int o = 16; o > 0; o >>= 1) {
+        nt += __shfl_down_sync(0xffffffffu, nt, o);
+        nw += __shfl_down_sync(0xffffffffu, nw, o);
+      }
+      if (wl == 0) {
+        if (nt) atomicAdd(&a.ctr->s2_tests, (unsigned long long)nt);
+        if (nw) atomicAdd(&a.ctr->s1_words, (unsigned long long)nw);
+      }
+      if (done) break;
+      __syncthreads();   // every warp is past the old item's tables
+      gitem = next;
+      const u32 eidx = a.items[gitem].engine;
+      const DevEngine& eg = a.engines[eidx];
+      if (S.eng != eidx) {
+        // ---- engine switch: stage its pattern table into shared memory ----
+        if (!stage_patterns<P0, NS>(spat, eg, &S.mbar, &S.status, phase, a.ctr))
+          return;
+        for (u32 i = tid; i < (u32)NS; i += kBlock) S.minv[i] = eg.pat_minv[i];
+        for (u32 i = tid; i <= eg.sbits_words; i += kBlock)
+          S.sbits[i] = i < eg.sbits_words ? eg.sbits[i] : 0u;
+        __syncthreads();   // and every warp has read S.eng
+        if (tid == 0) S.eng = eidx;
+      }
+      const u32 first = eg.rounds[0];
+      if (tid < (u32)kStaged && first < eg.NP) {
+        const u32 p = min(first + tid, eg.NP - 1);  // past the end: the last
+        S.srec[tid] = eg.trec[p];
+        S.skq[tid] = a.xq[a.items[gitem].xq_off + p];
+        if (eg.kind == KIND_DICKSON)
+          S.sboff[tid] = eg.boff[p - kNSMin] - eg.boff[first - kNSMin];
+      }
+      if (eg.kind == KIND_DICKSON && first < eg.NP) {
+        const u32 b0 = eg.boff[first - kNSMin];
+        const u32 b1 = eg.boff[min(first + kStaged, eg.NP) - kNSMin];
+        for (u32 i = b0 + tid; i < b1; i += kBlock) S.sbit[i - b0] = eg.bits[i];
+      }
+      if (tid == 0) {
+        S.ctx = TestCtx{eg.trec, eg.filt, a.xq + a.items[gitem].xq_off,
+                        eg.lists, S.sbits, eg.n, eg.xxmax, eg.sbits_words,
+                        eg.ap_div};
+        S.rounds = eg.rounds;
+        S.NP = eg.NP;
+        S.deep = eg.deep;
+        S.kind = eg.kind;
+      }
+      __syncthreads();
     }
-    if (wl == 0) {
-      if (nt) atomicAdd(&a.ctr->s2_tests, (unsigned long long)nt);
-      if (nw) atomicAdd(&a.ctr->s1_words, (unsigned long long)nw);
+    if (tid == 0) claim_task(a, S, p ^ 1u, entry);
+    const DevItem& it = a.items[gitem];
+    const DevEngine& e = a.engines[it.engine];
+    const u32 G = it.lane_threads, nblock = it.blocks;
+    const u32 cpw = G == 32 ? 1u : (G == 8 ? 4u : 32u);  // chains per block
+    const u64 nchain = it.nchunk * e.L;
+    const u64 b0 = (task - a.task_prefix[entry]) * (u64)nblock;
+    for (;;) {
+      u32 wt = 0;
+      if (wl == 0) wt = atomicAdd(&S.wnext[p], 1u);
+      wt = __shfl_sync(0xffffffffu, wt, 0);
+      if (wt >= nblock) break;
+      const u64 gw = (b0 + wt) * cpw;      // the block's first chain
+      if (gw >= nchain) break;             // and every later one's too
+      sieve_block<P0, NS>(spat, S, Q, qn, a, e, it, gitem, gw, nchain, ntest,
+                          nword);
     }
-    __syncthreads();
+    __syncthreads();   // the next task is claimed, this one's counter free
   }
 }
 

@@ -1,4 +1,4 @@
-// fk_sieve_k.cu -- the pattern-sieve kernel variants k_sieve<P0, NS, DYN>
+// fk_sieve_k.cu -- the pattern-sieve kernel variants k_sieve<P0, NS>
 // and the dispatch of every sieve launch (fk_launch.h).
 #include "fk_launch.h"
 
@@ -12,23 +12,14 @@ size_t sieve_smem() {
 
 template <int P0, int NS>
 cudaError_t sieve_limit() {
-  cudaError_t r = cudaFuncSetAttribute(
-      k_sieve<P0, NS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-      (int)sieve_smem<P0, NS>());
-  if (r != cudaSuccess) return r;
-  return cudaFuncSetAttribute(k_sieve<P0, NS, true>,
+  return cudaFuncSetAttribute(k_sieve<P0, NS>,
                               cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)sieve_smem<P0, NS>());
 }
 
-// Eight blocks per task is one per warp: the variant without the shared
-// counter; more blocks per task take the claiming variant.
 template <int P0, int NS>
 cudaError_t sieve_launch(u32 grid, cudaStream_t s, const SieveArgs& a) {
-  if (a.warp_tasks == kBlock / 32)
-    k_sieve<P0, NS, false><<<grid, kBlock, sieve_smem<P0, NS>(), s>>>(a);
-  else
-    k_sieve<P0, NS, true><<<grid, kBlock, sieve_smem<P0, NS>(), s>>>(a);
+  k_sieve<P0, NS><<<grid, kBlock, sieve_smem<P0, NS>(), s>>>(a);
   return cudaGetLastError();
 }
 

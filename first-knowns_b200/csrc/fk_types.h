@@ -2,6 +2,8 @@
 #pragma once
 #include <cstdint>
 
+#include "fk_redc.h"
+
 namespace fk {
 
 enum Kind : uint32_t { KIND_EULER = 0, KIND_DICKSON = 1, KIND_AP = 2 };
@@ -13,15 +15,23 @@ enum Mode : uint32_t {
   MODE_DENSE = 2,   // no sieve: every x in the range is classified
 };
 
-// Per-prime record for the per-candidate stage (16 bytes).
+// Per-prime record of the set-up work: base residues, lane shifts (16
+// bytes).  The per-candidate tests have their own (TestRec, fk_redc.h).
 struct PrimeRec {
   uint32_t q;
-  uint32_t aux;     // kind test data (see fk_engine.cu, build_tests)
+  uint32_t pad;
   uint64_t magic;   // floor(2^64 / q)
 };
 
+// Screen of a prime whose forbidden residues are an explicit list: bit
+// (r & 31) of f0, (r >> 5 & 31) of f1 and (r >> 10 & 31) of f2 are set for
+// every listed r, so a residue off the list passes all three only rarely;
+// list = offset | count << 24 into the residue lists, in groups of four.
+struct alignas(16) ListFilter {
+  uint32_t f0, f1, f2, list;
+};
+
 constexpr int kBlock = 256;       // threads per CTA, every kernel
-constexpr int kQcap = 4096;       // candidate queue entries per CTA (8 warps)
 constexpr int kNS = 32;           // pattern primes per CTA (default)
 constexpr int kNSMin = 24;        // fewest pattern primes a kernel variant
                                   // stages; marking tables start here
@@ -33,6 +43,10 @@ constexpr int kClassChunk = 128;  // candidates a warp fetches at once
 constexpr int kBucketFill = 1024; // expected entries per ordering bucket
 constexpr int kWarpMode = 32;     // warp queue below which a candidate
                                   // takes a whole warp
+constexpr int kSbits = 512;       // Euler: most words of the {x^2 + x} bitset
+constexpr int kStaged = 128;      // rounds: test primes held in shared memory
+constexpr int kStagedBits = 1536; // Dickson: words of their residue bitmaps
+constexpr int kMaxTaskBlocks = 256;  // rounds: most warp blocks per CTA task
 constexpr int kSeg = 32768;       // marking: periods per shared segment
                                   // (default; variants 16384 and 65536)
 constexpr int kNumSeg = 3;        // marking segment variants
@@ -61,9 +75,21 @@ struct DevEngine {
   const uint32_t* pat_i64;        // [kNSMax] 64^-1 mod q
   const PrimeRec* recs;           // [NP]
   const uint32_t* c64;            // [NP] 2^64 mod q
+  // per-candidate tests: the scaled residue r = (X0 + v) * a mod q
+  // (fk_redc.h), a by kind -- Euler -1 (killed: r among the x^2 + x), AP
+  // -1/d (killed: r < n; for the primes dividing d a = -1 and r = 0),
+  // Dickson 1 (killed: min(r, q - r) on the prime's list)
+  const TestRec* trec;            // [NP]
+  const ListFilter* filt;         // Dickson [NP]; AP with ap_div [NP]: f0 =
+                                  // 1 when q divides d
   const uint32_t* lists;          // explicit forbidden-residue lists
-  const uint64_t* hmask;          // [NP] Dickson: bit (h mod 64) set for
-                                  // each half residue h on the prime's list
+  // Dickson, the primes from index kNSMin that a drain can stage: exact
+  // bitmaps of the killed min(r, q - r), prime i's at word boff[i - kNSMin]
+  const uint32_t* boff;
+  const uint32_t* bits;
+  uint32_t deep;                  // rounds: first prime past which 128 primes
+                                  // kill less than a quarter
+  uint32_t ap_div;                // AP: a sieve prime divides d
   const uint32_t* rounds;         // [nrounds + 1] prime-index cuts
   const uint32_t* sbits;          // Euler: bitset of {x^2 + x : x < n}
   // marking sieve (long lanes): primes [NS, NPm) are marked in a per-lane
@@ -104,8 +130,11 @@ struct DevItem {
                                   // t + lane_threads, ... of its block
   uint64_t nchunk;                // chains per lane
   uint64_t task0, ntask;          // first task, task count
-  uint64_t xq_off;                // this item's base-residue table
-  uint32_t marked, pad2;          // 1: the marking kernel sweeps this item
+  uint64_t xq_off;                // this item's base-residue table: X0 mod q
+                                  // of the primes sieved by pattern or mark,
+                                  // X0 * c1 mod q of the primes tested
+  uint32_t marked;                // 1: the marking kernel sweeps this item
+  uint32_t blocks;                // rounds: warp blocks per CTA task
   uint64_t nchunk_u;              // marking: u-chunks per lane
 };
 
