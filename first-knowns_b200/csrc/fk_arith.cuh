@@ -71,9 +71,9 @@ __host__ __device__ constexpr u32 fk_inv64(u32 q) {
 }
 
 // Word offset of pattern prime I (counted from prime index P0) in the
-// concatenated pattern table: the sum of the I primes before it.
-__host__ __device__ constexpr u32 fk_pat_prefix(int P0, int I) {
+// concatenated pattern tables of q + pad words each.
+__host__ __device__ constexpr u32 fk_pat_prefix(int P0, int I, u32 pad = 0) {
   u32 s = 0;
-  for (int k = 0; k < I; ++k) s += fk_nth_prime(P0 + k);
+  for (int k = 0; k < I; ++k) s += fk_nth_prime(P0 + k) + pad;
   return s;
 }

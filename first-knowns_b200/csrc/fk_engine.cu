@@ -409,8 +409,9 @@ static fk_status build_engine(fk_engine* e) {
   // rho = 64k mod q, so a lane's consecutive words are consecutive entries
   // and the 32 lanes of a warp sweeping one lane read 32 consecutive
   // entries (no bank conflict)
-  std::vector<u64> pat;
+  std::vector<u64> pat, patw, patn;
   std::vector<u32> minv(kNSMax), i64(kNSMax);
+  std::vector<TestRec> prec(kNSMax);
   for (int i = 0; i < kNSMax; ++i) {
     const u32 q = e->sieve[i];
     if (q != fk_nth_prime((int)P0 + i))
@@ -428,6 +429,10 @@ static fk_status build_engine(fk_engine* e) {
         if (g[(rho + b) % q]) w |= 1ull << b;
       pat.push_back(w);
     }
+    const size_t t = pat.size() - q;
+    for (u32 k = 0; k < q + kPadWide; ++k) patw.push_back(pat[t + k % q]);
+    for (u32 k = 0; k < q + kPadNarrow; ++k) patn.push_back(pat[t + k % q]);
+    prec[i] = redc_rec(q, minv[i]);
     e->survival *= 1.0 - (double)e->forb[i].size() / q;
   }
   // ---- per-candidate primes -----------------------------------------------
@@ -565,6 +570,11 @@ static fk_status build_engine(fk_engine* e) {
   fk_status st;
   if ((st = upload(e, e->lanes, &d.lanes))) return st;
   if ((st = upload(e, pat, &d.pat, pat_bytes_for(P0)))) return st;
+  if ((st = upload(e, patw, &d.patw, pat_bytes_for(P0) + kNSMax * kPadWide * 8)))
+    return st;
+  if ((st = upload(e, patn, &d.patn, pat_bytes_for(P0) + kNSMax * kPadNarrow * 8)))
+    return st;
+  if ((st = upload(e, prec, &d.prec))) return st;
   if ((st = upload(e, minv, &d.pat_minv))) return st;
   if ((st = upload(e, i64, &d.pat_i64))) return st;
   if ((st = upload(e, recs, &d.recs))) return st;
@@ -686,6 +696,7 @@ struct fk_batch {
   DevBuf<u32> d_nb, d_bcount, d_bfill, d_nbuckets;
   DevBuf<u64> d_bbase, d_boff;
   DevBuf<unsigned long long> d_task_ctr;
+  DevBuf<unsigned long long> d_block_ctr;  // rounds: blocks claimed per item
   DevBuf<u32> d_nitems;
   DevBuf<u32> d_rounds;         // per engine: this batch's round cuts
   DevCounters* d_ctr = nullptr;
@@ -800,7 +811,7 @@ static void batch_free(fk_batch* b) {
   b->d_item_off.release(); b->d_sorted.release(); b->d_scratch.release();
   b->d_nb.release(); b->d_bcount.release(); b->d_bfill.release();
   b->d_nbuckets.release(); b->d_bbase.release(); b->d_boff.release();
-  b->d_task_ctr.release(); b->d_nitems.release(); b->d_rounds.release();
+  b->d_task_ctr.release(); b->d_block_ctr.release(); b->d_nitems.release(); b->d_rounds.release();
   for (auto& f : b->fam) { f.d_idx.release(); f.d_prefix.release(); }
   b->h_items.release(); b->h_ctr.release(); b->h_off.release();
   b->h_sorted.release(); b->h_small.release(); b->h_prefix.release();
@@ -930,14 +941,13 @@ static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
         di.Tc = (u32)tc;
         di.nchunk = (words + G * tc - 1) / (G * tc);
         const u64 chains = di.nchunk * L;      // one per group
-        const u64 blocks = (chains + 32 / G - 1) / (32 / G);
-        // blocks per CTA task: as many as leave every CTA about 16 tasks
-        // (the last ones' imbalance), at most kMaxTaskBlocks
-        const u64 ctas = (u64)b->nsm * b->tune.sieve_ctas_per_sm;
-        di.blocks = (u32)std::min<u64>(
-            std::max<u64>(blocks / (ctas * 16), b->tune.warp_tasks),
-            kMaxTaskBlocks);
-        di.ntask = (blocks + di.blocks - 1) / di.blocks;
+        di.ntask = (chains + 32 / G - 1) / (32 / G);
+        // blocks a warp claims at once: as many as leave every warp about
+        // 16 claims (the last ones' imbalance), times warp_tasks / 8
+        const u64 warps = (u64)b->nsm * b->tune.sieve_ctas_per_sm * (kBlock / 32);
+        di.run = (u32)std::min<u64>(
+            std::max<u64>(di.ntask / (warps * 16), 1) * (b->tune.warp_tasks / 8),
+            kMaxRun);
       }
       Family& f = b->fam[fam_of(e->P0, mark)];
       di.task0 = f.prefix.back();
@@ -982,6 +992,7 @@ static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
   }
   const u64 ni = b->items.size();
   if ((st = b->d_items.ensure(ni + 1))) return st;
+  if ((st = b->d_block_ctr.ensure(ni + 1))) return st;
   if ((st = b->d_item_count.ensure(ni + 1))) return st;
   if ((st = b->d_item_fill.ensure(ni + 1))) return st;
   if ((st = b->d_item_off.ensure(ni + 2))) return st;
@@ -1023,6 +1034,8 @@ static fk_status enqueue(fk_batch* b, bool capturing = false) {
   FK_CUDA(cudaMemsetAsync(b->d_task_ctr.p, 0, 8 * sizeof(unsigned long long), s));
   FK_CUDA(cudaMemsetAsync(b->d_item_count.p, 0, (ni + 1) * sizeof(u32), s));
   FK_CUDA(cudaMemsetAsync(b->d_item_fill.p, 0, (ni + 1) * sizeof(u32), s));
+  FK_CUDA(cudaMemsetAsync(b->d_block_ctr.p, 0,
+                          (ni + 1) * sizeof(unsigned long long), s));
   FK_CUDA(record(b->ev[0], s, capturing));
   u64 nl = 1;  // k_classify
   if (!b->sieve_idx.empty()) {
@@ -1038,6 +1051,7 @@ static fk_status enqueue(fk_batch* b, bool capturing = false) {
                                           b->d_cand_key.p, b->d_cand_item.p,
                                           b->cand_cap, b->d_ctr);
   }
+  u64 blocks0 = 0;   // the rounds families' items share one counter array
   for (int f = 0; f < 8; ++f) {
     Family& F = b->fam[f];
     b->fam_ran[f] = !F.idx.empty();
@@ -1056,11 +1070,14 @@ static fk_status enqueue(fk_batch* b, bool capturing = false) {
     a.cand_cap = b->cand_cap;
     a.ctr = b->d_ctr;
     a.task_ctr = b->d_task_ctr.p + f;
+    a.block_ctr = b->d_block_ctr.p + blocks0;
+    if (!F.mark) blocks0 += F.idx.size();
     a.warp_queue = b->tune.warp_queue;
     a.seg_per_task = b->tune.seg_per_task;
-    const u64 grid = std::min<u64>(
-        a.ntask, (u64)b->nsm * (F.mark ? b->tune.mark_ctas_per_sm
-                                       : b->tune.sieve_ctas_per_sm));
+    const u64 grid =
+        F.mark ? std::min<u64>(a.ntask, (u64)b->nsm * b->tune.mark_ctas_per_sm)
+               : std::min<u64>((a.ntask + kBlock / 32 - 1) / (kBlock / 32),
+                               (u64)b->nsm * b->tune.sieve_ctas_per_sm);
     ++nl;
     const u32 P0 = F.P0;
     if (F.mark)
@@ -1164,6 +1181,7 @@ static fk_status launch(fk_batch* b, int use_graph) {
   for (auto& f : b->fam) { key.push_back(f.idx.size()); key.push_back(f.prefix.back()); }
   key.push_back((u64)(uintptr_t)b->d_items.p);
   key.push_back((u64)(uintptr_t)b->d_cand_key.p);
+  key.push_back((u64)(uintptr_t)b->d_block_ctr.p);
   key.push_back(((u64)b->tune.sieve_ctas_per_sm << 32) | b->tune.mark_ctas_per_sm);
   key.push_back(((u64)b->tune.warp_queue << 32) | b->tune.seg_per_task);
   key.push_back(((u64)b->tune.warp_tasks << 32) | b->tune.classify_ctas_per_sm);

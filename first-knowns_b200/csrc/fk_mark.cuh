@@ -81,7 +81,7 @@ template <int KIND>
 __device__ __forceinline__ bool tail_alive(u64 v, const DevEngine& e,
                                            const u32* __restrict__ kq,
                                            const u32* s_sbits, u64& ntest) {
-  const TestCtx c{e.trec, e.filt, kq, e.lists, s_sbits,
+  const TestCtx c{e.trec, e.filt, kq, e.lists,
                   e.n, e.xxmax, e.sbits_words, e.ap_div};
   const u32 vl = (u32)v & ((1u << kRedcSplit) - 1u);
   const u32 vh = (u32)(v >> kRedcSplit);
@@ -89,7 +89,7 @@ __device__ __forceinline__ bool tail_alive(u64 v, const DevEngine& e,
     ++ntest;
     Prime<KIND> p;
     p.load(c, i);
-    if (p.kills(c, vl, vh))
+    if (p.kills(c, s_sbits, vl, vh))
       return false;
   }
   return true;
@@ -139,7 +139,8 @@ __global__ void __launch_bounds__(kBlock, 3) k_mark(SieveArgs a) {
     const u32 eidx = it.engine;
     const DevEngine& eg = a.engines[eidx];
     if (S.eng != eidx) {
-      if (!stage_patterns<P0, NS>(spat, eg, &S.mbar, &S.status, phase, a.ctr))
+      if (!stage_patterns<pat_bytes<P0, NS>()>(spat, eg.pat, &S.mbar, &S.status,
+                                               phase, a.ctr))
         return;
       for (u32 i = tid; i < (u32)NS; i += kBlock) S.minv[i] = eg.pat_minv[i];
       for (u32 i = tid; i <= eg.sbits_words; i += kBlock)

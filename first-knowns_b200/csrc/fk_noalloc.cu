@@ -333,11 +333,11 @@ extern "C" fk_status fk_sieve_noalloc(fk_engine* e, const uint64_t lo[2],
   it.Tc = (u32)tc;
   it.lane_threads = 1;  // one lane per thread, Tc consecutive words
   it.nchunk = (words + tc - 1) / tc;
-  const u64 ntask = (it.nchunk * v.L + kBlock - 1) / kBlock;
+  const u64 ntask = (it.nchunk * v.L + 31) / 32;  // blocks of 32 chains
   it.ntask = ntask;
+  it.run = 1;
   it.xq_off = 0;
   it.marked = 0;
-  it.blocks = kBlock / 32;  // ntask above counts kBlock chains per task
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   k_na_init<<<1, kBlock, 0, s>>>(base, v.dev, it, ntask);
   k_na_xq<<<64, kBlock, 0, s>>>(base);
@@ -353,10 +353,11 @@ extern "C" fk_status fk_sieve_noalloc(fk_engine* e, const uint64_t lo[2],
   a.cand_item = at<u32>(base, kOffCandItem);
   a.cand_cap = kMaxCand;
   a.ctr = at<DevCounters>(base, kOffCtr);
-  a.task_ctr = at<unsigned long long>(base, kOffTaskCtr);
+  a.block_ctr = at<unsigned long long>(base, kOffTaskCtr);
   a.warp_queue = kWarpMode;
   a.seg_per_task = kSegPerTask;
-  const u32 grid = (u32)(ntask < (u64)nsm * 2 ? ntask : (u64)nsm * 2);
+  const u64 ctas = (ntask + kBlock / 32 - 1) / (kBlock / 32);
+  const u32 grid = (u32)(ctas < (u64)nsm * 2 ? ctas : (u64)nsm * 2);
   // the engine's own descriptor is the default variant: kNS pattern primes
   ce = launch_sieve(v.P0, kNS, grid, s, a);
   if (ce != cudaSuccess) return set_error(FK_ERR_DEVICE, cudaGetErrorString(ce));

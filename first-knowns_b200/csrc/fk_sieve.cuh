@@ -5,10 +5,9 @@
 // Tc 64-period words per thread: either one thread per lane on Tc
 // consecutive words, or -- for long lanes -- one warp per lane, thread t
 // on words t, t + 32, ... (so a warp's pattern loads are 32 consecutive
-// table entries).  32 threads' chains are a BLOCK; a CTA task is a run of
-// one item's blocks, pulled from a device counter by a persistent grid, so
-// thousands of items of uneven length run in one launch, and inside a task
-// the warps claim blocks from a shared counter.
+// table entries).  32 threads' chains are a BLOCK; the warps of a persistent
+// grid claim runs of an item's blocks from the item's counter, so thousands
+// of items of uneven length run in one launch.
 //
 // S1 (pattern sieve).  For the NS pattern primes starting at prime index
 // P0 (NS = 24, 32 or 40: a template variant chosen per batch) --
@@ -33,13 +32,13 @@
 // kill test on the scaled residue.  Final survivors are appended to a
 // global candidate list with warp-aggregated atomics.
 //
-// What bounds it, and what this shape measured (B200, kernel ms against
-// the 64-bit Barrett tests with a queue drained at every block's end): the
-// kernel issues instructions, so the tests' length is what counts -- 10
-// to 20 warp instructions a test against 58 -- then the pattern loads'
-// shared-memory wavefronts.  256 mixed intervals 204 -> 119 ms, the Dickson
-// window of 2^38 j 12.7 -> 7.8, the Euler n = 17 windows of 5e14 and 2e16
-// 42.2 -> 32.2 and 795 -> 627, the 13# line's quarter 19.3 -> 15.5.
+// What bounds it, and what this shape measured (B200, kernel ms): the
+// kernel issues instructions (65-75% of the slots), in the sparse windows
+// the pattern loads' shared-memory wavefronts, two a load.  Against 64-bit
+// Barrett tests with a queue drained at every block's end and a CTA barrier
+// after every eight blocks: 256 mixed intervals 204 -> 112 ms, the Dickson
+// window of 2^38 j 12.7 -> 6.9, the Euler n = 17 windows of 5e14 and 2e16
+// 42.2 -> 23.9 and 795 -> 483, the 13# line's quarter 19.3 -> 13.5.
 #pragma once
 #include "fk_arith.cuh"
 #include "fk_types.h"
@@ -78,14 +77,16 @@ __device__ __forceinline__ u32 block_scan(u32 v, u32* s_warp, u32* total) {
 }
 
 // The base of every (item, prime) of sieve items: X0 mod q for the primes
-// sieved by pattern or mark, X0 * c1 mod q for those tested per candidate
-// (the rounds' from their first cut, the marking sieve's past NPm).
+// the marking sieve sweeps, else X0 * c1 mod q with the constants the prime
+// is used with -- the rounds' pattern index up to their first cut, the
+// per-candidate test past it (and past NPm for the marking sieve).
 __device__ __forceinline__ u32 base_residue(const DevEngine& e,
                                             const DevItem& it, u32 i) {
   const PrimeRec pr = e.recs[i];
   const u32 x = fk_bmod128(it.X0_lo, it.X0_hi, pr.q, pr.magic, e.c64[i]);
-  const u32 first = it.marked ? e.NPm : e.rounds[0];
-  return i < first ? x : fk_mulmod(x, e.trec[i].c1, pr.q, pr.magic);
+  if (it.marked && i < e.NPm) return x;
+  const bool pattern = !it.marked && i < e.rounds[0];
+  return fk_mulmod(x, pattern ? e.prec[i].c1 : e.trec[i].c1, pr.q, pr.magic);
 }
 
 // ---- per-candidate kill tests ------------------------------------------
@@ -96,7 +97,6 @@ struct TestCtx {
   const ListFilter* filt;
   const u32* kq;        // this item's X0 * c1 mod q
   const u32* lists;
-  const u32* sbits;     // Euler: bitset of {x^2 + x : x < n}
   u32 n, xxmax, xxwords, ap_div;
 };
 
@@ -118,10 +118,11 @@ __device__ __forceinline__ bool list_kill(const ListFilter& f, u32 r,
   return k;
 }
 
-// Does prime i kill a value of scaled residue r (Euler, AP)?
+// Does prime i kill a value of scaled residue r (Euler, AP)?  sbits (shared
+// memory): Euler's bitset of {x^2 + x : x < n}.
 template <int KIND>
-__device__ __forceinline__ bool kill_test(const TestCtx& c, u32 i,
-                                          const TestRec& t, u32 r) {
+__device__ __forceinline__ bool kill_test(const TestCtx& c, const u32* sbits,
+                                          u32 i, const TestRec& t, u32 r) {
   bool kill;
   if (KIND == KIND_AP) {
     kill = r < c.n;
@@ -129,11 +130,11 @@ __device__ __forceinline__ bool kill_test(const TestCtx& c, u32 i,
   } else {
     // r = -x is killed when it is one of the x^2 + x: the bitset's last
     // word (xxwords) is zero
-    kill = (c.sbits[min(r >> 5, c.xxwords)] >> (r & 31)) & 1u;
+    kill = (sbits[min(r >> 5, c.xxwords)] >> (r & 31)) & 1u;
     // the primes up to max(x^2 + x): so are r + q, r + 2q, ...
     if (t.q <= c.xxmax)
       for (u32 s = r + t.q; s <= c.xxmax; s += t.q)
-        kill |= (c.sbits[s >> 5] >> (s & 31)) & 1u;
+        kill |= (sbits[s >> 5] >> (s & 31)) & 1u;
   }
   return kill;
 }
@@ -160,108 +161,88 @@ struct Prime {
     k = __ldg(c.kq + p);
     if (KIND == KIND_DICKSON) f = load_filt(c.filt + p);
   }
-  __device__ __forceinline__ bool kills(const TestCtx& c, u32 vl,
-                                        u32 vh) const {
+  // the same from the tables staged in shared memory, for prime first + j
+  __device__ __forceinline__ void load(const TestCtx& c, const TestRec* srec,
+                                       const u32* skq, u32 first, u32 j) {
+    i = first + j;
+    t = srec[j];
+    k = skq[j];
+    if (KIND == KIND_DICKSON) f = load_filt(c.filt + i);
+  }
+  __device__ __forceinline__ bool kills(const TestCtx& c, const u32* sbits,
+                                        u32 vl, u32 vh) const {
     const u32 r = redc_residue(t, k, vl, vh);
     if (KIND == KIND_DICKSON) return list_kill(f, min(r, t.q - r), c.lists);
-    return kill_test<KIND>(c, i, t, r);
+    return kill_test<KIND>(c, sbits, i, t, r);
   }
 };
 
 // ---- S1 helpers, unrolled over the compile-time pattern primes ----------
-// k[I] is the lane's current TABLE INDEX for pattern prime I (entry k =
-// phase 64k mod q), so one word forward is k + 1 and STRIDE words forward
-// is k + STRIDE (mod q).
+// Padding of a variant's pattern tables: entry q + i repeats entry i, so a
+// group of G threads on consecutive words reads one run of entries from its
+// base index with no wrap inside it.  (With the wrap taken per thread, a
+// run that crossed the table's end touched banks twice: 2.45 wavefronts a
+// load against 2.)  64 also covers the second word of a step; the variants
+// of more primes keep 32 and step twice, to leave room for three CTAs.
+template <int NS>
+constexpr u32 kPad = NS <= 24 ? kPadWide : kPadNarrow;
+
+// k[I] is the table index of the GROUP's first word for pattern prime I
+// (entry k = phase 64k mod q), the same in all its threads: one word forward
+// is k + 1 and STRIDE words forward is k + STRIDE (mod q).
 template <int P0, int I, int NS>
 struct Pat {
   // Two words of the chain, STRIDE words apart, each OR-ed into two
   // accumulators by prime parity, so the loads and ORs of one prime do not
   // wait on the previous prime's; the index then moves 2 * STRIDE words.
+  // pt: the tables, advanced by the thread's place in its group.
   template <u32 STRIDE>
-  static __device__ __forceinline__ void word2(const u64* __restrict__ spat,
+  static __device__ __forceinline__ void word2(const u64* __restrict__ pt,
                                                u32* k, u64* acc) {
     constexpr u32 q = fk_nth_prime(P0 + I);
-    constexpr u32 off = fk_pat_prefix(P0, I);
-    constexpr u32 st = STRIDE % q;
+    constexpr u32 off = fk_pat_prefix(P0, I, kPad<NS>);
+    constexpr bool once = 2 * STRIDE <= kPad<NS>;
+    constexpr u32 st = (once ? 2 * STRIDE : STRIDE) % q;
     const u32 r0 = k[I];
     u32 r1 = r0 + st;
     r1 = min(r1, r1 - q);  // unsigned: r1 - q wraps when r1 < q
-    u32 r2 = r1 + st;
-    r2 = min(r2, r2 - q);
-    acc[I & 1] |= spat[off + r0];
-    acc[2 + (I & 1)] |= spat[off + r1];
-    k[I] = r2;
-    Pat<P0, I + 1, NS>::template word2<STRIDE>(spat, k, acc);
-  }
-  // The table index of period u0 of lane R: phase (u0 + s_l) mod q with
-  // s_l = (X0 + R) * (M mod q)^-1, times 64^-1 (s_minv already carries it).
-  static __device__ __forceinline__ void setup(u32* k, u64 R, u64 u0,
-                                               const u32* __restrict__ xq,
-                                               const u32* s_minv) {
-    constexpr u32 q = fk_nth_prime(P0 + I);
-    constexpr u32 i64 = fk_inv64(q);
-    const u32 rq = (u32)(R % q);
-    const u32 s = (u32)(((xq[I] + rq) % q) * (u64)s_minv[I] % q);
-    k[I] = (u32)(((u32)(u0 % q) * i64 + s) % q);
-    Pat<P0, I + 1, NS>::setup(k, R, u0, xq, s_minv);
-  }
-  // The table indexes of a group of GW threads sweeping one lane, thread
-  // t of the group from word base + t: (base_I + t) mod q, base_I held in
-  // v[I / GW] by thread I mod GW of the group.
-  template <int GW>
-  static __device__ __forceinline__ void spread(u32* k, const u32* v,
-                                                u32 t) {
-    constexpr u32 q = fk_nth_prime(P0 + I);
-    const u32 b = __shfl_sync(0xffffffffu, v[I / GW], I % GW, GW);
-    // t < GW: below q for every prime when GW = 8 and from the 37 up when
-    // GW = 32; the 17 ... 31 of the 13# and 17# families reduce it first,
-    // so one subtraction still ends in [0, q)
-    const u32 r = b + (q >= (u32)GW ? t : t % q);
-    k[I] = min(r, r - q);
-    Pat<P0, I + 1, NS>::template spread<GW>(k, v, t);
+    acc[I & 1] |= pt[off + r0];
+    if (once) {
+      acc[2 + (I & 1)] |= pt[off + r0 + STRIDE];
+      k[I] = r1;
+    } else {
+      acc[2 + (I & 1)] |= pt[off + r1];
+      r1 += st;
+      k[I] = min(r1, r1 - q);
+    }
+    Pat<P0, I + 1, NS>::template word2<STRIDE>(pt, k, acc);
   }
 };
 template <int P0, int NS>
 struct Pat<P0, NS, NS> {
   template <u32 STRIDE>
   static __device__ __forceinline__ void word2(const u64*, u32*, u64*) {}
-  static __device__ __forceinline__ void setup(u32*, u64, u64, const u32*,
-                                               const u32*) {}
-  template <int GW>
-  static __device__ __forceinline__ void spread(u32*, const u32*, u32) {}
 };
 
-// Pattern prime I's table index at word wb of lane R: (wb + s) mod q with
-// s = (X0 + R) * (M mod q)^-1 * 64^-1 mod q the lane's phase (xq holds X0
-// mod q, s_minv the product of the two inverses), from the prime's record.
-__device__ __forceinline__ u32 lane_base(const DevEngine& e,
-                                         const u32* __restrict__ xq,
-                                         const u32* s_minv, u64 R, u64 wb,
-                                         u32 I) {
-  const PrimeRec pr = e.recs[I];
-  u32 x = xq[I] + fk_bmod(R, pr.q, pr.magic);
-  x = min(x, x - pr.q);
-  const u32 s = fk_mulmod(x, s_minv[I], pr.q, pr.magic);
-  const u32 t = s + fk_bmod(wb, pr.q, pr.magic);
-  return min(t, t - pr.q);
-}
-
-// The table indexes of a group of GW threads sweeping one lane from word
-// wb, thread t at word wb + t: thread t computes the base index of the
-// pattern primes t, t + GW, ... and the group shares them by shuffle.
-template <int P0, int NS, int GW>
-__device__ __forceinline__ void shared_setup(u32* rho, const DevEngine& e,
-                                             const u32* __restrict__ xq,
-                                             const u32* s_minv, u64 R,
-                                             u64 wb, u32 t) {
+// The table indexes of a group of GW threads sweeping lane R from word w0
+// (the line offset v = 64 * M * w0 + R): (X0 + v) / (64 * M) mod q, one
+// scaled residue each.  Thread t of the group (t) computes the pattern
+// primes t, t + GW, ... and the group shares them by shuffle.
+template <int NS, int GW>
+__device__ __forceinline__ void shared_setup(u32* rho, const TestRec* prec,
+                                             const u32* pk, u64 v, u32 t) {
   constexpr int K = (NS + GW - 1) / GW;
-  u32 v[K];
+  const u32 vl = (u32)v & ((1u << kRedcSplit) - 1u);
+  const u32 vh = (u32)(v >> kRedcSplit);
+  u32 x[K];
 #pragma unroll
   for (int j = 0; j < K; ++j) {
-    const u32 I = t + (u32)(j * GW);
-    v[j] = I < (u32)NS ? lane_base(e, xq, s_minv, R, wb, I) : 0u;
+    const u32 i = min(t + (u32)(j * GW), (u32)NS - 1);
+    x[j] = redc_residue(prec[i], pk[i], vl, vh);
   }
-  Pat<P0, 0, NS>::template spread<GW>(rho, v, t);
+#pragma unroll
+  for (int i = 0; i < NS; ++i)
+    rho[i] = GW == 1 ? x[i] : __shfl_sync(0xffffffffu, x[i / GW], i % GW, GW);
 }
 
 struct SieveArgs {
@@ -277,29 +258,12 @@ struct SieveArgs {
   u32* cand_item;
   u64 cand_cap;
   DevCounters* ctr;
-  unsigned long long* task_ctr;
+  unsigned long long* task_ctr;   // marking: next task
+  unsigned long long* block_ctr;  // rounds: [nitems] blocks claimed per item
   u32 warp_queue;     // compaction: warp queues below this go one
                       // candidate per warp
   u32 seg_per_task;   // marking: segments per task
 };
-
-// The entry of the item holding task t: the last i with task_prefix[i] <=
-// t, searched forward from `from` (a CTA's claims only grow, so its next
-// task's item is at or after its last one): a few steps, then bisection.
-__device__ __forceinline__ u32 task_item(const SieveArgs& a, u64 t, u32 from) {
-  u32 lo = from;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    if (lo + 1 < a.nitems && a.task_prefix[lo + 1] <= t) ++lo;
-    else return lo;
-  }
-  u32 hi = a.nitems;
-  while (hi - lo > 1) {
-    const u32 mid = (lo + hi) >> 1;
-    if (a.task_prefix[mid] <= t) lo = mid; else hi = mid;
-  }
-  return lo;
-}
 
 // Per-warp candidate queues of line offsets v = u * M + R.  A queue
 // outlives its warp's blocks and tasks: it is drained when it is full and
@@ -309,45 +273,103 @@ __device__ __forceinline__ u32 task_item(const SieveArgs& a, u64 t, u32 from) {
 // are turned into offsets a row at a time, when one is full or the block
 // ends.
 constexpr u32 kWarps = kBlock / 32;
-constexpr u32 kWq = 384;
+constexpr u32 kWq = 192;
+constexpr u32 kWq2 = 64;
 constexpr u32 kColSlots = 16;
+
+// What a block needs of its item and engine, read from shared memory where
+// it is used: held in registers these values would be spilled around the
+// calls below, and local memory of 768 threads an SM does not fit in L1.
+struct BlockCtx {
+  u64 U, M, lo_off, hi_last, nchain;
+  const u64* lanes;
+  u64 nblock;
+  unsigned long long* next;  // the item's counter of claimed blocks
+  u32 L, Tc, G, run, gitem;
+};
 
 struct SieveSmem {
   u64 queue[kWarps * kWq];
-  unsigned short col[kWarps * kColSlots * 32];
+  u64 queue2[kWarps * kWq2];  // past the staged primes
+  u64 chain_R[kBlock];    // each thread's chain: its lane and first word
+  u64 ntest[kWarps], nword[kWarps];  // work since the last report
   // the first kStaged test primes: every drain starts on these, and a
   // shared load answers in a tenth of the time of one from L2
   TestRec srec[kStaged];
+  TestRec prec[kNSMax];   // pattern primes: the scale of their table index
+  BlockCtx blk;
+  TestCtx ctx;            // the current item's tests
+  const u32* rounds;
+  u32 entry;              // the item joined
   u32 skq[kStaged];
   u32 sboff[kStaged];     // Dickson: the prime's first word in sbit
   u32 sbit[kStagedBits];  // bit h: min(r, q - r) = h is killed
-  TestCtx ctx;            // the current item's tests
-  const u32* rounds;
-  u32 NP, kind, deep;
-  u32 wnext[2];           // next warp block of the current / next CTA task
-  u64 task[2];
-  u32 item[2];
-  u32 minv[kNSMax];
+  u32 chain_w0[kBlock];
+  u32 qn[kWarps], qn2[kWarps];  // queue lengths
+  u32 pk[kNSMax];
   u32 sbits[kSbits + 1];
+  u32 NP, kind, deep;
   u32 eng;
   u32 status;
   unsigned long long mbar;
+  unsigned short col[kWarps * kColSlots * 32];
 };
+
+// The rounds kernel's shared memory: SieveSmem first, then the pattern
+// tables, so a function called out of line finds it at a known shared
+// address (through a pointer argument its accesses would be generic loads
+// with 64-bit address arithmetic: twice the instructions of a test).
+constexpr u32 kSieveSmemBytes = (sizeof(SieveSmem) + 127) / 128 * 128;
+
+__device__ __forceinline__ SieveSmem& sieve_smem_ref() {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  return *reinterpret_cast<SieveSmem*>(smem_raw);
+}
 
 // Shared bytes of the first NS pattern primes' tables (the prefix a kernel
 // variant stages), padded to 16 bytes.
-template <int P0, int NS = kNS>
+template <int P0, int NS = kNS, u32 PAD = 0>
 __host__ __device__ constexpr u32 pat_bytes() {
-  return ((fk_pat_prefix(P0, NS) + 1) / 2) * 16;
+  return ((fk_pat_prefix(P0, NS, PAD) + 1) / 2) * 16;
 }
 
-// A warp's n candidates against the primes [at, end), 32 at a time: each
-// lane holds one prime, every candidate is tested against all of them at
-// once and the survivors are compacted in place; the next 32 primes' loads
-// are in flight meanwhile.  Returns the survivors' count.
+// A warp's n candidates against the 32 primes its lanes hold: the survivors
+// compacted in place, their count returned.
+template <int KIND>
+__device__ __forceinline__ u32 test_group(u64* Q, u32 n, const TestCtx& c,
+                                          const u32* sbits,
+                                          const Prime<KIND>& p) {
+  const u32 lane = threadIdx.x & 31;
+  u32 out = 0;
+  for (u32 idx = 0; idx < n; idx += 2) {
+    const bool two = idx + 1 < n;
+    const u64 v = Q[idx], w = Q[two ? idx + 1 : idx];
+    const u32 vl = (u32)v & ((1u << kRedcSplit) - 1u);
+    const u32 vh = (u32)(v >> kRedcSplit);
+    const u32 wl = (u32)w & ((1u << kRedcSplit) - 1u);
+    const u32 wh = (u32)(w >> kRedcSplit);
+    const bool kv = p.kills(c, sbits, vl, vh), kw = p.kills(c, sbits, wl, wh);
+    const bool dv = __any_sync(0xffffffffu, kv);
+    const bool dw = __any_sync(0xffffffffu, kw) || !two;
+    if (!dv) {
+      if (lane == 0) Q[out] = v;  // out <= idx: read already
+      ++out;
+    }
+    if (!dw) {
+      if (lane == 0) Q[out] = w;
+      ++out;
+    }
+  }
+  __syncwarp();
+  return out;
+}
+
+// A warp's n candidates against the primes [at, end), 32 at a time, the
+// next 32 primes' loads in flight meanwhile.  Returns the survivors' count.
 template <int KIND>
 __device__ __forceinline__ u32 drain_groups(u64* Q, u32 n, const TestCtx& c,
-                                            u32 at, u32 end, u32& ntest) {
+                                            const u32* sbits, u32 at, u32 end,
+                                            u32& ntest) {
   const u32 lane = threadIdx.x & 31;
   if (n == 0 || at >= end) return n;
   Prime<KIND> p, next;
@@ -355,99 +377,29 @@ __device__ __forceinline__ u32 drain_groups(u64* Q, u32 n, const TestCtx& c,
   for (;;) {
     at += 32;
     next.load(c, min(at + lane, end - 1));
-    u32 out = 0;
-    for (u32 idx = 0; idx < n; idx += 2) {
-      const bool two = idx + 1 < n;
-      const u64 v = Q[idx], w = Q[two ? idx + 1 : idx];
-      const u32 vl = (u32)v & ((1u << kRedcSplit) - 1u);
-      const u32 vh = (u32)(v >> kRedcSplit);
-      const u32 wl = (u32)w & ((1u << kRedcSplit) - 1u);
-      const u32 wh = (u32)(w >> kRedcSplit);
-      const bool kv = p.kills(c, vl, vh), kw = p.kills(c, wl, wh);
-      const bool dv = __any_sync(0xffffffffu, kv);
-      const bool dw = __any_sync(0xffffffffu, kw) || !two;
-      if (!dv) {
-        if (lane == 0) Q[out] = v;  // out <= idx: read already
-        ++out;
-      }
-      if (!dw) {
-        if (lane == 0) Q[out] = w;
-        ++out;
-      }
-    }
     ntest += n;
-    __syncwarp();
-    n = out;
+    n = test_group<KIND>(Q, n, c, sbits, p);
     if (at >= end || n == 0) return n;
     p = next;
   }
 }
 
-// Drain one warp's queue of n candidates in place.  Over the first primes
-// past the pattern (the staged ones, which kill most): rounds with one
-// candidate per lane, the survivors compacted by ballot after each.  Once
-// fewer than a.warp_queue are left, or the staged primes are done, the
-// candidates share the warp instead: each lane holds one prime and every
-// candidate is tested against the warp's 32 primes at once, so no lane
-// idles behind a dead candidate and the records of 32 primes are loaded
-// (one group ahead) once for all of them.  The survivors go to the global
-// list.  Warp-synchronous: every lane calls it with the same n.  Returns
-// the lane's prime tests.  Not inlined: the pattern loop around it keeps
-// its NS table indexes in registers and runs between drains.
+// A warp's n candidates (its first or second queue) against every prime
+// from index `at` on, in place, and the survivors into the global list: 32 primes at a time, then, once
+// few candidates die among 128 primes (S.deep), kDeep groups of 32 at a
+// time (fewer votes, more loads in flight).
 template <int KIND>
-__device__ __noinline__ u32 warp_drain(u64* Q, u32 n, const SieveSmem& S,
-                                       u32 gitem, u32 wq_short, u64* cand_key,
-                                       u32* cand_item, u64 cand_cap,
-                                       DevCounters* ctr) {
-  const u32 lane = threadIdx.x & 31;
-  const u32 lt = (1u << lane) - 1u;
+__device__ __noinline__ void drain_rest(bool second, u32 n, u32 at,
+                                        u64* cand_key, u32* cand_item,
+                                        u64 cand_cap, DevCounters* ctr) {
+  SieveSmem& S = sieve_smem_ref();
+  const u32 lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  u64* Q = second ? S.queue2 + wid * kWq2 : S.queue + wid * kWq;
   const TestCtx c = S.ctx;
-  const u32 NP = S.NP, first = __ldg(S.rounds);
-  const u32 nstaged = min(kStaged, NP - first);
-  u32 ntest = 0, at = 0;
-  for (u32 r = 0; n >= wq_short && n > 0 && at < nstaged; ++r) {
-    // a round's cut, rounded up to whole trips (testing past it is no
-    // mistake, and past the last prime the tables repeat it)
-    const u32 i0 = at;
-    at = min((__ldg(S.rounds + r + 1) - first + kRoundUnroll - 1) /
-                 kRoundUnroll * kRoundUnroll, (u32)kStaged);
-    u32 out = 0;
-    for (u32 base = 0; base < n; base += 32) {
-      const u32 idx = base + lane;
-      bool alive = idx < n;
-      const u64 v = alive ? Q[idx] : 0;
-      const u32 vl = (u32)v & ((1u << kRedcSplit) - 1u);
-      const u32 vh = (u32)(v >> kRedcSplit);
-      // a dead lane idles until the chunk's last candidate dies
-      for (u32 i = i0; i < at && __any_sync(0xffffffffu, alive);
-           i += kRoundUnroll) {
-        if (alive) ntest += kRoundUnroll;
-        bool kill = false;
-#pragma unroll
-        for (u32 j = 0; j < kRoundUnroll; ++j) {
-          const TestRec t = S.srec[i + j];
-          const u32 q = redc_residue(t, S.skq[i + j], vl, vh);
-          if (KIND == KIND_DICKSON) {
-            const u32 h = min(q, t.q - q);
-            kill |= (S.sbit[S.sboff[i + j] + (h >> 5)] >> (h & 31)) & 1u;
-          } else {
-            kill |= kill_test<KIND>(c, first + i + j, t, q);
-          }
-        }
-        alive = alive && !kill;
-      }
-      const u32 bal = __ballot_sync(0xffffffffu, alive);
-      if (alive) Q[out + __popc(bal & lt)] = v;  // out <= base: read already
-      out += __popc(bal);
-    }
-    __syncwarp();
-    n = out;
-  }
-  at = min(first + at, NP);
+  const u32 NP = S.NP;
+  u32 ntest = 0;
   const u32 deep = min(max(S.deep, at), NP);
-  n = drain_groups<KIND>(Q, n, c, at, deep, ntest);
-  // kDeep groups at a time: fewer votes and more loads in flight, once few
-  // candidates die among 128 primes
+  n = drain_groups<KIND>(Q, n, c, S.sbits, at, deep, ntest);
   constexpr u32 kDeep = KIND == KIND_DICKSON ? 2 : 4;
   at = deep;
   for (; n > 0 && at + 32 * kDeep <= NP; at += 32 * kDeep) {
@@ -461,7 +413,7 @@ __device__ __noinline__ u32 warp_drain(u64* Q, u32 n, const SieveSmem& S,
       const u32 vh = (u32)(v >> kRedcSplit);
       bool kill = false;
 #pragma unroll
-      for (u32 j = 0; j < kDeep; ++j) kill |= p[j].kills(c, vl, vh);
+      for (u32 j = 0; j < kDeep; ++j) kill |= p[j].kills(c, S.sbits, vl, vh);
       if (!__any_sync(0xffffffffu, kill)) {
         if (lane == 0) Q[out] = v;  // out <= idx: read already
         ++out;
@@ -471,7 +423,7 @@ __device__ __noinline__ u32 warp_drain(u64* Q, u32 n, const SieveSmem& S,
     __syncwarp();
     n = out;
   }
-  n = drain_groups<KIND>(Q, n, c, at, NP, ntest);
+  n = drain_groups<KIND>(Q, n, c, S.sbits, at, NP, ntest);
   // survivors: one atomic per warp
   if (n) {
     u64 base = 0;
@@ -480,28 +432,132 @@ __device__ __noinline__ u32 warp_drain(u64* Q, u32 n, const SieveSmem& S,
     for (u32 idx = lane; idx < n; idx += 32) {
       if (base + idx < cand_cap) {
         cand_key[base + idx] = Q[idx];
-        cand_item[base + idx] = gitem;
+        cand_item[base + idx] = S.blk.gitem;
       } else {
         atomicOr(&ctr->overflow, 1u);
       }
     }
   }
+  ntest = __reduce_add_sync(0xffffffffu, ntest);
+  if (lane == 0) S.ntest[wid] += ntest;
   __syncwarp();
-  return ntest;
 }
 
-__device__ __forceinline__ u32 drain_any(u64* Q, u32 n, const SieveSmem& S,
-                                         u32 gitem, const SieveArgs& a) {
-  if (n == 0) return 0;
+// Drain one warp's queue.  Over the staged primes (the first past the
+// pattern, which kill most): rounds with one candidate per lane, the
+// survivors compacted in place by ballot after each, down to a.warp_queue
+// of them; then one prime per lane.  Those left gather in the warp's
+// second queue, until enough of them share the loads of the
+// deeper primes' records: there each lane holds one prime and every
+// candidate is tested against the warp's 32 primes at once, so no lane
+// idles behind a dead candidate.  `final` (the item's end) empties both
+// queues; a first queue shorter than a.warp_queue then skips the rounds.
+// Warp-synchronous: every lane calls it.  Not inlined: the pattern loop
+// around it keeps its NS table indexes in registers and runs between
+// drains.
+template <int KIND>
+__device__ __noinline__ void warp_drain(bool final, u32 wq_short, u64* cand_key,
+                                        u32* cand_item, u64 cand_cap,
+                                        DevCounters* ctr) {
+  SieveSmem& S = sieve_smem_ref();
+  const u32 lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const u32 lt = (1u << lane) - 1u;
+  u64* Q = S.queue + wid * kWq;
+  u64* Q2 = S.queue2 + wid * kWq2;
+  u32 n = S.qn[wid], n2 = S.qn2[wid];
+  const u32 NP = S.NP, first = __ldg(S.rounds);
+  const u32 nstaged = min((u32)kStaged, NP - first);
+  u32 from = first;
+  if (n > 0 && (!final || n >= wq_short)) {
+    const TestCtx c = S.ctx;
+    u32 ntest = 0, at = 0;
+    for (u32 r = 0; n >= wq_short && n > 0 && at < nstaged; ++r) {
+      // a round's cut, rounded up to whole trips (testing past it is no
+      // mistake, and past the last prime the tables repeat it)
+      const u32 i0 = at;
+      at = min((__ldg(S.rounds + r + 1) - first + kRoundUnroll - 1) /
+                   kRoundUnroll * kRoundUnroll, (u32)kStaged);
+      u32 out = 0;
+      for (u32 base = 0; base < n; base += 32) {
+        const u32 idx = base + lane;
+        bool alive = idx < n;
+        const u64 v = alive ? Q[idx] : 0;
+        const u32 vl = (u32)v & ((1u << kRedcSplit) - 1u);
+        const u32 vh = (u32)(v >> kRedcSplit);
+        // a dead lane idles until the chunk's last candidate dies
+        for (u32 i = i0; i < at && __any_sync(0xffffffffu, alive);
+             i += kRoundUnroll) {
+          if (alive) ntest += kRoundUnroll;
+          bool kill = false;
+#pragma unroll
+          for (u32 j = 0; j < kRoundUnroll; ++j) {
+            const TestRec t = S.srec[i + j];
+            const u32 q = redc_residue(t, S.skq[i + j], vl, vh);
+            if (KIND == KIND_DICKSON) {
+              const u32 h = min(q, t.q - q);
+              kill |= (S.sbit[S.sboff[i + j] + (h >> 5)] >> (h & 31)) & 1u;
+            } else {
+              kill |= kill_test<KIND>(c, S.sbits, first + i + j, t, q);
+            }
+          }
+          alive = alive && !kill;
+        }
+        const u32 bal = __ballot_sync(0xffffffffu, alive);
+        if (alive) Q[out + __popc(bal & lt)] = v;  // out <= base: read already
+        out += __popc(bal);
+      }
+      __syncwarp();
+      n = out;
+    }
+    // too few to fill the lanes: one staged prime per lane instead
+    for (; n > 0 && at < nstaged; at += 32) {
+      Prime<KIND> p;
+      p.load(c, S.srec, S.skq, first, min(at + lane, nstaged - 1));
+      ntest += n;
+      n = test_group<KIND>(Q, n, c, S.sbits, p);
+    }
+    ntest = __reduce_add_sync(0xffffffffu, ntest);
+    if (lane == 0) S.ntest[wid] += ntest;
+    from = first + nstaged;
+  }
+  if (n >= kWq2 / 2) {   // enough by themselves
+    drain_rest<KIND>(false, n, from, cand_key, cand_item, cand_cap, ctr);
+    n = 0;
+  }
+  if (n2 + n > kWq2) {
+    drain_rest<KIND>(true, n2, first + nstaged, cand_key, cand_item, cand_cap,
+                     ctr);
+    n2 = 0;
+  }
+  if (lane < n) Q2[n2 + lane] = Q[lane];  // n < kWq2 / 2 = 32
+  __syncwarp();
+  n2 += n;
+  if (final && n2 > 0) {
+    drain_rest<KIND>(true, n2, n > 0 ? from : first + nstaged, cand_key,
+                     cand_item, cand_cap, ctr);
+    n2 = 0;
+  }
+  if (lane == 0) {
+    S.qn[wid] = 0;
+    S.qn2[wid] = n2;
+  }
+  __syncwarp();
+}
+
+static_assert(kWq2 / 2 <= 32, "a lane appends one candidate");
+
+__device__ __forceinline__ void drain_any(SieveSmem& S, bool final,
+                                          const SieveArgs& a) {
+  if ((S.qn[threadIdx.x >> 5] | S.qn2[threadIdx.x >> 5]) == 0) return;
   switch (S.kind) {
     case KIND_EULER:
-      return warp_drain<KIND_EULER>(Q, n, S, gitem, a.warp_queue, a.cand_key,
+      return warp_drain<KIND_EULER>(final, a.warp_queue, a.cand_key,
                                     a.cand_item, a.cand_cap, a.ctr);
     case KIND_DICKSON:
-      return warp_drain<KIND_DICKSON>(Q, n, S, gitem, a.warp_queue, a.cand_key,
+      return warp_drain<KIND_DICKSON>(final, a.warp_queue, a.cand_key,
                                       a.cand_item, a.cand_cap, a.ctr);
     default:
-      return warp_drain<KIND_AP>(Q, n, S, gitem, a.warp_queue, a.cand_key,
+      return warp_drain<KIND_AP>(final, a.warp_queue, a.cand_key,
                                  a.cand_item, a.cand_cap, a.ctr);
   }
 }
@@ -527,8 +583,8 @@ __device__ __forceinline__ bool mbar_wait(u32 mb, u32 phase, u32 spins) {
 // copy to land: the CTA then exits, and a copy still writing into the
 // shared memory of an exited CTA is what the second wait avoids.  Every
 // thread of the CTA calls it.
-template <int P0, int NS>
-__device__ __forceinline__ bool stage_patterns(u64* spat, const DevEngine& eg,
+template <u32 BYTES>
+__device__ __forceinline__ bool stage_patterns(u64* spat, const void* pat,
                                                unsigned long long* mbar,
                                                u32* status, u32& phase,
                                                DevCounters* ctr) {
@@ -536,7 +592,7 @@ __device__ __forceinline__ bool stage_patterns(u64* spat, const DevEngine& eg,
   if (threadIdx.x == 0) {
     *status = 0;
     const u32 mb = smem_u32(mbar);
-    const u32 bytes = pat_bytes<P0, NS>();
+    const u32 bytes = BYTES;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile(
         "mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb),
@@ -545,7 +601,7 @@ __device__ __forceinline__ bool stage_patterns(u64* spat, const DevEngine& eg,
     asm volatile(
         "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes"
         " [%0], [%1], %2, [%3];" ::"r"(smem_u32(spat)),
-        "l"((u64)__cvta_generic_to_global(eg.pat)), "r"(bytes), "r"(mb)
+        "l"((u64)__cvta_generic_to_global(pat)), "r"(bytes), "r"(mb)
         : "memory");
     if (!mbar_wait(mb, phase, kWaitSpins)) {
       *status = 1;
@@ -559,31 +615,29 @@ __device__ __forceinline__ bool stage_patterns(u64* spat, const DevEngine& eg,
 }
 
 // Move a warp's columns (cn codes in this thread's) into its queue, which
-// holds qn entries and is drained when a row may not fit.  The thread's
-// chain: lane R, words w0, w0 + G, ...  Returns the queue's new length and
-// adds the lane's prime tests to ntest.  Not inlined, as warp_drain.
-static __device__ __noinline__ u32 flush_columns(const SieveSmem& S, u64* Q,
-                                          const unsigned short* C, u32 qn,
-                                          u32 cn, u64 R, u64 M, u32 w0, u32 G,
-                                          u32 gitem, const SieveArgs& a,
-                                          u32* ntest) {
-  const u32 wl = threadIdx.x & 31;
+// is drained when a row may not fit.  Not inlined, as warp_drain.
+static __device__ __noinline__ void flush_columns(u32 cn, const SieveArgs& a) {
+  SieveSmem& S = sieve_smem_ref();
+  const u32 wl = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const unsigned short* C = S.col + wid * (kColSlots * 32) + wl;
   const u32 rows = __reduce_max_sync(0xffffffffu, cn);
   for (u32 r = 0; r < rows; ++r) {
     const u32 bal = __ballot_sync(0xffffffffu, r < cn);
+    u32 qn = S.qn[wid];
     if (qn + 32 > kWq) {
-      *ntest += drain_any(Q, qn, S, gitem, a);
+      drain_any(S, false, a);
       qn = 0;
     }
     if (r < cn) {
       const u32 code = C[32 * r];
-      const u64 u = 64ull * (w0 + (code >> 6) * G) + (code & 63u);
-      Q[qn + __popc(bal & ((1u << wl) - 1u))] = u * M + R;
+      const u64 u = 64ull * (S.chain_w0[threadIdx.x] + (code >> 6) * S.blk.G) +
+                    (code & 63u);
+      S.queue[wid * kWq + qn + __popc(bal & ((1u << wl) - 1u))] =
+          u * S.blk.M + S.chain_R[threadIdx.x];
     }
-    qn += __popc(bal);
+    if (wl == 0) S.qn[wid] = qn + __popc(bal);
+    __syncwarp();
   }
-  __syncwarp();
-  return qn;
 }
 
 // Push the set bits of one 32-bit half word into the thread's column while
@@ -598,122 +652,148 @@ __device__ __forceinline__ void push_half(u32& x, u32 code, unsigned short* C,
   }
 }
 
+// The periods of word w the item covers, of which R's are admitted: all 64
+// except in the item's first word (lo_off) and its last (U, hi_last).
+__device__ __forceinline__ u64 word_mask(const BlockCtx& c, u32 w, u64 R) {
+  if (64ull * w >= c.U) return 0;
+  const u64 left = c.U - 64ull * w;
+  u64 m = left >= 64 ? ~0ull : (1ull << left) - 1ull;
+  if (w == 0 && R < c.lo_off) m &= ~1ull;
+  if (left <= 64 && R >= c.hi_last) m &= ~(1ull << (left - 1));
+  return m;
+}
+
 // One block of 32 threads' chains: thread wl of the warp sweeps chain
-// gw + (wl >> gsh) of the item and pushes its pattern survivors through its
-// column into the warp's queue (qn entries).
+// g = gw + (wl >> log2 G) of the item and pushes its pattern survivors
+// through its column into the warp's queue.
 template <int P0, int NS>
-__device__ __forceinline__ void sieve_block(
-    const u64* __restrict__ spat, SieveSmem& S, u64* Q, u32& qn,
-    const SieveArgs& a, const DevEngine& e, const DevItem& it, u32 gitem,
-    u64 gw, u64 nchain, u32& ntest, u32& nword) {
-  const u32 wl = threadIdx.x & 31;
-  const u32 G = it.lane_threads;
-  const u32 gsh = G == 32 ? 5u : (G == 8 ? 3u : 0u);
-  const u32 Tc = it.Tc, L = e.L;
-  const u64 U = it.U, M = e.M;
-  // ---- this thread's chain -----------------------------------------
-  const u64 g = gw + (wl >> gsh);
-  const bool active = g < nchain;
-  u32 chunk = 0, lane = 0;   // chunks per lane: below 2^30 words
-  if (active) {
-    if (nchain <= 0xFFFFFFFFull) {
-      chunk = (u32)g / L;
-      lane = (u32)g - chunk * L;
-    } else {
-      chunk = (u32)(g / L);
-      lane = (u32)(g % L);
-    }
-  }
-  const u64 R = active ? e.lanes[lane] : 0;
-  const u32 w0 = chunk * (G * Tc) + (wl & (G - 1));
-  const u32* xq = a.xq + it.xq_off;
+__device__ __forceinline__ void sieve_block(const u64* __restrict__ spat,
+                                            SieveSmem& S, const SieveArgs& a,
+                                            u64 gw) {
+  const u32 wl = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  u32 G = S.blk.G, Tc = S.blk.Tc;
+  // words of this thread's chain inside the item, and the fewest over the
+  // warp: words 1 ... least - 2 of every chain are whole
+  u32 words = 0;
   u32 rho[NS];
-  if (G == 32) {
-    // the whole warp sweeps one lane: thread I works out prime I's base
-    // index once and the warp shares it (instead of every thread
-    // computing all NS of them)
-    shared_setup<P0, NS, 32>(rho, e, xq, S.minv, R, chunk * 32ull * Tc, wl);
-  } else if (G == 8) {
-    // the same within each group of eight threads sweeping one lane
-    shared_setup<P0, NS, 8>(rho, e, xq, S.minv, R, chunk * 8ull * Tc, wl & 7u);
-  } else {
-    Pat<P0, 0, NS>::setup(rho, R, 64ull * w0, xq, S.minv);
+  {
+    const u32 gsh = G == 32 ? 5u : (G == 8 ? 3u : 0u);
+    const u32 L = S.blk.L;
+    const u64 nchain = S.blk.nchain, g = gw + (wl >> gsh);
+    u32 chunk = 0, lane = 0;   // chunks per lane: below 2^30 words
+    const bool active = g < nchain;
+    if (active) {
+      if (nchain <= 0xFFFFFFFFull) {
+        chunk = (u32)g / L;
+        lane = (u32)g - chunk * L;
+      } else {
+        chunk = (u32)(g / L);
+        lane = (u32)(g % L);
+      }
+    }
+    const u64 R = active ? S.blk.lanes[lane] : 0;
+    const u32 w0 = chunk * (G * Tc) + (wl & (G - 1));
+    const u32 wend = (u32)((S.blk.U + 63) >> 6);
+    if (active && w0 < wend) words = min(Tc, (wend - w0 + G - 1) / G);
+    S.chain_R[threadIdx.x] = R;
+    S.chain_w0[threadIdx.x] = w0;
+    // the group's first word is chunk * G * Tc
+    const u64 v0 = 64ull * S.blk.M * (chunk * (G * Tc)) + R;
+    if (G == 32)
+      shared_setup<NS, 32>(rho, S.prec, S.pk, v0, wl);
+    else if (G == 8)
+      shared_setup<NS, 8>(rho, S.prec, S.pk, v0, wl & 7u);
+    else
+      shared_setup<NS, 1>(rho, S.prec, S.pk, v0, 0);
   }
-  unsigned short* C = S.col + (threadIdx.x >> 5) * (kColSlots * 32) + wl;
+  const u32 total = __reduce_add_sync(0xffffffffu, words);
+  u32 least = __reduce_min_sync(0xffffffffu, words);
+  if (wl == 0) S.nword[wid] += total;
+  const u64* pt = spat + (wl & (G - 1));
+  unsigned short* C = S.col + wid * (kColSlots * 32) + wl;
   u32 cn = 0;
-  // words in range: below wend; words from 1 to wfull - 1 lie whole inside
-  // the item, so only the first word (lo_off) and the last (hi_last, U)
-  // need a validity mask
-  const u32 wend = (u32)((U + 63) >> 6);
-  const u32 wfull = U ? (u32)((U - 1) >> 6) : 0;
-  if (active && w0 < wend) nword += min(Tc, (wend - w0 + G - 1) / G);
   for (u32 wi = 0; wi < Tc; wi += 2) {
     // two words of the chain: j = wi and wi + 1
     u64 acc[4] = {0, 0, 0, 0};
     if (G == 32)
-      Pat<P0, 0, NS>::template word2<32>(spat, rho, acc);
+      Pat<P0, 0, NS>::template word2<32>(pt, rho, acc);
     else if (G == 8)
-      Pat<P0, 0, NS>::template word2<8>(spat, rho, acc);
+      Pat<P0, 0, NS>::template word2<8>(pt, rho, acc);
     else
-      Pat<P0, 0, NS>::template word2<1>(spat, rho, acc);
-    u64 sv[2];
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const u32 w = w0 + (wi + k) * G;
-      u64 s = ~(acc[k * 2] | acc[k * 2 + 1]);
-      if (!active || wi + k >= Tc || w >= wend) {
-        s = 0;
-      } else if (w == 0 || w >= wfull) {
-        const u64 left = U - 64ull * w;
-        if (left < 64) s &= (1ull << left) - 1ull;
-        if (w == 0 && R < it.lo_off) s &= ~1ull;
-        if (left <= 64 && R >= it.hi_last) s &= ~(1ull << (left - 1));
-      }
-      sv[k] = s;
+      Pat<P0, 0, NS>::template word2<1>(pt, rho, acc);
+    u64 s0 = ~(acc[0] | acc[1]), s1 = ~(acc[2] | acc[3]);
+    if (wi == 0 || wi + 2 >= least) {
+      const u64 R = S.chain_R[threadIdx.x];
+      const u32 w = S.chain_w0[threadIdx.x] + wi * G;
+      s0 = wi < words ? s0 & word_mask(S.blk, w, R) : 0ull;
+      s1 = wi + 1 < words ? s1 & word_mask(S.blk, w + G, R) : 0ull;
     }
     // into the columns; a full one empties the warp's
-    u32 x[4] = {(u32)sv[0], (u32)(sv[0] >> 32), (u32)sv[1],
-                (u32)(sv[1] >> 32)};
+    u32 x[4] = {(u32)s0, (u32)(s0 >> 32), (u32)s1, (u32)(s1 >> 32)};
     for (;;) {
 #pragma unroll
       for (int k = 0; k < 4; ++k) push_half(x[k], (wi << 6) + 32 * k, C, cn);
       if (!__any_sync(0xffffffffu, (x[0] | x[1] | x[2] | x[3]) != 0)) break;
-      // the table indexes wait out the flush in local memory: live across
+      // the loop's values wait out the flush in local memory: live across
       // the call they would be spilled in the word loop instead
-      volatile u32 keep[NS];
+      volatile u32 keep[NS + 9];
 #pragma unroll
       for (int i = 0; i < NS; ++i) keep[i] = rho[i];
-      qn = flush_columns(S, Q, C, qn, cn, R, M, w0, G, gitem, a, &ntest);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) keep[NS + k] = x[k];
+      keep[NS + 4] = wi;
+      keep[NS + 5] = words;
+      keep[NS + 6] = least;
+      keep[NS + 7] = Tc;
+      keep[NS + 8] = G;
+      flush_columns(cn, a);
       cn = 0;
 #pragma unroll
       for (int i = 0; i < NS; ++i) rho[i] = keep[i];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) x[k] = keep[NS + k];
+      wi = keep[NS + 4];
+      words = keep[NS + 5];
+      least = keep[NS + 6];
+      Tc = keep[NS + 7];
+      G = keep[NS + 8];
     }
   }
   // the codes refer to this block's chains
-  qn = flush_columns(S, Q, C, qn, cn, R, M, w0, G, gitem, a, &ntest);
+  flush_columns(cn, a);
 }
 
-// Claim the CTA's next task into slot p: its number and its item (entry of
-// the family's list).
-__device__ __forceinline__ void claim_task(const SieveArgs& a, SieveSmem& S,
-                                           u32 p, u32 from) {
-  const u64 t = atomicAdd(a.task_ctr, 1ull);
-  S.task[p] = t;
-  S.wnext[p] = 0;
-  S.item[p] = t < a.ntask ? task_item(a, t, from) : 0u;
+// The first entry of the family's list with blocks left, from `from` on
+// and around; nitems when none has.  Called by one whole warp.
+__device__ __forceinline__ u32 find_item(const SieveArgs& a, u32 from) {
+  const u32 wl = threadIdx.x & 31;
+  for (u32 k = 0; k < a.nitems; k += 32) {
+    u32 e = from + k + wl;
+    if (e >= a.nitems) e -= a.nitems;
+    const bool left = k + wl < a.nitems &&
+                      *(volatile unsigned long long*)(a.block_ctr + e) <
+                          a.items[a.item_index[e]].ntask;
+    const u32 bal = __ballot_sync(0xffffffffu, left);
+    if (bal) return __shfl_sync(0xffffffffu, e, __ffs((int)bal) - 1);
+  }
+  return a.nitems;
 }
 
 // NS: the pattern primes this variant stages (the engine descriptor's NS
-// and round cuts must match it).  A CTA task is it.blocks blocks of 32
-// threads' chains, claimed by the warps from the CTA's counter, so a warp
-// held up by a queue drain takes fewer of them; the next task is claimed
-// while this one runs, so a task costs one barrier.
+// and round cuts must match it).  A CTA joins an item -- stages its
+// engine's tables and its base residues -- and its warps claim runs of the
+// item's blocks from the item's counter until none is left, each at its own
+// pace; then they drain their queues and the CTA joins the next item with
+// work.  CTAs start spread over the list, so short items run side by side
+// and long ones draw every CTA in the end.  (With CTA-wide tasks the
+// barrier ending each one cost a fifth to a third of the warps' time: a
+// warp in a drain held up the other seven.)
 template <int P0, int NS>
 __global__ void __launch_bounds__(kBlock, 3)
     k_sieve(const __grid_constant__ SieveArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  u64* spat = reinterpret_cast<u64*>(smem_raw);
-  SieveSmem& S = *reinterpret_cast<SieveSmem*>(smem_raw + pat_bytes<P0, NS>());
+  SieveSmem& S = sieve_smem_ref();
+  u64* spat = reinterpret_cast<u64*>(smem_raw + kSieveSmemBytes);
   const u32 tid = threadIdx.x, wl = tid & 31, wid = tid >> 5;
   if (tid == 0) {
     S.eng = 0xFFFFFFFFu;
@@ -722,54 +802,44 @@ __global__ void __launch_bounds__(kBlock, 3)
                  : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    claim_task(a, S, 0, 0);
   }
-  __syncthreads();
+  if (wl == 0) {
+    S.qn[wid] = S.qn2[wid] = 0;
+    S.ntest[wid] = S.nword[wid] = 0;
+  }
   u32 phase = 0;
-  u64* Q = S.queue + wid * kWq;
-  u32 qn = 0, gitem = 0xFFFFFFFFu;
-  u32 ntest = 0, nword = 0;  // since the last report
-  for (u32 p = 0;; p ^= 1u) {
-    const u64 task = S.task[p];
-    const u32 entry = S.item[p];
-    const bool done = task >= a.ntask;
-    const u32 next = done ? 0xFFFFFFFFu : a.item_index[entry];
-    if (done || next != gitem) {
-      // another item, or the end (a CTA may find every task claimed before
-      // its first): drain this one's queue and report
-      ntest += drain_any(Q, qn, S, gitem, a);
-      qn = 0;
-      u64 nt = ntest, nw = nword;  // warp sums in 64 bits
-      ntest = nword = 0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        nt += __shfl_down_sync(0xffffffffu, nt, o);
-        nw += __shfl_down_sync(0xffffffffu, nw, o);
-      }
-      if (wl == 0) {
-        if (nt) atomicAdd(&a.ctr->s2_tests, (unsigned long long)nt);
-        if (nw) atomicAdd(&a.ctr->s1_words, (unsigned long long)nw);
-      }
-      if (done) break;
-      __syncthreads();   // every warp is past the old item's tables
-      gitem = next;
-      const u32 eidx = a.items[gitem].engine;
+  u32 entry = (u32)((u64)blockIdx.x * a.nitems / gridDim.x);
+  for (;;) {
+    if (wid == 0) {
+      const u32 e = find_item(a, entry);
+      if (wl == 0) S.entry = e;
+    }
+    __syncthreads();   // and every warp is past the old item's tables
+    entry = S.entry;
+    if (entry >= a.nitems) break;
+    {
+      const u32 gitem = a.item_index[entry];
+      const DevItem& it = a.items[gitem];
+      const u32 eidx = it.engine;
       const DevEngine& eg = a.engines[eidx];
       if (S.eng != eidx) {
         // ---- engine switch: stage its pattern table into shared memory ----
-        if (!stage_patterns<P0, NS>(spat, eg, &S.mbar, &S.status, phase, a.ctr))
+        if (!stage_patterns<pat_bytes<P0, NS, kPad<NS>>()>(
+                spat, kPad<NS> == kPadWide ? eg.patw : eg.patn, &S.mbar,
+                &S.status, phase, a.ctr))
           return;
-        for (u32 i = tid; i < (u32)NS; i += kBlock) S.minv[i] = eg.pat_minv[i];
+        if (tid < (u32)NS) S.prec[tid] = eg.prec[tid];
         for (u32 i = tid; i <= eg.sbits_words; i += kBlock)
           S.sbits[i] = i < eg.sbits_words ? eg.sbits[i] : 0u;
         __syncthreads();   // and every warp has read S.eng
         if (tid == 0) S.eng = eidx;
       }
+      if (tid < (u32)NS) S.pk[tid] = a.xq[it.xq_off + tid];
       const u32 first = eg.rounds[0];
       if (tid < (u32)kStaged && first < eg.NP) {
         const u32 p = min(first + tid, eg.NP - 1);  // past the end: the last
         S.srec[tid] = eg.trec[p];
-        S.skq[tid] = a.xq[a.items[gitem].xq_off + p];
+        S.skq[tid] = a.xq[it.xq_off + p];
         if (eg.kind == KIND_DICKSON)
           S.sboff[tid] = eg.boff[p - kNSMin] - eg.boff[first - kNSMin];
       }
@@ -779,9 +849,12 @@ __global__ void __launch_bounds__(kBlock, 3)
         for (u32 i = b0 + tid; i < b1; i += kBlock) S.sbit[i - b0] = eg.bits[i];
       }
       if (tid == 0) {
-        S.ctx = TestCtx{eg.trec, eg.filt, a.xq + a.items[gitem].xq_off,
-                        eg.lists, S.sbits, eg.n, eg.xxmax, eg.sbits_words,
-                        eg.ap_div};
+        S.ctx = TestCtx{eg.trec, eg.filt, a.xq + it.xq_off, eg.lists,
+                        eg.n, eg.xxmax, eg.sbits_words, eg.ap_div};
+        S.blk = BlockCtx{it.U, eg.M, it.lo_off, it.hi_last, it.nchunk * eg.L,
+                         reinterpret_cast<const u64*>(eg.lanes), it.ntask,
+                         a.block_ctr + entry, eg.L, it.Tc, it.lane_threads,
+                         it.run, gitem};
         S.rounds = eg.rounds;
         S.NP = eg.NP;
         S.deep = eg.deep;
@@ -789,24 +862,28 @@ __global__ void __launch_bounds__(kBlock, 3)
       }
       __syncthreads();
     }
-    if (tid == 0) claim_task(a, S, p ^ 1u, entry);
-    const DevItem& it = a.items[gitem];
-    const DevEngine& e = a.engines[it.engine];
-    const u32 G = it.lane_threads, nblock = it.blocks;
-    const u32 cpw = G == 32 ? 1u : (G == 8 ? 4u : 32u);  // chains per block
-    const u64 nchain = it.nchunk * e.L;
-    const u64 b0 = (task - a.task_prefix[entry]) * (u64)nblock;
     for (;;) {
-      u32 wt = 0;
-      if (wl == 0) wt = atomicAdd(&S.wnext[p], 1u);
-      wt = __shfl_sync(0xffffffffu, wt, 0);
-      if (wt >= nblock) break;
-      const u64 gw = (b0 + wt) * cpw;      // the block's first chain
-      if (gw >= nchain) break;             // and every later one's too
-      sieve_block<P0, NS>(spat, S, Q, qn, a, e, it, gitem, gw, nchain, ntest,
-                          nword);
+      u64 b = 0;
+      if (wl == 0) b = atomicAdd(S.blk.next, (unsigned long long)S.blk.run);
+      b = __shfl_sync(0xffffffffu, b, 0);
+      if (b >= S.blk.nblock) break;
+      const u64 end = min(b + S.blk.run, S.blk.nblock);
+      for (; b < end; ++b) {
+        const u32 G = S.blk.G;
+        // chains per block: 32 / G
+        sieve_block<P0, NS>(spat, S, a,
+                            b * (G == 32 ? 1u : (G == 8 ? 4u : 32u)));
+      }
     }
-    __syncthreads();   // the next task is claimed, this one's counter free
+    // drain the queues and report
+    drain_any(S, true, a);
+    if (wl == 0) {
+      if (S.ntest[wid]) atomicAdd(&a.ctr->s2_tests, S.ntest[wid]);
+      if (S.nword[wid]) atomicAdd(&a.ctr->s1_words, S.nword[wid]);
+      S.ntest[wid] = S.nword[wid] = 0;
+    }
+    __syncwarp();
+    if (++entry == a.nitems) entry = 0;
   }
 }
 

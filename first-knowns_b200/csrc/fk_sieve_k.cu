@@ -7,7 +7,7 @@ namespace {
 
 template <int P0, int NS>
 size_t sieve_smem() {
-  return pat_bytes<P0, NS>() + sizeof(SieveSmem);
+  return pat_bytes<P0, NS, kPad<NS>>() + kSieveSmemBytes;
 }
 
 template <int P0, int NS>

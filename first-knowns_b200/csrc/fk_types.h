@@ -37,6 +37,7 @@ constexpr int kNSMin = 24;        // fewest pattern primes a kernel variant
                                   // stages; marking tables start here
 constexpr int kNSMax = 40;        // most: the engine's pattern tables hold
                                   // this many primes
+constexpr uint32_t kPadWide = 64, kPadNarrow = 32;  // pattern table padding
 constexpr int kMaxRounds = 64;
 constexpr int kSortSmem = 4096;   // entries a CTA sorts in shared memory
 constexpr int kClassChunk = 128;  // candidates a warp fetches at once
@@ -46,7 +47,7 @@ constexpr int kWarpMode = 32;     // warp queue below which a candidate
 constexpr int kSbits = 512;       // Euler: most words of the {x^2 + x} bitset
 constexpr int kStaged = 128;      // rounds: test primes held in shared memory
 constexpr int kStagedBits = 1536; // Dickson: words of their residue bitmaps
-constexpr int kMaxTaskBlocks = 256;  // rounds: most warp blocks per CTA task
+constexpr int kMaxRun = 32;       // rounds: most blocks a warp claims at once
 constexpr int kSeg = 32768;       // marking: periods per shared segment
                                   // (default; variants 16384 and 65536)
 constexpr int kNumSeg = 3;        // marking segment variants
@@ -71,6 +72,13 @@ struct DevEngine {
   // entry k = the kill mask of the 64 periods from phase 64k mod q, so
   // consecutive words of a lane are consecutive entries
   const uint64_t* pat;
+  // the rounds kernel's copies, every prime's table padded by kPadWide or
+  // kPadNarrow entries that repeat its first ones
+  const uint64_t* patw;
+  const uint64_t* patn;
+  const TestRec* prec;            // [kNSMax] pattern primes, a = 1 / (64 M):
+                                  // the scaled residue of v = 64 M w + R is
+                                  // the table index of word w of lane R
   const uint32_t* pat_minv;       // [kNSMax] (M mod q)^-1 * 64^-1 mod q
   const uint32_t* pat_i64;        // [kNSMax] 64^-1 mod q
   const PrimeRec* recs;           // [NP]
@@ -129,12 +137,12 @@ struct DevItem {
                                   // thread t of a group takes words t,
                                   // t + lane_threads, ... of its block
   uint64_t nchunk;                // chains per lane
-  uint64_t task0, ntask;          // first task, task count
+  uint64_t task0, ntask;          // first task, task count (rounds: blocks)
   uint64_t xq_off;                // this item's base-residue table: X0 mod q
                                   // of the primes sieved by pattern or mark,
                                   // X0 * c1 mod q of the primes tested
   uint32_t marked;                // 1: the marking kernel sweeps this item
-  uint32_t blocks;                // rounds: warp blocks per CTA task
+  uint32_t run;                   // rounds: blocks a warp claims at once
   uint64_t nchunk_u;              // marking: u-chunks per lane
 };
 
