@@ -7,7 +7,8 @@
 //             the 128-bit base.
 // k_dense     fills the candidate list with every x of a DENSE item (the
 //             launchers' low passes below the engine floors).
-// k_classify  the on-device SPRP stage: each candidate's chain depth by
+// k_classify, k_exact
+//             the on-device SPRP stage: each candidate's chain depth by
 //             the reference's definition for its engine (Euler
 //             mr_run_length, Dickson run_length / sprp_run, AP two-pass
 //             chain_depth), kept when it reaches the item's threshold.
@@ -34,6 +35,8 @@ struct ClassArgs {
   OutRec* out;
   u64 out_cap;
   u32* item_count;
+  u64* exact;               // [cand_cap] candidate index << 8 | base-2 depth
+  u64 spec_lanes;           // lanes worth filling with a candidate's values
 };
 
 __device__ __forceinline__ void emit_out(const ClassArgs& a, u32 item,
@@ -123,96 +126,124 @@ __device__ int chain_depth_thr(const Chain& c, u32 mode, u32 thr, u32 cap,
   return depth >= thr ? (int)depth : -1;
 }
 
-// The SPRP stage as a step interpreter.  Each lane holds the state of one
-// candidate's chain and performs exactly ONE strong test per step -- one
-// value, one base -- then advances its own state machine:
-//   phase 0  base-2 chain: test value t to base 2; pass -> t + 1 (until the
-//            limit), fail -> d2 = t, the base-2 depth, an upper bound on
-//            every engine's depth (mr_is_prime implies sprp_base2)
-//   decide   by the engine's rules (chain_depth_thr): drop the candidate
-//            when d2 already proves it below the threshold, report d2 for
-//            the two-pass engines below their exact-from depth, else
-//   phase 1  the exact chain: values t < d2 tested to the six other bases,
-//            one base per step; the first failure ends the chain
-// A lane whose candidate is finished takes the next one at once from a
-// chunk its warp fetched, so a warp never waits for its longest chain, and
-// lanes of one warp run the same loop shape on same-sized values.
+// The SPRP stage, in two kernels.
+//
+// k_classify finds each candidate's base-2 depth d2 -- the first t whose
+// value fails the strong test to base 2, an upper bound on every engine's
+// depth (mr_is_prime implies sprp_base2) -- and decides by the engine's
+// rules (chain_depth_thr): dropped when d2 already proves it below the
+// threshold, reported for the two-pass engines below their exact-from depth,
+// else put on the exact list with its d2.  k_exact then tests the values t <
+// d2 of the listed candidates to the six other bases: all 6 * d2 tests of a
+// candidate are independent, so a warp's lanes share them out instead of one
+// lane running them one after the other (which alone took 0.6 ms of an 0.78
+// ms hunt of 32 candidates, at 6 of 32 lanes active).
+//
+// In k_classify a chain of G lanes tests G consecutive values of one
+// candidate at once when the candidates are too few to fill the chip (G up
+// to 32: the tests past the first failure cost nothing there).  With G = 1
+// it is a step interpreter: each lane holds the state of one candidate and
+// performs exactly one strong test per step, and a lane whose candidate is
+// finished takes the next one at once from a chunk its warp fetched, so a
+// warp never waits for its longest chain.
 struct LaneState {
   Chain c;
-  u64 v;
+  u64 v, i;
   u32 item, mode, thr, cap;
-  u32 phase, t, bi, lim, d2, pass;
+  u32 t, lim, pass;
 };
 
-__device__ __forceinline__ bool lane_init(LaneState& s, const ClassArgs& a,
-                                          u64 i) {
-  s.item = a.cand_item[i];
-  const DevItem it = a.items[s.item];
-  const DevEngine& e = a.engines[it.engine];
-  s.v = a.cand_key[i];
-  if (it.mode == MODE_SIEVE) {
-    emit_out(a, s.item, s.v << 8);
-    return false;
-  }
-  s.mode = it.mode;
-  s.thr = it.threshold;
-  s.cap = it.cap;
-  s.c.kind = e.kind;
-  s.c.x = (((u128)it.X0_hi << 64) | it.X0_lo) + s.v;
+// The chain of candidate i's value at line offset v of item `item`; false
+// when a Dickson square does not fit 192 bits.
+__device__ __forceinline__ bool chain_init(Chain& c, const ClassArgs& a,
+                                           const DevItem& it,
+                                           const DevEngine& e, u64 v) {
+  c.kind = e.kind;
+  c.x = (((u128)it.X0_hi << 64) | it.X0_lo) + v;
   if (e.kind == KIND_DICKSON) {
     const u64 W = (it.mode == MODE_DENSE) ? 1ull : e.W;
     bool of = false;
-    const u128 k = s.c.x * (u128)W;
-    s.c.kk = v3_mul_128(k, k, &of);
+    const u128 k = c.x * (u128)W;
+    c.kk = v3_mul_128(k, k, &of);
     if (of) {
       atomicOr(&a.ctr->overflow, 8u);
       return false;
     }
   } else if (e.kind == KIND_AP) {
-    s.c.d = V3{{e.d_lo, e.d_hi, 0}};
+    c.d = V3{{e.d_lo, e.d_hi, 0}};
   }
+  return true;
+}
+
+__device__ __forceinline__ bool lane_init(LaneState& s, const ClassArgs& a,
+                                          u64 i, bool emit) {
+  s.i = i;
+  s.item = a.cand_item[i];
+  const DevItem& it = a.items[s.item];
+  const DevEngine& e = a.engines[it.engine];
+  s.v = a.cand_key[i];
+  s.mode = it.mode;
+  if (s.mode == MODE_SIEVE) {
+    if (emit) emit_out(a, s.item, s.v << 8);
+    return false;
+  }
+  s.thr = it.threshold;
+  s.cap = it.cap;
+  if (!chain_init(s.c, a, it, e, s.v)) return false;
   s.pass = (e.kind == KIND_AP) ? 6u
            : (e.kind == KIND_DICKSON ? (e.two_pass ? 5u : 0u) : 0u);
   s.lim = (e.kind == KIND_EULER) ? max(s.thr, s.cap) : s.cap;
-  s.phase = 0;
   s.t = 0;
-  s.bi = 0;
   return true;
 }
 
 // Finish with the exact depth: emit when it reaches the threshold.
-__device__ __forceinline__ void lane_final(const LaneState& s,
-                                           const ClassArgs& a, u32 exact) {
-  if (s.c.kind == KIND_EULER) {
-    const u32 depth = min(exact, s.cap);
-    const u32 test = (s.mode == MODE_DENSE) ? depth : exact;
-    if (test >= s.thr) emit_out(a, s.item, (s.v << 8) | (u64)min(depth, 255u));
-  } else if (exact >= s.thr) {
-    emit_out(a, s.item, (s.v << 8) | (u64)min(exact, 255u));
+__device__ __forceinline__ void emit_final(const ClassArgs& a, u32 kind,
+                                           u32 mode, u32 thr, u32 cap,
+                                           u32 item, u64 v, u32 exact) {
+  if (kind == KIND_EULER) {
+    const u32 depth = min(exact, cap);
+    const u32 test = (mode == MODE_DENSE) ? depth : exact;
+    if (test >= thr) emit_out(a, item, (v << 8) | (u64)min(depth, 255u));
+  } else if (exact >= thr) {
+    emit_out(a, item, (v << 8) | (u64)min(exact, 255u));
   }
 }
 
-// After the base-2 chain: returns true when the exact phase must run.
-__device__ __forceinline__ bool lane_decide(LaneState& s, const ClassArgs& a) {
-  const u32 d2 = s.d2;
+// After the base-2 chain of depth d2: report it, drop it, or list it for
+// the exact tests.
+__device__ __forceinline__ void lane_decide(const LaneState& s,
+                                            const ClassArgs& a, u32 d2) {
   if (s.c.kind == KIND_EULER) {
     const u32 bound = (s.mode == MODE_DENSE) ? min(d2, s.cap) : d2;
-    if (bound < s.thr) return false;
+    if (bound < s.thr) return;
   } else {
     if (d2 < s.pass) {
       if (d2 >= s.thr) emit_out(a, s.item, (s.v << 8) | (u64)min(d2, 255u));
-      return false;
+      return;
     }
-    if (d2 < s.thr) return false;
+    if (d2 < s.thr) return;
   }
   if (d2 == 0) {
-    lane_final(s, a, 0);
-    return false;
+    emit_final(a, s.c.kind, s.mode, s.thr, s.cap, s.item, s.v, 0);
+    return;
   }
-  s.phase = 1;
-  s.t = 0;
-  s.bi = 1;
-  return true;
+  // at most one entry per candidate, so the list never overflows
+  a.exact[atomicAdd(&a.ctr->nexact, 1ull)] = (s.i << 8) | (u64)d2;
+}
+
+// One atomic per warp for the work counters.
+__device__ __forceinline__ void report_work(const ClassArgs& a, u64 imad,
+                                            u64 nval) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    imad += __shfl_down_sync(0xffffffffu, imad, o);
+    nval += __shfl_down_sync(0xffffffffu, nval, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (imad) atomicAdd(&a.ctr->imad_alg, (unsigned long long)imad);
+    if (nval) atomicAdd(&a.ctr->sprp_values, (unsigned long long)nval);
+  }
 }
 
 __global__ void __launch_bounds__(kBlock) k_classify(ClassArgs a) {
@@ -220,10 +251,48 @@ __global__ void __launch_bounds__(kBlock) k_classify(ClassArgs a) {
   if (n > a.cand_cap) n = a.cand_cap;
   const u32 lane = threadIdx.x & 31;
   const u32 lt = (1u << lane) - 1u;
-  u64 chunk_pos = 0, chunk_end = 0;  // warp-uniform
-  bool active = false, drained = false;
   LaneState st;
   u64 imad = 0, nval = 0;
+  // lanes per candidate: the most that keep every lane's warp resident with
+  // few enough others that a step takes no longer than it takes alone
+  u32 G = 32;
+  while (G > 1 && n * G > a.spec_lanes) G >>= 1;
+  if (G > 1) {
+    const u32 gl = lane & (G - 1), g0 = lane & ~(G - 1);
+    const u32 gmask = (G == 32 ? 0xffffffffu : ((1u << G) - 1u)) << g0;
+    const u64 groups = (u64)gridDim.x * (kBlock / G);
+    // consecutive candidates go to different CTAs.  The whole warp stays in
+    // the loop while one of its groups has a candidate, so the votes are
+    // warp-wide
+    for (u64 i = ((u64)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * (32 / G) +
+                 lane / G;
+         __any_sync(0xffffffffu, i < n); i += groups) {
+      bool active = i < n && lane_init(st, a, i, gl == 0);
+      while (__any_sync(0xffffffffu, active)) {
+        const u32 t = st.t + gl;
+        bool fail = false;
+        if (active && t < st.lim) {
+          ++nval;
+          fail = !sprp_step(chain_value(st.c, t), 0, &imad);
+        }
+        const u32 bad = __ballot_sync(0xffffffffu, fail) & gmask;
+        if (active) {
+          if (bad || st.t + G >= st.lim) {
+            if (gl == 0)
+              lane_decide(st, a,
+                          bad ? st.t + __ffs((int)bad) - 1 - g0 : st.lim);
+            active = false;
+          } else {
+            st.t += G;
+          }
+        }
+      }
+    }
+    report_work(a, imad, nval);
+    return;
+  }
+  u64 chunk_pos = 0, chunk_end = 0;  // warp-uniform
+  bool active = false, drained = false;
   for (;;) {
     // hand new candidates to idle lanes
     while (!drained) {
@@ -242,47 +311,93 @@ __global__ void __launch_bounds__(kBlock) k_classify(ClassArgs a) {
       }
       const u32 rank = __popc(idle & lt);
       const u32 take = (u32)min((u64)__popc(idle), chunk_end - chunk_pos);
-      if (!active && rank < take) active = lane_init(st, a, chunk_pos + rank);
+      if (!active && rank < take)
+        active = lane_init(st, a, chunk_pos + rank, true);
       chunk_pos += take;
     }
     if (__ballot_sync(0xffffffffu, active) == 0) break;
     if (active) {
-      ++nval;
-      const bool pass = sprp_step(chain_value(st.c, st.t), st.bi, &imad);
-      if (st.phase == 0) {
-        if (pass && st.t + 1 < st.lim) {
-          ++st.t;
-        } else {
-          st.d2 = pass ? st.lim : st.t;
-          active = lane_decide(st, a);
-        }
+      bool pass = false;
+      if (st.lim > 0) {
+        ++nval;
+        pass = sprp_step(chain_value(st.c, st.t), 0, &imad);
+      }
+      if (pass && st.t + 1 < st.lim) {
+        ++st.t;
       } else {
-        if (!pass) {
-          lane_final(st, a, st.t);
-          active = false;
-        } else if (st.bi < 6) {
-          ++st.bi;
-        } else if (st.t + 1 < st.d2) {
-          ++st.t;
-          st.bi = 1;
-        } else {
-          lane_final(st, a, st.d2);
-          active = false;
-        }
+        lane_decide(st, a, pass ? st.lim : st.t);
+        active = false;
       }
     }
   }
-  // one atomic per warp for the work counters
-  u64 s1 = imad, s2 = nval;
+  report_work(a, imad, nval);
+}
+
+// The exact tests: a warp takes up to kExactChunk listed candidates and its
+// lanes share out all their (value, base) tests in order; a failure lowers
+// the candidate's depth to the value's index.
+constexpr u32 kExactChunk = 16;
+__global__ void __launch_bounds__(kBlock) k_exact(ClassArgs a) {
+  __shared__ u32 s_first[kBlock / 32][kExactChunk];
+  const u64 n = a.ctr->nexact;
+  const u32 lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  u32* first = s_first[wid];
+  u64 imad = 0, nval = 0;
+  // fewer at a time when they are too few to go round
+  const u64 warps = (u64)gridDim.x * (kBlock / 32);
+  const u32 chunk =
+      (u32)min((u64)kExactChunk, max((u64)1, n / (warps * 2)));
+  for (;;) {
+    unsigned long long base = 0;
+    if (lane == 0) base = atomicAdd(&a.ctr->exact_next, (u64)chunk);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (base >= n) break;
+    const u32 m = (u32)min((u64)chunk, n - base);
+    const u64 rec = lane < m ? a.exact[base + lane] : 0;
+    const u32 d2 = (u32)(rec & 255u);
+    if (lane < m) first[lane] = d2;
+    u32 end = 6 * d2;   // inclusive prefix of the test counts
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    s1 += __shfl_down_sync(0xffffffffu, s1, o);
-    s2 += __shfl_down_sync(0xffffffffu, s2, o);
+    for (int o = 1; o < (int)kExactChunk; o <<= 1) {
+      const u32 y = __shfl_up_sync(0xffffffffu, end, o);
+      if (lane >= (u32)o) end += y;
+    }
+    const u32 total = __shfl_sync(0xffffffffu, end, m - 1);
+    __syncwarp();
+    for (u32 k0 = 0; k0 < total; k0 += 32) {
+      const u32 k = k0 + lane;
+      // the candidate of test k: the first whose prefix passes k
+      u32 c = 0, from = 0;
+      for (u32 j = 0; j < m; ++j) {
+        const u32 e = __shfl_sync(0xffffffffu, end, j);
+        if (e <= k) {
+          c = j + 1;
+          from = e;
+        }
+      }
+      const u64 r = __shfl_sync(0xffffffffu, rec, c < m ? c : 0);
+      if (k < total) {
+        const u32 t = (k - from) / 6u, b = (k - from) % 6u + 1u;
+        const u64 i = r >> 8;
+        const DevItem& it = a.items[a.cand_item[i]];
+        Chain ch;
+        chain_init(ch, a, it, a.engines[it.engine], a.cand_key[i]);
+        ++nval;
+        if (!sprp_step(chain_value(ch, t), (int)b, &imad))
+          atomicMin(&first[c], t);
+      }
+      __syncwarp();
+    }
+    if (lane < m) {
+      const u64 i = rec >> 8;
+      const u32 item = a.cand_item[i];
+      const DevItem& it = a.items[item];
+      emit_final(a, a.engines[it.engine].kind, it.mode, it.threshold, it.cap,
+                 item, a.cand_key[i], first[lane]);
+    }
+    __syncwarp();
   }
-  if ((threadIdx.x & 31) == 0) {
-    if (s1) atomicAdd(&a.ctr->imad_alg, (unsigned long long)s1);
-    if (s2) atomicAdd(&a.ctr->sprp_values, (unsigned long long)s2);
-  }
+  report_work(a, imad, nval);
 }
 
 // Every x of dense items, into the candidate list.

@@ -721,6 +721,7 @@ struct fk_batch {
   u64 last_launches = 0;
   u64 h2d = 0, d2h = 0;
   u32 reruns = 0;               // overflow reruns of the last run
+  bool hunts = false;           // the run has items to classify
 };
 
 static const fk_tuning kDefaultTuning = {3, 3, 2048, (u32)kWarpMode,
@@ -855,6 +856,7 @@ fk_status check_interval(const fk_engine* e, const uint64_t lo[2],
 static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
   b->user.assign(items, items + nitems);
   b->items.clear();
+  b->hunts = false;
   b->sub.clear();
   b->dense_idx.clear();
   b->sieve_idx.clear();
@@ -870,6 +872,7 @@ static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
     const u128 lo = u128_of(it.lo), hi = u128_of(it.hi);
     if (hi <= lo) continue;
     if (it.mode > MODE_DENSE) return set_err(FK_ERR_ARG, "bad mode");
+    b->hunts |= it.mode != MODE_SIEVE;
     if (it.cap > 250) return set_err(FK_ERR_DOMAIN, "cap above 250");
     fk_status cs = check_interval(e, it.lo, it.hi,
                                   std::max(it.cap, it.threshold),
@@ -1099,7 +1102,15 @@ static fk_status enqueue(fk_batch* b, bool capturing = false) {
   c.out = b->d_out.p;
   c.out_cap = b->out_cap;
   c.item_count = b->d_item_count.p;
+  // the exact list takes the ordering scratch (2 * out_cap words, and
+  // cand_cap is never above out_cap), free until the sort
+  c.exact = b->d_scratch.p;
+  c.spec_lanes = (u64)b->nsm * kSpecLanes;
   k_classify<<<b->nsm * b->tune.classify_ctas_per_sm, kBlock, 0, s>>>(c);
+  if (b->hunts) {   // pre-primality streams list nothing
+    ++nl;
+    k_exact<<<b->nsm * b->tune.classify_ctas_per_sm, kBlock, 0, s>>>(c);
+  }
   FK_CUDA(record(b->ev[2], s, capturing));
   // order: per-item counts -> per-item buckets by key range -> bucket
   // counts -> scatter -> every bucket sorted in shared memory
@@ -1175,6 +1186,7 @@ static fk_status launch(fk_batch* b, int use_graph) {
   key.push_back(b->items.size());
   key.push_back(b->dense_idx.size());
   key.push_back(b->sieve_idx.size());
+  key.push_back(b->hunts);
   key.push_back(b->cand_cap);
   key.push_back(b->out_cap);
   key.push_back(b->d_xq.cap);

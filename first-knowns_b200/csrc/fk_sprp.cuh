@@ -219,10 +219,14 @@ __device__ __forceinline__ void ctx_init64(Ctx64<L>& c, const u64* m) {
   for (int i = 0; i < 5; ++i) minv *= 2 - m[0] * minv;
   c.minv = (u64)0 - minv;  // -m^-1 mod 2^64
   c.bl = bitlen64<L>(m);
+  if (L == 1) {
+    c.one[0] = ((u64)0 - m[0]) % m[0];  // 2^64 mod m
+  } else {
 #pragma unroll
-  for (int i = 0; i < L; ++i) c.one[i] = 0;
-  c.one[(c.bl - 1) >> 6] = 1ull << ((c.bl - 1) & 63);  // 2^(bl-1) < m
-  for (int i = 0; i < 64 * L - c.bl + 1; ++i) mdbl64<L>(c.one, m);
+    for (int i = 0; i < L; ++i) c.one[i] = 0;
+    c.one[(c.bl - 1) >> 6] = 1ull << ((c.bl - 1) & 63);  // 2^(bl-1) < m
+    for (int i = 0; i < 64 * L - c.bl + 1; ++i) mdbl64<L>(c.one, m);
+  }
   u64 br = 0;
 #pragma unroll
   for (int i = 0; i < L; ++i) {  // m - (R mod m): -1 in Montgomery form
@@ -271,15 +275,18 @@ __device__ __forceinline__ bool tail64(const Ctx64<L>& c, u64* x) {
   return false;
 }
 
-// One strong test of m to base kMrBases[bi] (bi = 0 is base 2), with the
-// trial division first: the unit of work of the step interpreter in
-// k_classify.  Every base runs the same loop shape -- square, then on a set
+// One strong test of m to base kMrBases[bi] (bi = 0 is base 2): the unit of
+// work of k_classify and k_exact.  Base 2 runs the trial division first; the
+// other bases are asked only of values that passed base 2, so of those only
+// the primes to 37 themselves still meet it.  Every base runs the same loop shape -- square, then on a set
 // bit of d multiply by the base (a modular doubling for base 2) -- so lanes
 // testing different bases of same-sized values stay converged.
 template <int L>
 __device__ __forceinline__ bool step64(const u64* m, int bi, u64* imad) {
-  const int t = trial64<L>(m);
-  if (t != 2) return t == 1;
+  if (bi == 0 || (L == 1 && m[0] <= 37)) {
+    const int t = trial64<L>(m);
+    if (t != 2) return t == 1;
+  }
   Ctx64<L> c;
   ctx_init64<L>(c, m);
   u64 at[L];
@@ -293,7 +300,10 @@ __device__ __forceinline__ bool step64(const u64* m, int bi, u64* imad) {
     u64 r2m[L], av[L];
 #pragma unroll
     for (int i = 0; i < L; ++i) { r2m[i] = c.one[i]; av[i] = 0; }
-    for (int i = 0; i < 64 * L; ++i) mdbl64<L>(r2m, c.m);
+    // R^2 = 2^(64 L) in Montgomery form: 2 squared 6 times is 2^64 (L = 1)
+    static_assert(L == 1, "one-limb values");
+    mdbl64<L>(r2m, c.m);
+    for (int i = 0; i < 6; ++i) mmul64<L>(r2m, r2m, r2m, c.m, c.minv);
     av[0] = a;
     mmul64<L>(at, av, r2m, c.m, c.minv);  // a * R mod m
   }
@@ -478,15 +488,17 @@ __device__ __forceinline__ bool strong_tail(const Ctx<N>& c, u32* x) {
   return false;
 }
 
-// One strong test of m to base kMrBases[bi] (bi = 0 is base 2), with the
-// trial division first.  Every base runs the same loop shape -- square,
+// One strong test of m to base kMrBases[bi] (bi = 0 is base 2, with the
+// trial division first).  Every base runs the same loop shape -- square,
 // then on a set bit of d multiply by the base (a modular doubling for base
 // 2, so base 2 needs no R^2) -- so lanes testing different bases of
 // same-sized values stay converged.
 template <int N>
 __device__ __forceinline__ bool step_N(const u32* m, int bi, u64* imad) {
-  const int t = trial_small<N>(m);
-  if (t != 2) return t == 1;
+  if (bi == 0) {   // N >= 2 values are above 37
+    const int t = trial_small<N>(m);
+    if (t != 2) return t == 1;
+  }
   Ctx<N> c;
   ctx_init<N>(c, m);
   u32 at[N];
@@ -503,7 +515,16 @@ __device__ __forceinline__ bool step_N(const u32* m, int bi, u64* imad) {
     u32 r2m[N], av[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) { r2m[i] = c.one[i]; av[i] = 0; }
-    for (int i = 0; i < 32 * N; ++i) mdbl32<N>(r2m, c.m);  // R^2 mod m
+    // R^2 = 2^(32 N) in Montgomery form: 2 squared five times is y = 2^32,
+    // and y^N by a short addition chain
+    mdbl32<N>(r2m, c.m);
+    for (int i = 0; i < 5; ++i) mmul32<N>(r2m, r2m, r2m, c.m, c.minv);
+#pragma unroll
+    for (int i = 0; i < N; ++i) at[i] = r2m[i];
+    for (int k = N >= 4 ? 1 : 0; k >= 0; --k) {  // the bits of N below its top
+      mmul32<N>(r2m, r2m, r2m, c.m, c.minv);
+      if ((N >> k) & 1) mmul32<N>(r2m, r2m, at, c.m, c.minv);
+    }
     av[0] = a;
     mmul32<N>(at, av, r2m, c.m, c.minv);  // a * R mod m
   }

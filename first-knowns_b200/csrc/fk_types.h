@@ -41,6 +41,7 @@ constexpr uint32_t kPadWide = 64, kPadNarrow = 32;  // pattern table padding
 constexpr int kMaxRounds = 64;
 constexpr int kSortSmem = 4096;   // entries a CTA sorts in shared memory
 constexpr int kClassChunk = 128;  // candidates a warp fetches at once
+constexpr int kSpecLanes = 512;   // SPRP: lanes an SM runs at no cost to each
 constexpr int kBucketFill = 1024; // expected entries per ordering bucket
 constexpr int kWarpMode = 32;     // warp queue below which a candidate
                                   // takes a whole warp
@@ -166,6 +167,8 @@ struct DevCounters {
   unsigned long long sprp_values; // values strong-tested
   unsigned long long marks;       // marking-sieve byte marks
   unsigned long long class_next;  // SPRP stage: next candidate chunk
+  unsigned long long nexact;      // candidates listed for the exact tests
+  unsigned long long exact_next;  // exact tests: next candidate chunk
 };
 
 }  // namespace fk
