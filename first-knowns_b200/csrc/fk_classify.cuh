@@ -426,7 +426,8 @@ __global__ void k_xq(const DevEngine* engines, const DevItem* items,
   for (u32 s = blockIdx.y; s < nsieve; s += gridDim.y) {
     const DevItem it = items[sieve_idx[s]];
     const DevEngine& e = engines[it.engine];
-    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < e.NP;
+    const u32 n = base_entries(e, it);
+    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += gridDim.x * blockDim.x)
       xq[it.xq_off + i] = base_residue(e, it, i);
   }

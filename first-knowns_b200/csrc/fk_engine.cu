@@ -137,11 +137,15 @@ struct fk_engine {
                               // every sieve prime (f_q forbidden residues)
   bool use_mark = false;      // long lanes go to the marking sieve
   bool force_mark = false;    // every item goes to the marking sieve
-  // per segment length (index seg_index(SEG)): marking work entries before
-  // each prime from index kNSMin, and the device tables (mq, mitems)
-  std::vector<u32> mprefix[kNumSeg];
-  const uint64_t* d_mq[kNumSeg] = {};
-  const uint64_t* d_mitems[kNumSeg] = {};
+  // marking: residues before each prime from index kNSMin (for the cost
+  // model), and per segment length (index seg_index(SEG)) the device tables;
+  // the work lists without and with the primes below the 32nd past the wheel
+  std::vector<u32> mprefix;
+  const uint32_t* d_mq[kNumSeg] = {};
+  const MarkItem* d_mwork[kNumSeg][2] = {};
+  const uint32_t* d_mpair[kNumSeg][2] = {};
+  const uint32_t* d_mwoff[kNumSeg][2] = {};
+  u32 nslots = 0;
   Cost cost;                  // cost model with every prime below 2^16 marked
   DevEngine dev{};
   std::vector<void*> allocs;
@@ -258,7 +262,7 @@ static Cost engine_cost(const fk_engine* e, u32 NPm, u32 ns_sieve, u32 ns,
     surv_m *= 1.0 - kill;
   }
   const double npm = NPm > ns ? NPm - ns : 0;
-  const std::vector<u32>& mp = e->mprefix[seg_index(seg)];
+  const std::vector<u32>& mp = e->mprefix;
   const double items = NPm > ns && !mp.empty()
                            ? (double)mp[NPm - kNSMin] - mp[ns - kNSMin] : 0;
   c.round = 2.5 + 22.0 * s1r * tests;
@@ -305,21 +309,175 @@ static std::vector<u32> compute_rounds(const fk_engine* e, double cut,
 static void set_mark_tables(const fk_engine* e, DevEngine& d, u32 ns,
                             u32 seg, u32 npm) {
   const int si = seg_index(seg);
-  const std::vector<u32>& mp = e->mprefix[si];
+  const int low = ns < (u32)kNS;   // the primes below index kNS are marked too
   d.NS = ns;
   d.NPm = npm;
+  d.qlim = npm < (u32)e->sieve.size() ? e->sieve[npm] : 65536u;
+  d.nslots = e->nslots;
+  d.slot0 = low ? 0 : 32;          // they fill the first block
   d.mq = e->d_mq[si];
-  const u32 first = npm > ns ? mp[ns - kNSMin] : 0;
-  d.mitems = e->d_mitems[si] + first;
-  d.nmitems = npm > ns ? mp[npm - kNSMin] - first : 0;
-  // the hit classes: primes from q >= seg / 2 on hit a segment at most
-  // twice per residue, from q >= seg on at most once
-  u32 p2 = ns, p1 = ns;
-  while (p2 < npm && e->sieve[p2] < seg / 2) ++p2;
-  p1 = p2;
-  while (p1 < npm && e->sieve[p1] < seg) ++p1;
-  d.nm2 = npm > ns ? mp[p2 - kNSMin] - first : 0;
-  d.nm1 = npm > ns ? mp[p1 - kNSMin] - first : 0;
+  d.mwork = e->d_mwork[si][low];
+  d.mpair = e->d_mpair[si][low];
+  d.mwoff = e->d_mwoff[si][low];
+}
+
+// The marking sieve's slots and work lists (DevEngine, MarkItem): the primes
+// from index kNSMin to NPm, those before kNS in a block of their own, the
+// rest by octave and within an octave by residue count.
+struct MarkTables {
+  std::vector<u32> sprime, mres, prefix;   // prefix: residues before a prime
+  std::vector<TestRec> mrec;
+  std::vector<u32> mq[kNumSeg];
+  std::vector<MarkItem> work[kNumSeg][2];
+  std::vector<u32> woff[kNumSeg][2], pair[kNumSeg][2];
+};
+
+static fk_status build_marks(const fk_engine* e, u32 NPm, MarkTables& t) {
+  const u32 NP = (u32)e->sieve.size();
+  std::vector<std::vector<u32>> g(NP);     // forbidden period residues
+  for (u32 i = kNSMin; i < NPm; ++i) {
+    t.prefix.push_back(t.prefix.empty() ? 0
+                                        : t.prefix.back() + (u32)g[i - 1].size());
+    const u32 q = e->sieve[i];
+    const u64 mi = invmod(e->M % q, q);
+    if (e->forb[i].size() > 127) return set_err(FK_ERR_DOMAIN, "forbidden set too large");
+    for (u32 r : e->forb[i]) g[i].push_back((u32)mulmod64(r, mi, q));
+    std::sort(g[i].begin(), g[i].end());
+  }
+  if (NPm > (u32)kNSMin) t.prefix.push_back(t.prefix.back() + (u32)g[NPm - 1].size());
+  struct Block { u32 res, f, qmin, qmax; bool low; };
+  std::vector<Block> blocks;
+  for (u32 i = kNSMin; i < NPm;) {
+    // one octave (or the primes before kNS), the most residues first
+    std::vector<u32> c;
+    const bool low = i < (u32)kNS;
+    const u32 end = low ? (u32)kNS : NP;
+    u32 top = 1;
+    while (top <= e->sieve[i]) top *= 2;
+    for (; i < NPm && i < end && (low || e->sieve[i] < top); ++i) c.push_back(i);
+    std::stable_sort(c.begin(), c.end(),
+                     [&](u32 x, u32 y) { return g[x].size() > g[y].size(); });
+    // primes without residues are never marked (the low ones keep their
+    // block, so the first slot past them is fixed)
+    if (!low) while (!c.empty() && g[c.back()].empty()) c.pop_back();
+    for (size_t k = 0; k < c.size(); k += 32) {
+      Block b{(u32)t.mres.size(), (u32)g[c[k]].size(), ~0u, 0, low};
+      t.mres.resize(t.mres.size() + (b.f + 1) / 2 * 32, 0);
+      for (u32 l = 0; l < 32; ++l) {
+        u32 p = c[std::min(k + l, c.size() - 1)];
+        if (g[p].empty()) p = c[k];        // a low prime without residues
+        t.sprime.push_back(p);
+        const u32 q = e->sieve[p];
+        t.mrec.push_back(redc_rec(q, invmod(e->M % q, q)));
+        b.qmin = std::min(b.qmin, q);
+        b.qmax = std::max(b.qmax, q);
+        for (u32 j = 0; j < (b.f + 1) / 2 * 2; ++j)
+          t.mres[b.res + j / 2 * 32 + l] |=
+              g[p][std::min<size_t>(j, g[p].size() - 1)] << (16 * (j & 1));
+      }
+      blocks.push_back(b);
+    }
+  }
+  if (t.sprime.size() > (size_t)kMarkSlots)
+    return set_err(FK_ERR_DOMAIN, "too many marking slots");
+  for (int si = 0; si < kNumSeg; ++si) {
+    const u32 seg = (u32)kSegOf(si);
+    for (u32 p : t.sprime) {
+      const u32 q = e->sieve[p];
+      t.mq[si].push_back(q | (seg % q) << 16);
+    }
+    for (int low = 0; low < 2; ++low) {
+      struct Piece { MarkItem m; double cost; };
+      std::vector<Piece> pieces;
+      // hits per lane and residue: floor(seg / qmax) to ceil(seg / qmin)
+      auto add_pairs = [&](u32 at, u32 qmin, u32 qmax) {
+        const u32 kmin = seg / qmax, kmax = (seg + qmin - 1) / qmin;
+        const u32 parts = std::max<u32>(1, (kmax + kMarkHits / 2) / kMarkHits);
+        const u32 K = kmin / parts;
+        for (u32 k = 0; k < parts; ++k) {
+          const bool last = k + 1 == parts;
+          const u32 kk = last ? kmin - k * K : K;
+          const u32 E = last ? kmax - kmin : 0;
+          pieces.push_back({{MARK_PAIRS, 0, at, k * K | kk << 16 | E << 24},
+                            60.0 + 2.5 * kk + 7.0 * E});
+        }
+      };
+      auto add_block = [&](u32 bi) {
+        const Block& b = blocks[bi];
+        const u32 kmin = seg / b.qmax;
+        u32 E = (seg + b.qmin - 1) / b.qmin - kmin;
+        u32 kind = MARK_BLOCKS;
+        if (kmin <= 7 && E <= (kmin ? 2u : 1u)) {
+          kind = MARK_FIXED;
+          if (kmin >= 2) E = 2;    // the variants that exist
+        }
+        const double cost = 25.0 + b.f * (kind == MARK_FIXED ? 5.0 + 2.0 * kmin + 4.0 * E
+                                                            : 14.0 + 3.0 * kmin + 7.0 * E);
+        // after the last item's blocks, when they are of one form
+        if (!pieces.empty()) {
+          Piece& p = pieces.back();
+          const u32 nblk = (p.m.kind >> 8) & 0xFFu;
+          if ((p.m.kind & 0xFFu) == kind && p.m.kind >> 16 == b.f &&
+              p.m.hits == (kmin << 16 | E << 24) && p.m.block + nblk == bi &&
+              p.cost + cost <= kMarkCost && nblk < 255) {
+            p.m.kind += 1u << 8;
+            p.cost += cost;
+            return;
+          }
+        }
+        pieces.push_back({{kind | 1u << 8 | b.f << 16, bi, b.res, kmin << 16 | E << 24},
+                          20.0 + cost});
+      };
+      // primes below seg / 16 by pairs of nearly equal step
+      std::vector<std::pair<u32, u32>> pairs;   // q, residue | slot << 16
+      std::vector<u32>& pv = t.pair[si][low];
+      for (u32 bi = 0; bi < blocks.size(); ++bi) {
+        const Block& b = blocks[bi];
+        if ((b.low && !low) || b.f == 0) continue;
+        if (b.qmax < seg / 16) {
+          u32 seen = ~0u;
+          for (u32 l = 0; l < 32; ++l) {
+            const u32 slot = bi * 32 + l, p = t.sprime[slot];
+            if (p == seen || (l && p == t.sprime[bi * 32])) break;  // filled up
+            seen = p;
+            for (u32 r : g[p]) pairs.push_back({e->sieve[p], r | slot << 16});
+          }
+          continue;
+        }
+        add_block(bi);
+      }
+      std::sort(pairs.begin(), pairs.end());
+      for (size_t k = 0, n; k < pairs.size(); k += n) {
+        const u32 at = (u32)pv.size();
+        n = std::min<size_t>(32, pairs.size() - k);
+        // trip counts within 64 of one another (E has eight bits)
+        while (n > 1 && seg / pairs[k].first - seg / pairs[k + n - 1].first > 64) --n;
+        for (size_t l = 0; l < 32; ++l)
+          pv.push_back(pairs[k + std::min(l, n - 1)].second);
+        add_pairs(at, pairs[k].first, pairs[k + n - 1].first);
+      }
+      // the dearest piece first, each to the warp with the least so far
+      std::stable_sort(pieces.begin(), pieces.end(),
+                       [](const Piece& x, const Piece& y) { return x.cost > y.cost; });
+      constexpr int kW = kBlock / 32;
+      std::vector<MarkItem> list[kW];
+      double load[kW] = {};
+      for (const Piece& p : pieces) {
+        int best = 0;
+        for (int w = 1; w < kW; ++w) if (load[w] < load[best]) best = w;
+        load[best] += p.cost;
+        list[best].push_back(p.m);
+      }
+      auto& work = t.work[si][low];
+      auto& off = t.woff[si][low];
+      for (int w = 0; w < kW; ++w) {
+        off.push_back((u32)work.size());
+        work.insert(work.end(), list[w].begin(), list[w].end());
+      }
+      off.push_back((u32)work.size());
+    }
+  }
+  return FK_OK;
 }
 
 static fk_status build_engine(fk_engine* e) {
@@ -410,7 +568,6 @@ static fk_status build_engine(fk_engine* e) {
   // and the 32 lanes of a warp sweeping one lane read 32 consecutive
   // entries (no bank conflict)
   std::vector<u64> pat, patw, patn;
-  std::vector<u32> minv(kNSMax), i64(kNSMax);
   std::vector<TestRec> prec(kNSMax);
   for (int i = 0; i < kNSMax; ++i) {
     const u32 q = e->sieve[i];
@@ -418,8 +575,6 @@ static fk_status build_engine(fk_engine* e) {
       return set_err(FK_ERR_DEVICE, "pattern prime layout mismatch");
     const u64 mq = e->M % q;
     const u64 mi = invmod(mq, q);
-    i64[i] = fk_inv64(q);
-    minv[i] = (u32)mulmod64(mi, i64[i], q);
     std::vector<uint8_t> g(q, 0);
     for (u32 f : e->forb[i]) g[mulmod64(f, mi, q)] = 1;
     for (u32 k = 0; k < q; ++k) {
@@ -432,7 +587,7 @@ static fk_status build_engine(fk_engine* e) {
     const size_t t = pat.size() - q;
     for (u32 k = 0; k < q + kPadWide; ++k) patw.push_back(pat[t + k % q]);
     for (u32 k = 0; k < q + kPadNarrow; ++k) patn.push_back(pat[t + k % q]);
-    prec[i] = redc_rec(q, minv[i]);
+    prec[i] = redc_rec(q, mulmod64(mi, fk_inv64(q), q));
     e->survival *= 1.0 - (double)e->forb[i].size() / q;
   }
   // ---- per-candidate primes -----------------------------------------------
@@ -502,50 +657,13 @@ static fk_status build_engine(fk_engine* e) {
     e->survival *= 1.0 - (double)e->forb[i].size() / e->sieve[i];
   // ---- compaction rounds: a round ends when survival within it halves ----
   const std::vector<u32> rounds = compute_rounds(e, kDefaultRoundCut, kNS);
-  // ---- marking tables: u-residue lists for every prime, (M mod q)^-1 ------
-  std::vector<u32> minv_all(NP), gaux(NP), glist;
-  u32 NPm = NS_marked_end(e);
-  for (u32 i = 0; i < NP; ++i) {
-    const u32 q = e->sieve[i];
-    const u64 mi = invmod(e->M % q, q);
-    minv_all[i] = (u32)mi;
-    const auto& f = e->forb[i];
-    if (f.size() > 127) return set_err(FK_ERR_DOMAIN, "forbidden set too large");
-    gaux[i] = (u32)glist.size() | ((u32)f.size() << 24);
-    std::vector<u32> g;
-    for (u32 r : f) g.push_back((u32)mulmod64(r, mi, q));
-    std::sort(g.begin(), g.end());
-    glist.insert(glist.end(), g.begin(), g.end());
-  }
-  if (glist.size() >= (1u << 24)) return set_err(FK_ERR_DOMAIN, "glist too large");
-  // ---- marking work lists, one per segment length SEG: every (prime,
-  // forbidden residue) progression from prime index kNSMin, cut into
-  // sub-ranges of at least kMarkHits hits and at most 8 per segment,
-  // ordered by prime so a warp's entries share q and trip counts
-  std::vector<u64> mq[kNumSeg];
-  std::vector<u64> mitems[kNumSeg];
-  for (int si = 0; si < kNumSeg; ++si) {
-    const u32 seg = (u32)kSegOf(si);
-    e->mprefix[si].clear();
-    for (u32 i = kNSMin; i < NPm; ++i) {
-      const u32 q = e->sieve[i];
-      const u32 pi = i - kNSMin;
-      u32 S = 0, nsub = 1;
-      if (q < seg / kMarkHits) {
-        const u32 K = std::max<u32>(kMarkHits, (seg / 8 + q - 1) / q);
-        S = K * q;
-        nsub = (seg + S - 1) / S;
-      }
-      mq[si].push_back((u64)q | ((u64)(seg % q) << 16));
-      e->mprefix[si].push_back((u32)mitems[si].size());
-      const u32 go = gaux[i] & 0x00FFFFFFu, gc = gaux[i] >> 24;
-      for (u32 k = 0; k < nsub; ++k)
-        for (u32 c = 0; c < gc; ++c)
-          mitems[si].push_back((u64)(glist[go + c] | (pi << 16) | (k << 29)) |
-                               ((u64)q << 32) | ((u64)S << 48));
-    }
-    e->mprefix[si].push_back((u32)mitems[si].size());
-  }
+  // ---- marking tables -------------------------------------------------------
+  const u32 NPm = NS_marked_end(e);
+  MarkTables marks;
+  const fk_status ms = build_marks(e, NPm, marks);
+  if (ms) return ms;
+  e->nslots = (u32)marks.sprime.size();
+  e->mprefix = marks.prefix;
   e->cost = engine_cost(e, NPm, kNS, kNS, kSeg);
   e->use_mark = e->cost.mark;
   if (p.sieve == 1) e->use_mark = false;
@@ -575,8 +693,6 @@ static fk_status build_engine(fk_engine* e) {
   if ((st = upload(e, patn, &d.patn, pat_bytes_for(P0) + kNSMax * kPadNarrow * 8)))
     return st;
   if ((st = upload(e, prec, &d.prec))) return st;
-  if ((st = upload(e, minv, &d.pat_minv))) return st;
-  if ((st = upload(e, i64, &d.pat_i64))) return st;
   if ((st = upload(e, recs, &d.recs))) return st;
   if ((st = upload(e, c64, &d.c64))) return st;
   if ((st = upload(e, lists, &d.lists))) return st;
@@ -596,12 +712,16 @@ static fk_status build_engine(fk_engine* e) {
   if ((st = upload(e, sbits, &d.sbits))) return st;
   d.NPm = NPm;
   d.use_mark = e->use_mark ? 1 : 0;
-  if ((st = upload(e, minv_all, &d.minv_all))) return st;
-  if ((st = upload(e, gaux, &d.gaux))) return st;
-  if ((st = upload(e, glist, &d.glist))) return st;
+  if ((st = upload(e, marks.mrec, &d.mrec))) return st;
+  if ((st = upload(e, marks.sprime, &d.sprime))) return st;
+  if ((st = upload(e, marks.mres, &d.mres))) return st;
   for (int si = 0; si < kNumSeg; ++si) {
-    if ((st = upload(e, mq[si], &e->d_mq[si]))) return st;
-    if ((st = upload(e, mitems[si], &e->d_mitems[si]))) return st;
+    if ((st = upload(e, marks.mq[si], &e->d_mq[si]))) return st;
+    for (int low = 0; low < 2; ++low) {
+      if ((st = upload(e, marks.work[si][low], &e->d_mwork[si][low]))) return st;
+      if ((st = upload(e, marks.woff[si][low], &e->d_mwoff[si][low]))) return st;
+      if ((st = upload(e, marks.pair[si][low], &e->d_mpair[si][low]))) return st;
+    }
   }
   // the engine's own descriptor: the default variant (kNS pattern primes,
   // kSeg-period segments)
@@ -964,8 +1084,9 @@ static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
   // base-residue table offsets
   u64 xo = 0;
   for (u32 i : b->sieve_idx) {
+    const fk_engine* e = b->engines[b->items[i].engine];
     b->items[i].xq_off = xo;
-    xo += b->engines[b->items[i].engine]->sieve.size();
+    xo += e->sieve.size() + (b->items[i].marked ? mark_tests_at(e->nslots) : 0);
   }
   if (xo >= (1ull << 32) * 4) return set_err(FK_ERR_DOMAIN, "batch too large");
   fk_status st;

@@ -8,19 +8,25 @@
 // periods (16384, 32768 or 65536: a template variant chosen per batch) it
 //   (a) ORs the NS compile-time pattern primes into SEG / 16384 words per
 //       thread (the stage-1a pattern sieve of fk_sieve.cuh),
-//   (b) marks every other prime below 2^16 into a SEG-byte shared map.
-//       Each (prime, forbidden residue) progression of step q is one or
-//       more work entries of at least kMarkHits hits (the large primes:
-//       one entry of at most two hits), built once per engine and
-//       segment length and ordered by prime; the threads take the entries
-//       round robin, so the heavy small primes spread over every warp and
-//       a warp's entries share q and trip count.  Marks are plain byte
-//       stores (a mark is idempotent: no read-modify-write, no atomic),
-//       four per loop trip, and
+//   (b) marks every other prime below 2^16 into a SEG-byte shared map: plain
+//       byte stores (a mark is idempotent: no read-modify-write, no atomic),
 //   (c) extracts the periods that neither marked, tests any primes beyond
 //       the marked range one by one, and appends the survivors to the
 //       candidate list.
-// Each prime's first hit offset lives in shared memory and steps by the
+// The unit of (b) is a block of 32 primes of one octave, one per lane: a
+// lane reads its prime and its offset once and walks the prime's residues,
+// two to a coalesced 4-byte load, each a subtraction, a fold and its stores
+// -- fixed sequences of predicated stores, no loop, from q >= SEG / 2 on.
+// The primes with 16 hits a segment or more go by (prime, residue) pairs, 32
+// of nearly equal step to a warp, so the lanes share their trip counts.  A
+// whole segment holds floor(SEG / q) hits of every lane at least, and those
+// are stored without a bound's test.  The host cuts the work into pieces and
+// deals them to the eight warps by cost.  What bounds it: instructions (about 25 per 32 residues
+// besides the stores) and the byte stores' bank conflicts (32 random bytes
+// take 3.5 wavefronts).  With one 8-byte work entry per (prime, residue),
+// dealt to threads at 38 instructions for the two marks of a large prime, the
+// marking of 256 mixed intervals took 86.5 ms; now 69.
+// Each slot's first hit offset lives in shared memory and steps by the
 // tabulated SEG mod q from one segment to the next.
 // This is the reference AP engine's bitmap marking (primorial-ap/ap_gpu.py:
 // 204-369: tabulated small primes, shared-memory marks for mid primes,
@@ -34,12 +40,8 @@ namespace fk {
 template <int SEG>
 struct MarkSmem {
   unsigned char bytes[SEG];
-  unsigned short off16[kMarkPrimes];  // first hit offset of each prime from
-                                      // index kNSMin (marked ones are used)
+  unsigned short off16[kMarkSlots];   // first hit offset of each slot's prime
   u32 ph[kNSMax];                     // table index at the segment start
-  u32 lsh[kNSMax];                    // the lane's index shift per prime
-  u32 warp[kBlock / 32];
-  u32 minv[kNSMax];
   u32 sbits[kSbits + 1];
   u64 task;
   u32 item;
@@ -49,26 +51,27 @@ struct MarkSmem {
   unsigned long long mbar;
 };
 
-// The WPT pattern words of thread t in a segment (words WPT*t ...
-// WPT*t + WPT - 1), from each prime's table index at the segment start in
-// shared memory (ph[I]; consecutive words are consecutive entries): no
-// per-prime index occupies a register while the segment is marked.
+// The WPT pattern words of thread t in a segment (words t, t + kBlock, ...:
+// a warp's loads are consecutive entries), from each prime's table index at
+// the segment start in shared memory: no per-prime index occupies a register
+// while the segment is marked.
 template <int P0, int I, int NS, int WPT>
 struct PatSeg {
   static __device__ __forceinline__ void words(const u64* __restrict__ spat,
-                                               const u32* ph, u32 tw,
+                                               const u32* ph, u32 t,
                                                u64* acc) {
     constexpr u32 q = fk_nth_prime(P0 + I);
     constexpr u32 off = fk_pat_prefix(P0, I);
-    u32 r = ph[I] + tw % q;
+    constexpr u32 st = kBlock % q;
+    u32 r = ph[I] + t % q;
     r = min(r, r - q);
 #pragma unroll
     for (int k = 0; k < WPT; ++k) {
       acc[k] |= spat[off + r];
-      r += 1;
+      r += st;
       r = min(r, r - q);
     }
-    PatSeg<P0, I + 1, NS, WPT>::words(spat, ph, tw, acc);
+    PatSeg<P0, I + 1, NS, WPT>::words(spat, ph, t, acc);
   }
 };
 template <int P0, int NS, int WPT>
@@ -95,8 +98,176 @@ __device__ __forceinline__ bool tail_alive(u64 v, const DevEngine& e,
   return true;
 }
 
+// Mark one progression in a whole segment: a its first hit of the item,
+// step q, K hits without a test and E more with one.  K and E are the same
+// in all lanes.  Returns the hits stored.
+template <int SEG>
+__device__ __forceinline__ u32 mark_many(unsigned char* __restrict__ B, u32 a,
+                                         u32 q, u32 K, u32 E) {
+  for (u32 c = K >> 2; c > 0; --c, a += 4 * q) {
+    B[a] = 1;
+    B[a + q] = 1;
+    B[a + 2 * q] = 1;
+    B[a + 3 * q] = 1;
+  }
+  if (K & 2u) {
+    B[a] = 1;
+    B[a + q] = 1;
+    a += 2 * q;
+  }
+  if (K & 1u) {
+    B[a] = 1;
+    a += q;
+  }
+  u32 cnt = K;
+  for (u32 c = E; c > 0; --c, a += q)
+    if (a < SEG) {
+      B[a] = 1;
+      ++cnt;
+    }
+  return cnt;
+}
+
+// The same below len, in a segment cut short.
+__device__ __forceinline__ u32 mark_short(unsigned char* __restrict__ B, u32 a,
+                                          u32 q, u32 K, u32 E, u32 len) {
+  const u32 end = E ? len : min(len, a + K * q);
+  u32 cnt = 0;
+  for (; a < end; a += q, ++cnt) B[a] = 1;
+  return cnt;
+}
+
+// What the marks read besides the map.
+struct MarkCtx {
+  const unsigned short* off16;   // shared
+  const u32* mq;
+  const u32* mres;
+  u32 qlim, len;                 // len: the segment's periods
+};
+
+// The blocks of an item, two residues to a load; mark(a, q) stores the hits
+// of the progression a, a + q, ... and returns their count.
+template <typename F>
+__device__ __forceinline__ u32 mark_blocks(const MarkCtx& c, u32 nblk, u32 f,
+                                           u32 block, u32 r0, F mark) {
+  const u32 wl = threadIdx.x & 31;
+  u32 slot = block * 32 + wl, cnt = 0;
+  const u32* res = c.mres + r0 + wl;
+  for (; nblk > 0; --nblk, slot += 32) {
+    u32 g2 = __ldg(res);
+    const u32 q = __ldg(c.mq + slot) & 0xFFFFu, off = c.off16[slot];
+    for (u32 j = 0; j < f; j += 2) {
+      u32 h0 = (g2 & 0xFFFFu) - off, h1 = (g2 >> 16) - off;
+      res += 32;
+      if (j + 2 < f) g2 = __ldg(res);
+      h0 = min(h0, h0 + q);    // (g - off) mod q: the first hit
+      h1 = min(h1, h1 + q);
+      if (q >= c.qlim) continue;
+      cnt += mark(h0, q);
+      if (j + 1 < f) cnt += mark(h1, q);
+    }
+  }
+  return cnt;
+}
+
+// K hits and at most E more, in straight line: two instructions a hit
+// without a test, four with one.  (The variants stay few and their residue
+// loop rolled: the kernel's code has to stay in the instruction cache.  With
+// eight residues unrolled the warps waited for instructions, and the marking
+// of 256 mixed intervals took 131 ms instead of 69.)
+template <u32 K, u32 E, bool WHOLE>
+__device__ __forceinline__ u32 mark_fixed(unsigned char* __restrict__ B,
+                                          const MarkCtx& c, const uint4& w) {
+  return mark_blocks(c, (w.x >> 8) & 0xFFu, w.x >> 16, w.y, w.z,
+                     [&](u32 a, u32 q) {
+                       u32 cnt = 0;
+#pragma unroll
+                       for (u32 k = 0; k < K + E; ++k, a += q) {
+                         if ((WHOLE && k < K) || a < c.len) {
+                           B[a] = 1;
+                           ++cnt;
+                         }
+                       }
+                       return cnt;
+                     });
+}
+
+template <bool WHOLE>
+__device__ __forceinline__ u32 mark_fixed_any(unsigned char* __restrict__ B,
+                                              const MarkCtx& c, const uint4& w) {
+  const bool two = (w.w >> 24) == 2;
+  switch ((w.w >> 16) & 0xFFu) {
+    case 0: return mark_fixed<0, 1, WHOLE>(B, c, w);
+    case 1:
+      return two ? mark_fixed<1, 2, WHOLE>(B, c, w)
+                 : mark_fixed<1, 1, WHOLE>(B, c, w);
+    case 2: return mark_fixed<2, 2, WHOLE>(B, c, w);
+    case 3: return mark_fixed<3, 2, WHOLE>(B, c, w);
+    case 4: return mark_fixed<4, 2, WHOLE>(B, c, w);
+    case 5: return mark_fixed<5, 2, WHOLE>(B, c, w);
+    case 6: return mark_fixed<6, 2, WHOLE>(B, c, w);
+    default: return mark_fixed<7, 2, WHOLE>(B, c, w);
+  }
+}
+
+// A warp's items of one segment of len periods (WHOLE: SEG of them).
+template <bool WHOLE, int SEG>
+__device__ __forceinline__ u32 mark_segment(unsigned char* __restrict__ B,
+                                            const unsigned short* off16,
+                                            const DevEngine& e, u32 len) {
+  const u32 wl = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint4* work = reinterpret_cast<const uint4*>(e.mwork);
+  const u32 end = __ldg(e.mwoff + wid + 1);
+  u32 i = __ldg(e.mwoff + wid), cnt = 0;
+  if (i >= end) return 0;
+  const MarkCtx c{off16, e.mq, e.mres, e.qlim, WHOLE ? (u32)SEG : len};
+  const u32* mpair = e.mpair;
+  uint4 next = __ldg(work + i);
+  while (i < end) {
+    const uint4 w = next;
+    if (++i < end) next = __ldg(work + i);   // in flight meanwhile
+    const u32 kind = w.x & 0xFFu;
+    if (kind == MARK_FIXED) {
+      cnt += mark_fixed_any<WHOLE>(B, c, w);
+      continue;
+    }
+    const u32 hit0 = w.w & 0xFFFFu, K = (w.w >> 16) & 0xFFu, E = w.w >> 24;
+    const auto many = [&](u32 h, u32 q) {
+      return WHOLE ? mark_many<SEG>(B, h + hit0 * q, q, K, E)
+                   : mark_short(B, h + hit0 * q, q, K, E, len);
+    };
+    if (kind == MARK_PAIRS) {
+      const u32 x = __ldg(mpair + w.z + wl), slot = x >> 16;
+      const u32 q = __ldg(c.mq + slot) & 0xFFFFu;
+      const u32 h = (x & 0xFFFFu) - off16[slot];
+      if (q < c.qlim) cnt += many(min(h, h + q), q);
+    } else {
+      cnt += mark_blocks(c, (w.x >> 8) & 0xFFu, w.x >> 16, w.y, w.z, many);
+    }
+  }
+  return cnt;
+}
+
+// The 64 map bytes of word w as bits: four 16-byte loads, their order
+// rotated by the thread so that eight lanes at a stride of 64 bytes touch
+// all the banks.
+__device__ __forceinline__ u64 map_bits(const unsigned char* B, u32 w) {
+  const uint4* b = reinterpret_cast<const uint4*>(B + 64 * w);
+  const u32 rot = (threadIdx.x >> 1) & 3u;
+  u64 m = 0;
+#pragma unroll
+  for (u32 j = 0; j < 4; ++j) {
+    const uint4 x = b[(j + rot) & 3u];   // bytes are 0 or 1
+    const u32 k = 0x10204080u;
+    const u32 r = ((x.x * k) >> 28) | ((x.y * k) >> 28 << 4) |
+                  ((x.z * k) >> 28 << 8) | ((x.w * k) >> 28 << 12);
+    m |= (u64)r << (16 * j);
+  }
+  return rot ? (m << (16 * rot)) | (m >> (64 - 16 * rot)) : m;
+}
+
 // NS pattern primes, SEG periods per segment; the engine descriptor's NS
-// and marking tables (mq, mitems) must be the ones of this variant.
+// and marking tables (mq, mwork) must be the ones of this variant.
 template <int P0, int NS, int SEG>
 __global__ void __launch_bounds__(kBlock, 3) k_mark(SieveArgs a) {
   constexpr int WPT = SEG / (64 * kBlock);  // pattern words per thread
@@ -142,7 +313,6 @@ __global__ void __launch_bounds__(kBlock, 3) k_mark(SieveArgs a) {
       if (!stage_patterns<pat_bytes<P0, NS>()>(spat, eg.pat, &S.mbar, &S.status,
                                                phase, a.ctr))
         return;
-      for (u32 i = tid; i < (u32)NS; i += kBlock) S.minv[i] = eg.pat_minv[i];
       for (u32 i = tid; i <= eg.sbits_words; i += kBlock)
         S.sbits[i] = i < eg.sbits_words ? eg.sbits[i] : 0u;
       __syncthreads();
@@ -150,47 +320,33 @@ __global__ void __launch_bounds__(kBlock, 3) k_mark(SieveArgs a) {
     }
     const DevEngine e = eg;
     const u32* __restrict__ xq = a.xq + it.xq_off;
+    const u32* __restrict__ kq = xq + mark_tests_at(e.nslots);
     const u64 tl = task - a.task_prefix[S.item];
     const u32 lane = (u32)(tl % e.L);
     const u64 chunk = tl / e.L;
     const u64 R = e.lanes[lane];
     const u64 u_start = chunk * (u64)SEG * a.seg_per_task;
     const u64 u_end = min((u64)it.U, u_start + (u64)SEG * a.seg_per_task);
-    // marked primes: indices [NS, NPm), off16 / mq slots [pbeg, pend)
-    const u32 pbeg = (u32)(NS - kNSMin), pend = e.NPm - kNSMin;
-    // the lane's index shift and first-segment table index for every
-    // pattern prime: ((u + s_l) * 64^-1) mod q, s_l carrying 64^-1 already
-    if (tid < NS) {
-      const PrimeRec pr = e.recs[tid];
-      u32 x = xq[tid] + fk_bmod(R, pr.q, pr.magic);
-      x = min(x, x - pr.q);
-      const u32 sh = fk_mulmod(x, S.minv[tid], pr.q, pr.magic);
-      S.lsh[tid] = sh;
-      u32 p = fk_mulmod(fk_bmod(u_start, pr.q, pr.magic),
-                        __ldg(e.pat_i64 + tid), pr.q, pr.magic) + sh;
-      S.ph[tid] = min(p, p - pr.q);
-    }
-    // the first hit offset of every marked prime in the first segment
-    for (u32 pi = pbeg + tid; pi < pend; pi += kBlock) {
-      const u32 i = kNSMin + pi;
-      const PrimeRec pr = e.recs[i];
-      u32 x = xq[i] + fk_bmod(R, pr.q, pr.magic);
-      x = min(x, x - pr.q);
-      const u32 sh = fk_mulmod(x, __ldg(e.minv_all + i), pr.q, pr.magic);
-      u32 o = fk_bmod(u_start, pr.q, pr.magic) + sh;
-      S.off16[pi] = (unsigned short)min(o, o - pr.q);
-    }
+    // the line offset of the task's first period: one scaled residue gives
+    // each pattern prime's table index and each slot's first hit offset
+    const u64 v0 = u_start * e.M + R;
+    const u32 vl = (u32)v0 & ((1u << kRedcSplit) - 1u);
+    const u32 vh = (u32)(v0 >> kRedcSplit);
+    if (tid < NS) S.ph[tid] = redc_residue(load_rec(e.prec + tid), xq[tid], vl, vh);
+    for (u32 s = e.slot0 + tid; s < e.nslots; s += kBlock)
+      S.off16[s] = (unsigned short)redc_residue(
+          load_rec(e.mrec + s), __ldg(xq + kNSMax + s), vl, vh);
     __syncthreads();
     for (u64 useg = u_start; useg < u_end; useg += SEG) {
       const u32 seg_len = (u32)min((u64)SEG, u_end - useg);
-      // (a) the pattern words WPT*tid ... WPT*tid + WPT - 1
-      // (a thread whose words all lie past the segment's end skips it:
-      // a short lane's last segment leaves most threads idle)
+      // (a) the pattern words tid, tid + kBlock, ... (a warp whose words all
+      // lie past the segment's end skips them: a short lane's last segment
+      // leaves most warps idle)
       u64 acc[WPT];
 #pragma unroll
       for (int k = 0; k < WPT; ++k) acc[k] = 0;
-      if (64u * WPT * (u32)tid < seg_len) {
-        PatSeg<P0, 0, NS, WPT>::words(spat, S.ph, (u32)(WPT * tid), acc);
+      if (64u * ((u32)tid & ~31u) < seg_len) {
+        PatSeg<P0, 0, NS, WPT>::words(spat, S.ph, (u32)tid, acc);
         nword += WPT;
       }
       // zero the byte map up to the segment's end
@@ -204,71 +360,19 @@ __global__ void __launch_bounds__(kBlock, 3) k_mark(SieveArgs a) {
         }
       }
       __syncthreads();
-      // (b) mark: the work entries round robin over the threads, the next
-      // two entries' loads in flight while this one's progression is
-      // written (an entry carries its prime and sub-range length: one load
-      // each).
-      // Entries come ordered by prime, so a warp's 32 consecutive entries
-      // share a hit class: from index nm2 on, a residue hits the segment
-      // at most twice (q >= SEG / 2), from nm1 on at most once (q >= SEG),
-      // and those are written by a fixed predicated sequence instead of
-      // the loops
-      {
-        const u32 nm = e.nmitems, nm2 = e.nm2, nm1 = e.nm1;
-        const u64* __restrict__ mit = reinterpret_cast<const u64*>(e.mitems);
-        unsigned char* __restrict__ B = S.bytes;
-        u32 cnt = 0;
-        u32 i = tid;
-        // two entries' loads in flight ahead of the one being written: a
-        // large prime's entry is a handful of instructions, too few to
-        // cover one L2 round trip
-        u64 w = i < nm ? __ldg(mit + i) : 0ull;
-        u64 w1 = i + kBlock < nm ? __ldg(mit + i + kBlock) : 0ull;
-        while (i < nm) {
-          const u32 inext = i + kBlock;
-          const u64 wn = w1;
-          w1 = inext + kBlock < nm ? __ldg(mit + inext + kBlock) : 0ull;
-          const u32 wl = (u32)w, wh = (u32)(w >> 32);
-          const u32 g = wl & 0xFFFFu, pi = (wl >> 16) & 0x1FFFu;
-          const u32 q = wh & 0xFFFFu;
-          const u32 off = S.off16[pi];
-          const u32 d = g - off;
-          u32 h = min(d, d + q);   // (g - off) mod q: the first hit
-          if (i >= nm2) {
-            // whole-segment entries of large primes: h < q, so h + q is
-            // the last possible hit (h + 2q >= 2q >= SEG)
-            if (h < seg_len) { B[h] = 1; ++cnt; }
-            if (i < nm1) {
-              h += q;
-              if (h < seg_len) { B[h] = 1; ++cnt; }
-            }
-          } else {
-            const u32 k = wl >> 29, sl = wh >> 16;
-            h += k * sl;
-            const u32 end = sl ? min(seg_len, (k + 1) * sl) : seg_len;
-            const u32 q2 = 2 * q, q3 = 3 * q, q4 = 4 * q;
-            for (; h + q3 < end; h += q4, cnt += 4) {
-              B[h] = 1;
-              B[h + q] = 1;
-              B[h + q2] = 1;
-              B[h + q3] = 1;
-            }
-            for (; h < end; h += q, ++cnt) B[h] = 1;
-          }
-          i = inext;
-          w = wn;
-        }
-        nmark += cnt;
-      }
+      // (b) mark
+      nmark += seg_len == SEG
+                   ? mark_segment<true, SEG>(S.bytes, S.off16, e, SEG)
+                   : mark_segment<false, SEG>(S.bytes, S.off16, e, seg_len);
       __syncthreads();
       // advance the offsets and phases to the next segment (nothing below
       // reads them before the next segment's barrier)
       if (useg + SEG < u_end) {
-        for (u32 pi = pbeg + tid; pi < pend; pi += kBlock) {
-          const u64 m = __ldg(reinterpret_cast<const u64*>(e.mq) + pi);
-          const u32 q = (u32)m & 0xFFFFu;
-          const u32 o = S.off16[pi] + (((u32)m >> 16) & 0xFFFFu);
-          S.off16[pi] = (unsigned short)min(o, o - q);
+        for (u32 s = e.slot0 + tid; s < e.nslots; s += kBlock) {
+          const u32 m = __ldg(e.mq + s);
+          const u32 q = m & 0xFFFFu;
+          const u32 o = S.off16[s] + (m >> 16);
+          S.off16[s] = (unsigned short)min(o, o - q);
         }
         if (tid < NS) {
           const PrimeRec pr = e.recs[tid];
@@ -279,17 +383,10 @@ __global__ void __launch_bounds__(kBlock, 3) k_mark(SieveArgs a) {
       // (c) extract
 #pragma unroll
       for (int k = 0; k < WPT; ++k) {
-        const u32 w = WPT * tid + k;
+        const u32 w = tid + k * kBlock;
         const u64 uw = useg + 64ull * w;
         if (uw >= u_end) continue;
-        const uint2* bw = reinterpret_cast<const uint2*>(S.bytes + 64 * w);
-        u64 m = 0;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const uint2 b = bw[j];
-          const u64 x = ((u64)b.y << 32) | b.x;  // bytes are 0 or 1
-          m |= ((x * 0x0102040810204080ull) >> 56) << (8 * j);
-        }
+        const u64 m = map_bits(S.bytes, w);
         const u64 left = u_end - uw;
         u64 valid = left >= 64 ? ~0ull : ((1ull << left) - 1ull);
         if (uw == 0 && R < it.lo_off) valid &= ~1ull;
@@ -304,11 +401,11 @@ __global__ void __launch_bounds__(kBlock, 3) k_mark(SieveArgs a) {
           if (e.NPm < e.NP) {
             switch (e.kind) {
               case KIND_EULER:
-                alive = tail_alive<KIND_EULER>(v, e, xq, S.sbits, ntest); break;
+                alive = tail_alive<KIND_EULER>(v, e, kq, S.sbits, ntest); break;
               case KIND_DICKSON:
-                alive = tail_alive<KIND_DICKSON>(v, e, xq, S.sbits, ntest); break;
+                alive = tail_alive<KIND_DICKSON>(v, e, kq, S.sbits, ntest); break;
               default:
-                alive = tail_alive<KIND_AP>(v, e, xq, S.sbits, ntest); break;
+                alive = tail_alive<KIND_AP>(v, e, kq, S.sbits, ntest); break;
             }
           }
           if (!alive) continue;

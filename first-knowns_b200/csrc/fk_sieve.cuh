@@ -76,17 +76,36 @@ __device__ __forceinline__ u32 block_scan(u32 v, u32* s_warp, u32* total) {
   return base + x - v;
 }
 
-// The base of every (item, prime) of sieve items: X0 mod q for the primes
-// the marking sieve sweeps, else X0 * c1 mod q with the constants the prime
-// is used with -- the rounds' pattern index up to their first cut, the
-// per-candidate test past it (and past NPm for the marking sieve).
+// Entry i of an item's base-residue table: X0 * c1 mod q, the base folded
+// into the constants its prime is used with.  A rounds item has one entry
+// per prime: the pattern's index up to the first cut, the per-candidate test
+// past it.  A marking item has kNSMax entries for the pattern, one per slot
+// for the marks and one per prime for the tests past NPm.
+__host__ __device__ __forceinline__ u32 mark_tests_at(u32 nslots) {
+  return kNSMax + nslots;
+}
+__device__ __forceinline__ u32 base_entries(const DevEngine& e,
+                                            const DevItem& it) {
+  return !it.marked ? e.NP
+         : mark_tests_at(e.nslots) + (e.NPm < e.NP ? e.NP : 0u);
+}
 __device__ __forceinline__ u32 base_residue(const DevEngine& e,
                                             const DevItem& it, u32 i) {
-  const PrimeRec pr = e.recs[i];
-  const u32 x = fk_bmod128(it.X0_lo, it.X0_hi, pr.q, pr.magic, e.c64[i]);
-  if (it.marked && i < e.NPm) return x;
-  const bool pattern = !it.marked && i < e.rounds[0];
-  return fk_mulmod(x, pattern ? e.prec[i].c1 : e.trec[i].c1, pr.q, pr.magic);
+  u32 prime = i, c1;
+  if (!it.marked) {
+    c1 = i < e.rounds[0] ? e.prec[i].c1 : e.trec[i].c1;
+  } else if (i < (u32)kNSMax) {
+    c1 = e.prec[i].c1;
+  } else if (i < mark_tests_at(e.nslots)) {
+    prime = e.sprime[i - kNSMax];
+    c1 = e.mrec[i - kNSMax].c1;
+  } else {
+    prime = i - mark_tests_at(e.nslots);
+    c1 = e.trec[prime].c1;
+  }
+  const PrimeRec pr = e.recs[prime];
+  const u32 x = fk_bmod128(it.X0_lo, it.X0_hi, pr.q, pr.magic, e.c64[prime]);
+  return fk_mulmod(x, c1, pr.q, pr.magic);
 }
 
 // ---- per-candidate kill tests ------------------------------------------

@@ -57,7 +57,29 @@ constexpr int kSegPerTask = 8;    // marking: segments per task
 constexpr int kMarkPrimes = 6528; // marking: most primes one engine marks,
                                   // counted from pattern prime kNSMin
                                   // (every prime from 7 to 2^16 fits)
-constexpr int kMarkHits = 16;     // marking: least hits per work entry
+constexpr int kMarkSlots = 7168;  // marking: most prime slots (the primes in
+                                  // blocks of 32 by octave, each octave's
+                                  // last block filled up)
+constexpr int kMarkHits = 48;     // marking: hits per lane a pair item aims at
+constexpr int kMarkCost = 800;    // marking: instructions a block item aims at
+
+// One work item of the marking sieve, for one warp.  A lane's progressions
+// are the f residues of its prime in each of nblk blocks of 32 slots, or,
+// for the primes with many hits, one (slot, residue) pair of 32 of nearly
+// equal step.  Marked are the hits hit0 ... hit0 + K - 1 of each (all of
+// them inside a whole segment), then E more where they still lie inside it.
+enum MarkKind : uint32_t {
+  MARK_FIXED = 0,  // blocks, (K, E) one of (0, 1), (1, 1), (1 ... 7, 2);
+                   // hit0 = 0
+  MARK_BLOCKS = 1, // blocks, any K and E
+  MARK_PAIRS = 2,
+};
+struct alignas(16) MarkItem {
+  uint32_t kind;            // kind | nblk << 8 | f << 16
+  uint32_t block;           // the first
+  uint32_t res;             // first word of the residue pairs, or of the pairs
+  uint32_t hits;            // hit0 | K << 16 | E << 24
+};
 
 // Immutable per-engine tables (device-resident for the engine's life).
 struct DevEngine {
@@ -80,8 +102,6 @@ struct DevEngine {
   const TestRec* prec;            // [kNSMax] pattern primes, a = 1 / (64 M):
                                   // the scaled residue of v = 64 M w + R is
                                   // the table index of word w of lane R
-  const uint32_t* pat_minv;       // [kNSMax] (M mod q)^-1 * 64^-1 mod q
-  const uint32_t* pat_i64;        // [kNSMax] 64^-1 mod q
   const PrimeRec* recs;           // [NP]
   const uint32_t* c64;            // [NP] 2^64 mod q
   // per-candidate tests: the scaled residue r = (X0 + v) * a mod q
@@ -101,29 +121,24 @@ struct DevEngine {
   uint32_t ap_div;                // AP: a sieve prime divides d
   const uint32_t* rounds;         // [nrounds + 1] prime-index cuts
   const uint32_t* sbits;          // Euler: bitset of {x^2 + x : x < n}
-  // marking sieve (long lanes): primes [NS, NPm) are marked in a per-lane
-  // byte map; G lists hold each prime's forbidden residues of the PERIOD
-  // u for lane offset 0 (f * (M mod q)^-1 mod q)
-  uint32_t NPm, use_mark;
-  uint32_t nmitems;               // marking work entries of this batch
-  uint32_t nm2, nm1;              // entries before the first prime with
-                                  // q >= SEG / 2 (at most two hits per
-                                  // segment) and with q >= SEG (at most
-                                  // one); both relative to mitems
-  uint32_t pad3;
-  const uint32_t* minv_all;       // [NP] (M mod q)^-1 mod q
-  const uint32_t* gaux;           // [NP] offset | count << 24 into glist
-  const uint32_t* glist;
-  // tables of this batch's segment length SEG (one set per variant):
-  // [NPm - kNSMin] per prime from index kNSMin: q | (SEG mod q) << 16
-  const uint64_t* mq;
-  // [nmitems] work entries g | (prime - kNSMin) << 16 | sub-range k << 29 |
-  // q << 32 | S << 48: the hits u = g (mod q), shifted by the lane, of one
-  // forbidden period residue g inside sub-range k of length S (a multiple
-  // of q; S = 0 when the entry covers the whole segment), one 8-byte load
-  // per entry; ordered by prime, and the batch's pointer starts at the
-  // first prime past its pattern primes
-  const uint64_t* mitems;
+  // marking sieve (long lanes): the primes past the pattern are marked in a
+  // per-lane byte map, up to index NPm (q below qlim)
+  uint32_t NPm, use_mark, qlim;
+  // the marked primes sit in slots, 32 to a block: a block's primes are of
+  // one octave and of (nearly) one residue count, a short list repeating its
+  // last residue and a short block its last prime (a mark is idempotent)
+  uint32_t nslots, slot0;         // slot0: the first slot this batch marks
+  const TestRec* mrec;            // [nslots] a = 1 / M: the scaled residue of
+                                  // v = M u + R is the offset of the period u
+                                  // in the prime's hits
+  const uint32_t* sprime;         // [nslots] prime index
+  const uint32_t* mres;           // per block, word (j / 2) * 32 + lane: the
+                                  // lane's forbidden period residues j, j + 1
+  const uint32_t* mpair;          // residue | slot << 16
+  // tables of this batch's segment length SEG (one set per variant)
+  const uint32_t* mq;             // [nslots] q | (SEG mod q) << 16
+  const MarkItem* mwork;          // each warp's items one after the other
+  const uint32_t* mwoff;          // [9] where each warp's begin, and the end
 };
 
 // One unit of work: a sub-range of one engine's line.
@@ -139,9 +154,8 @@ struct DevItem {
                                   // t + lane_threads, ... of its block
   uint64_t nchunk;                // chains per lane
   uint64_t task0, ntask;          // first task, task count (rounds: blocks)
-  uint64_t xq_off;                // this item's base-residue table: X0 mod q
-                                  // of the primes sieved by pattern or mark,
-                                  // X0 * c1 mod q of the primes tested
+  uint64_t xq_off;                // this item's base-residue table
+                                  // (base_residue, fk_sieve.cuh)
   uint32_t marked;                // 1: the marking kernel sweeps this item
   uint32_t run;                   // rounds: blocks a warp claims at once
   uint64_t nchunk_u;              // marking: u-chunks per lane
