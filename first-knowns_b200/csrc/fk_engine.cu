@@ -19,6 +19,7 @@
 #include "fk_internal.h"
 #include "fk_launch.h"
 #include "fk_mark.cuh"
+#include "fk_rest.cuh"
 #include "fk_sieve.cuh"
 #include "fk_types.h"
 
@@ -680,6 +681,7 @@ static fk_status build_engine(fk_engine* e) {
   d.xxmax = xxmax;
   d.pat_words = (u32)pat.size();
   d.sbits_words = (u32)sbits.size();
+  sbits.push_back(0);   // the word every larger residue is looked up in
   d.two_pass = p.two_pass;
   d.M = e->M;
   d.W = e->W;
@@ -812,6 +814,8 @@ struct fk_batch {
   DevBuf<u32> d_cand_item;
   DevBuf<OutRec> d_out;
   DevBuf<u32> d_item_count, d_item_fill;
+  DevBuf<u64> d_rest_key;       // k_rest's list
+  DevBuf<u32> d_rest_item, d_rest_start, d_rest_state;
   DevBuf<u64> d_item_off, d_sorted, d_scratch;
   DevBuf<u32> d_nb, d_bcount, d_bfill, d_nbuckets;
   DevBuf<u64> d_bbase, d_boff;
@@ -913,6 +917,9 @@ static fk_status batch_init(fk_batch* b, fk_engine* const* engines,
   }
   FK_CUDA(b->d_task_ctr.ensure(8) == FK_OK ? cudaSuccess : cudaErrorMemoryAllocation);
   FK_CUDA(b->d_nitems.ensure(4) == FK_OK ? cudaSuccess : cudaErrorMemoryAllocation);
+  for (fk_status st : {b->d_rest_key.ensure(kRestCap), b->d_rest_item.ensure(kRestCap),
+                       b->d_rest_start.ensure(kRestCap), b->d_rest_state.ensure(kRestCap)})
+    if (st) return st;
   FK_CUDA(b->h_ctr.ensure(1) == FK_OK ? cudaSuccess : cudaErrorMemoryAllocation);
   static bool attrs_done = false;
   if (!attrs_done) {
@@ -928,6 +935,8 @@ static void batch_free(fk_batch* b) {
   if (b->graph) cudaGraphDestroy(b->graph);
   b->d_items.release(); b->d_dense.release(); b->d_sieve.release();
   b->d_xq.release(); b->d_cand_key.release(); b->d_cand_item.release();
+  b->d_rest_key.release(); b->d_rest_item.release(); b->d_rest_start.release();
+  b->d_rest_state.release();
   b->d_out.release(); b->d_item_count.release(); b->d_item_fill.release();
   b->d_item_off.release(); b->d_sorted.release(); b->d_scratch.release();
   b->d_nb.release(); b->d_bcount.release(); b->d_bfill.release();
@@ -1175,6 +1184,7 @@ static fk_status enqueue(fk_batch* b, bool capturing = false) {
                                           b->d_cand_key.p, b->d_cand_item.p,
                                           b->cand_cap, b->d_ctr);
   }
+  SieveArgs rest{};  // what k_rest shares with the rounds launches
   u64 blocks0 = 0;   // the rounds families' items share one counter array
   for (int f = 0; f < 8; ++f) {
     Family& F = b->fam[f];
@@ -1197,6 +1207,11 @@ static fk_status enqueue(fk_batch* b, bool capturing = false) {
     a.block_ctr = b->d_block_ctr.p + blocks0;
     if (!F.mark) blocks0 += F.idx.size();
     a.warp_queue = b->tune.warp_queue;
+    a.rest_key = b->d_rest_key.p;
+    a.rest_item = b->d_rest_item.p;
+    a.rest_start = b->d_rest_start.p;
+    a.rest_state = b->d_rest_state.p;
+    a.rest_cap = kRestCap;
     a.seg_per_task = b->tune.seg_per_task;
     const u64 grid =
         F.mark ? std::min<u64>(a.ntask, (u64)b->nsm * b->tune.mark_ctas_per_sm)
@@ -1210,6 +1225,14 @@ static fk_status enqueue(fk_batch* b, bool capturing = false) {
     else
       FK_CUDA(launch_sieve(P0, b->tune.pattern_primes, (u32)grid, s, a));
     FK_CUDA(record(b->fev[2 * f + 1], s, capturing));
+    if (!F.mark) rest = a;
+  }
+  if (rest.items) {   // some item went through the rounds
+    u32 max_np = 0;
+    for (const fk_engine* e : b->engines)
+      max_np = std::max(max_np, (u32)e->sieve.size());
+    ++nl;
+    k_rest<<<b->nsm * 3, kBlock, 0, s>>>(rest, max_np);
   }
   FK_CUDA(cudaGetLastError());
   FK_CUDA(record(b->ev[1], s, capturing));

@@ -279,6 +279,14 @@ struct SieveArgs {
   DevCounters* ctr;
   unsigned long long* task_ctr;   // marking: next task
   unsigned long long* block_ctr;  // rounds: [nitems] blocks claimed per item
+  // rounds: candidates left in short queues, for k_rest, with the first prime
+  // each was not tested against
+  u64* rest_key;
+  u32* rest_item;
+  u32* rest_start;
+  u32* rest_state;
+  u32 rest_cap;                   // 0: every warp finishes its own
+  u32 pad2;
   u32 warp_queue;     // compaction: warp queues below this go one
                       // candidate per warp
   u32 seg_per_task;   // marking: segments per task
@@ -295,6 +303,8 @@ constexpr u32 kWarps = kBlock / 32;
 constexpr u32 kWq = 192;
 constexpr u32 kWq2 = 64;
 constexpr u32 kColSlots = 16;
+constexpr u32 kRestFew = 8;        // fewer candidates than this, with more than
+constexpr u32 kRestPrimes = 1024;  // these primes to go, are listed for k_rest
 
 // What a block needs of its item and engine, read from shared memory where
 // it is used: held in registers these values would be spilled around the
@@ -403,17 +413,36 @@ __device__ __forceinline__ u32 drain_groups(u64* Q, u32 n, const TestCtx& c,
   }
 }
 
-// A warp's n candidates (its first or second queue) against every prime
-// from index `at` on, in place, and the survivors into the global list: 32 primes at a time, then, once
+// Append n of the warp's candidates, tested up to prime `at`, to the list
+// k_rest finishes, as far as it has room; returns how many it took, from the
+// front.  (None when no prime is left: the list holds work, not survivors.)
+__device__ __forceinline__ u32 list_rest(const SieveSmem& S, const u64* Q,
+                                         u32 n, u32 at, const SieveArgs& a) {
+  const u32 lane = threadIdx.x & 31;
+  if (n == 0 || a.rest_cap == 0 || at >= S.NP) return 0;
+  u64 base = 0;
+  if (lane == 0) base = atomicAdd(&a.ctr->nrest, (unsigned long long)n);
+  base = __shfl_sync(0xffffffffu, base, 0);
+  const u32 m = base < a.rest_cap ? (u32)min((u64)n, a.rest_cap - base) : 0u;
+  for (u32 i = lane; i < m; i += 32) {
+    a.rest_key[base + i] = Q[i];
+    a.rest_item[base + i] = S.blk.gitem;
+    a.rest_start[base + i] = at;
+    a.rest_state[base + i] = 0;
+  }
+  return m;
+}
+
+// n candidates of a warp's first or second queue, past the first `skip`,
+// against every prime from index `at` on, in place, and the survivors into the global list: 32 primes at a time, then, once
 // few candidates die among 128 primes (S.deep), kDeep groups of 32 at a
 // time (fewer votes, more loads in flight).
 template <int KIND>
-__device__ __noinline__ void drain_rest(bool second, u32 n, u32 at,
-                                        u64* cand_key, u32* cand_item,
-                                        u64 cand_cap, DevCounters* ctr) {
+__device__ __noinline__ void drain_rest(bool second, u32 skip, u32 n, u32 at,
+                                        const SieveArgs& a) {
   SieveSmem& S = sieve_smem_ref();
   const u32 lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  u64* Q = second ? S.queue2 + wid * kWq2 : S.queue + wid * kWq;
+  u64* Q = (second ? S.queue2 + wid * kWq2 : S.queue + wid * kWq) + skip;
   const TestCtx c = S.ctx;
   const u32 NP = S.NP;
   u32 ntest = 0;
@@ -421,7 +450,16 @@ __device__ __noinline__ void drain_rest(bool second, u32 n, u32 at,
   n = drain_groups<KIND>(Q, n, c, S.sbits, at, deep, ntest);
   constexpr u32 kDeep = KIND == KIND_DICKSON ? 2 : 4;
   at = deep;
+  bool room = true;
   for (; n > 0 && at + 32 * kDeep <= NP; at += 32 * kDeep) {
+    if (room && n < kRestFew && NP - at > kRestPrimes) {
+      // too few to be worth this warp's time: k_rest shares them out
+      const u32 m = list_rest(S, Q, n, at, a);
+      Q += m;
+      n -= m;
+      room = n == 0;
+      if (n == 0) break;
+    }
     Prime<KIND> p[kDeep];
 #pragma unroll
     for (u32 j = 0; j < kDeep; ++j) p[j].load(c, at + 32 * j + lane);
@@ -446,14 +484,14 @@ __device__ __noinline__ void drain_rest(bool second, u32 n, u32 at,
   // survivors: one atomic per warp
   if (n) {
     u64 base = 0;
-    if (lane == 0) base = atomicAdd(&ctr->ncand, (unsigned long long)n);
+    if (lane == 0) base = atomicAdd(&a.ctr->ncand, (unsigned long long)n);
     base = __shfl_sync(0xffffffffu, base, 0);
     for (u32 idx = lane; idx < n; idx += 32) {
-      if (base + idx < cand_cap) {
-        cand_key[base + idx] = Q[idx];
-        cand_item[base + idx] = S.blk.gitem;
+      if (base + idx < a.cand_cap) {
+        a.cand_key[base + idx] = Q[idx];
+        a.cand_item[base + idx] = S.blk.gitem;
       } else {
-        atomicOr(&ctr->overflow, 1u);
+        atomicOr(&a.ctr->overflow, 1u);
       }
     }
   }
@@ -470,15 +508,15 @@ __device__ __noinline__ void drain_rest(bool second, u32 n, u32 at,
 // deeper primes' records: there each lane holds one prime and every
 // candidate is tested against the warp's 32 primes at once, so no lane
 // idles behind a dead candidate.  `final` (the item's end) empties both
-// queues; a first queue shorter than a.warp_queue then skips the rounds.
+// queues, what is left past the staged primes into the list of k_rest while
+// that has room.
 // Warp-synchronous: every lane calls it.  Not inlined: the pattern loop
 // around it keeps its NS table indexes in registers and runs between
 // drains.
 template <int KIND>
-__device__ __noinline__ void warp_drain(bool final, u32 wq_short, u64* cand_key,
-                                        u32* cand_item, u64 cand_cap,
-                                        DevCounters* ctr) {
+__device__ __noinline__ void warp_drain(bool final, const SieveArgs& a) {
   SieveSmem& S = sieve_smem_ref();
+  const u32 wq_short = a.warp_queue;
   const u32 lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const u32 lt = (1u << lane) - 1u;
   u64* Q = S.queue + wid * kWq;
@@ -486,8 +524,7 @@ __device__ __noinline__ void warp_drain(bool final, u32 wq_short, u64* cand_key,
   u32 n = S.qn[wid], n2 = S.qn2[wid];
   const u32 NP = S.NP, first = __ldg(S.rounds);
   const u32 nstaged = min((u32)kStaged, NP - first);
-  u32 from = first;
-  if (n > 0 && (!final || n >= wq_short)) {
+  if (n > 0) {
     const TestCtx c = S.ctx;
     u32 ntest = 0, at = 0;
     for (u32 r = 0; n >= wq_short && n > 0 && at < nstaged; ++r) {
@@ -537,25 +574,26 @@ __device__ __noinline__ void warp_drain(bool final, u32 wq_short, u64* cand_key,
     }
     ntest = __reduce_add_sync(0xffffffffu, ntest);
     if (lane == 0) S.ntest[wid] += ntest;
-    from = first + nstaged;
   }
-  if (n >= kWq2 / 2) {   // enough by themselves
-    drain_rest<KIND>(false, n, from, cand_key, cand_item, cand_cap, ctr);
+  const u32 done = first + nstaged;
+  if (final) {
+    // the warp's last of the item: k_rest shares them out
+    u32 m = list_rest(S, Q, n, done, a);
+    if (m < n) drain_rest<KIND>(false, m, n - m, done, a);
+    m = list_rest(S, Q2, n2, done, a);
+    if (m < n2) drain_rest<KIND>(true, m, n2 - m, done, a);
+    n = n2 = 0;
+  } else if (n >= kWq2 / 2) {   // enough by themselves
+    drain_rest<KIND>(false, 0, n, done, a);
     n = 0;
   }
   if (n2 + n > kWq2) {
-    drain_rest<KIND>(true, n2, first + nstaged, cand_key, cand_item, cand_cap,
-                     ctr);
+    drain_rest<KIND>(true, 0, n2, done, a);
     n2 = 0;
   }
   if (lane < n) Q2[n2 + lane] = Q[lane];  // n < kWq2 / 2 = 32
   __syncwarp();
   n2 += n;
-  if (final && n2 > 0) {
-    drain_rest<KIND>(true, n2, n > 0 ? from : first + nstaged, cand_key,
-                     cand_item, cand_cap, ctr);
-    n2 = 0;
-  }
   if (lane == 0) {
     S.qn[wid] = 0;
     S.qn2[wid] = n2;
@@ -569,15 +607,9 @@ __device__ __forceinline__ void drain_any(SieveSmem& S, bool final,
                                           const SieveArgs& a) {
   if ((S.qn[threadIdx.x >> 5] | S.qn2[threadIdx.x >> 5]) == 0) return;
   switch (S.kind) {
-    case KIND_EULER:
-      return warp_drain<KIND_EULER>(final, a.warp_queue, a.cand_key,
-                                    a.cand_item, a.cand_cap, a.ctr);
-    case KIND_DICKSON:
-      return warp_drain<KIND_DICKSON>(final, a.warp_queue, a.cand_key,
-                                      a.cand_item, a.cand_cap, a.ctr);
-    default:
-      return warp_drain<KIND_AP>(final, a.warp_queue, a.cand_key,
-                                 a.cand_item, a.cand_cap, a.ctr);
+    case KIND_EULER: return warp_drain<KIND_EULER>(final, a);
+    case KIND_DICKSON: return warp_drain<KIND_DICKSON>(final, a);
+    default: return warp_drain<KIND_AP>(final, a);
   }
 }
 

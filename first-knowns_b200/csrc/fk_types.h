@@ -48,6 +48,7 @@ constexpr int kWarpMode = 32;     // warp queue below which a candidate
 constexpr int kSbits = 512;       // Euler: most words of the {x^2 + x} bitset
 constexpr int kStaged = 128;      // rounds: test primes held in shared memory
 constexpr int kStagedBits = 1536; // Dickson: words of their residue bitmaps
+constexpr int kRestCap = 1 << 17;  // rounds: candidates k_rest's list holds
 constexpr int kMaxRun = 32;       // rounds: most blocks a warp claims at once
 constexpr int kSeg = 32768;       // marking: periods per shared segment
                                   // (default; variants 16384 and 65536)
@@ -181,6 +182,7 @@ struct DevCounters {
   unsigned long long sprp_values; // values strong-tested
   unsigned long long marks;       // marking-sieve byte marks
   unsigned long long class_next;  // SPRP stage: next candidate chunk
+  unsigned long long nrest;       // candidates listed for k_rest
   unsigned long long nexact;      // candidates listed for the exact tests
   unsigned long long exact_next;  // exact tests: next candidate chunk
 };

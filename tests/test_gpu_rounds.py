@@ -62,3 +62,28 @@ def test_ap(n, q2, d):
     want = ref.survivors(lo, span).tolist()
     _check(fk_abi.Engine(fk_abi.AP, n, q2=q2, d=d, sieve="rounds"), lo,
            lo + span, want)
+
+
+def test_the_shared_out_rest_with_mixed_engines_and_a_full_list():
+    """Candidates left in the warps' queues go to one list over all items of
+    a batch: engines of every kind and depth side by side, in numbers that
+    leave the list nearly empty and that overflow it (131072 entries; 256
+    items leave up to 8 warps' queues on every CTA that joins them)."""
+    engs = [fk_abi.Engine(fk_abi.EULER, 7, sieve="rounds"),
+            fk_abi.Engine(fk_abi.DICKSON, 5, q2=1 << 18, sieve="rounds"),
+            fk_abi.Engine(fk_abi.AP, 6, q2=300, sieve="rounds"),
+            fk_abi.Engine(fk_abi.AP, 5, q2=1 << 17, sieve="rounds"),
+            fk_abi.Engine(fk_abi.EULER, 3, sieve="rounds")]
+    batch = fk_abi.Batch(engs)
+    for items, span in ((5, 3000), (256, 3 * 10 ** 7)):
+        specs = []
+        for i in range(items):
+            k = i % len(engs)
+            lo = 10 ** 12 + i * 10 ** 9
+            specs.append((k, fk_abi.MODE_SIEVE, 0, 0, lo,
+                          lo + (span // 100 if k == 1 else span)))
+        for graph in (False, True):
+            rows = batch.run(specs, graph=graph)
+            for (k, _m, _t, _c, lo, hi), (off, _d) in list(
+                    zip(specs, rows))[::7 if items > 9 else 1]:
+                assert off.tolist() == engs[k].sieve(lo, hi).tolist()
