@@ -610,7 +610,7 @@ static fk_status build_engine(fk_engine* e) {
   std::vector<u32> c64(NP), lists, boff, bits;
   u32 ap_div = 0;
   if (e->kind == KIND_AP)
-    for (u32 i = 0; i < NP; ++i) ap_div |= e->d % e->sieve[i] == 0;
+    for (u32 i = kNSMin; i < NP; ++i) ap_div |= e->d % e->sieve[i] == 0;
   if (e->kind == KIND_DICKSON || ap_div) filt.resize(NP);
   for (u32 i = 0; i < NP; ++i) {
     const u32 q = e->sieve[i];
@@ -625,7 +625,7 @@ static fk_status build_engine(fk_engine* e) {
     if (e->kind == KIND_AP) {
       const u64 dq = (u64)(e->d % q);
       a = q - (dq ? invmod(dq, q) : 1);
-      if (!dq) filt[i].f0 = 1;
+      if (!dq && ap_div) filt[i].f0 = 1;
     }
     trec[i] = redc_rec(q, a);
     if (e->kind != KIND_DICKSON || i < (u32)kNSMin) continue;

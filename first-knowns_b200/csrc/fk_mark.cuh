@@ -80,7 +80,7 @@ struct PatSeg<P0, NS, NS, WPT> {
                                                u64*) {}
 };
 
-template <int KIND>
+template <int MODE>
 __device__ __forceinline__ bool tail_alive(u64 v, const DevEngine& e,
                                            const u32* __restrict__ kq,
                                            const u32* s_sbits, u64& ntest) {
@@ -90,9 +90,9 @@ __device__ __forceinline__ bool tail_alive(u64 v, const DevEngine& e,
   const u32 vh = (u32)(v >> kRedcSplit);
   for (u32 i = e.NPm; i < e.NP; ++i) {
     ++ntest;
-    Prime<KIND> p;
+    Prime<MODE> p;
     p.load(c, i);
-    if (p.kills(c, s_sbits, vl, vh))
+    if (any_kill<MODE, 1>(&p, c, s_sbits, vl, vh))
       return false;
   }
   return true;
@@ -399,13 +399,16 @@ __global__ void __launch_bounds__(kBlock, 3) k_mark(SieveArgs a) {
           const u64 v = (uw + b) * e.M + R;
           bool alive = true;
           if (e.NPm < e.NP) {
-            switch (e.kind) {
-              case KIND_EULER:
-                alive = tail_alive<KIND_EULER>(v, e, kq, S.sbits, ntest); break;
-              case KIND_DICKSON:
-                alive = tail_alive<KIND_DICKSON>(v, e, kq, S.sbits, ntest); break;
+            switch (test_mode(e, e.NPm)) {
+              case TEST_EULER:
+              case TEST_EULER_LOW:
+                alive = tail_alive<TEST_EULER_LOW>(v, e, kq, S.sbits, ntest); break;
+              case TEST_DICKSON:
+                alive = tail_alive<TEST_DICKSON>(v, e, kq, S.sbits, ntest); break;
+              case TEST_AP:
+                alive = tail_alive<TEST_AP>(v, e, kq, S.sbits, ntest); break;
               default:
-                alive = tail_alive<KIND_AP>(v, e, kq, S.sbits, ntest); break;
+                alive = tail_alive<TEST_AP_DIV>(v, e, kq, S.sbits, ntest); break;
             }
           }
           if (!alive) continue;

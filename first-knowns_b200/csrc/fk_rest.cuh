@@ -21,26 +21,24 @@ constexpr u32 kRestDead = 0x80000000u;
 
 // The candidates `alive` (bits; lane i holds candidate i's offset v) against
 // the primes [at, end): those no prime kills.
-template <int KIND>
+template <int MODE>
 __device__ __forceinline__ u32 rest_group(const TestCtx& c, const u32* sbits,
                                           u64 v, u32 alive, u32 at, u32 end,
                                           u32& ntest) {
   const u32 lane = threadIdx.x & 31;
   const u32 vl = (u32)v & ((1u << kRedcSplit) - 1u);
   const u32 vh = (u32)(v >> kRedcSplit);
-  constexpr u32 kDeep = 4;
+  constexpr int kDeep = 4;
   for (; at < end && alive; at += 32 * kDeep) {
-    Prime<KIND> p[kDeep];
+    Prime<MODE> p[kDeep];
 #pragma unroll
-    for (u32 j = 0; j < kDeep; ++j)   // past the end: the last prime again
+    for (int j = 0; j < kDeep; ++j)   // past the end: the last prime again
       p[j].load(c, min(at + 32 * j + lane, end - 1));
     for (u32 m = alive; m; m &= m - 1) {
       const u32 i = __ffs((int)m) - 1;
       const u32 l = __shfl_sync(0xffffffffu, vl, i);
       const u32 h = __shfl_sync(0xffffffffu, vh, i);
-      bool kill = false;
-#pragma unroll
-      for (u32 j = 0; j < kDeep; ++j) kill |= p[j].kills(c, sbits, l, h);
+      const bool kill = any_kill<MODE, kDeep>(p, c, sbits, l, h);
       ntest += kDeep;
       if (__any_sync(0xffffffffu, kill)) alive &= ~(1u << i);
     }
@@ -83,15 +81,21 @@ __global__ void __launch_bounds__(kBlock)
       const TestCtx c{e.trec, e.filt, a.xq + it.xq_off, e.lists,
                       e.n, e.xxmax, e.sbits_words, e.ap_div};
       u32 alive;
-      switch (e.kind) {
-        case KIND_EULER:
-          alive = rest_group<KIND_EULER>(c, e.sbits, v, mask, from, end, ntest);
+      switch (test_mode(e, e.rounds[0])) {
+        case TEST_EULER:
+          alive = rest_group<TEST_EULER>(c, e.sbits, v, mask, from, end, ntest);
           break;
-        case KIND_DICKSON:
-          alive = rest_group<KIND_DICKSON>(c, e.sbits, v, mask, from, end, ntest);
+        case TEST_DICKSON:
+          alive = rest_group<TEST_DICKSON>(c, e.sbits, v, mask, from, end, ntest);
+          break;
+        case TEST_AP:
+          alive = rest_group<TEST_AP>(c, e.sbits, v, mask, from, end, ntest);
+          break;
+        case TEST_EULER_LOW:
+          alive = rest_group<TEST_EULER_LOW>(c, e.sbits, v, mask, from, end, ntest);
           break;
         default:
-          alive = rest_group<KIND_AP>(c, e.sbits, v, mask, from, end, ntest);
+          alive = rest_group<TEST_AP_DIV>(c, e.sbits, v, mask, from, end, ntest);
           break;
       }
       if (todo && item == it0) {

@@ -119,43 +119,51 @@ struct TestCtx {
   u32 n, xxmax, xxwords, ap_div;
 };
 
-// Is residue r on the prime's list?  The three filter bits settle nearly
-// every residue off it; the list itself (groups of four, padded with ~0) is
-// read only behind them.
-__device__ __forceinline__ bool list_kill(const ListFilter& f, u32 r,
-                                          const u32* __restrict__ lists) {
-  if (!((f.f0 >> (r & 31)) & (f.f1 >> ((r >> 5) & 31)) &
-        (f.f2 >> ((r >> 10) & 31)) & 1u))
-    return false;
+// Dickson: may residue h be on the prime's list (bit 0)?  The three filter
+// bits settle nearly every residue off it.
+__device__ __forceinline__ u32 list_maybe(const ListFilter& f, u32 h) {
+  return ((f.f0 >> (h & 31)) & (f.f1 >> ((h >> 5) & 31)) &
+          (f.f2 >> ((h >> 10) & 31))) & 1u;
+}
+// Is it?  (The list: groups of four, padded with ~0.)
+__device__ __forceinline__ bool list_has(const ListFilter& f, u32 h,
+                                         const u32* __restrict__ lists) {
   const uint4* l = reinterpret_cast<const uint4*>(lists) + (f.list & 0xFFFFFFu);
   const u32 cnt = f.list >> 24;
   bool k = false;
   for (u32 c = 0; c < cnt; ++c) {
     const uint4 x = __ldg(l + c);
-    k |= (x.x == r) | (x.y == r) | (x.z == r) | (x.w == r);
+    k |= (x.x == h) | (x.y == h) | (x.z == h) | (x.w == h);
   }
   return k;
 }
 
-// Does prime i kill a value of scaled residue r (Euler, AP)?  sbits (shared
-// memory): Euler's bitset of {x^2 + x : x < n}.
-template <int KIND>
+// Does prime i kill a value of scaled residue r (not Dickson)?  sbits (shared
+// memory in the rounds): Euler's bitset of {x^2 + x : x < n}, its last word
+// (xxwords) zero.
+template <int MODE>
 __device__ __forceinline__ bool kill_test(const TestCtx& c, const u32* sbits,
                                           u32 i, const TestRec& t, u32 r) {
   bool kill;
-  if (KIND == KIND_AP) {
+  if (MODE == TEST_AP || MODE == TEST_AP_DIV) {
     kill = r < c.n;
-    if (c.ap_div && kill && c.filt[i].f0) kill = r == 0;
+    if (MODE == TEST_AP_DIV && kill && c.filt[i].f0) kill = r == 0;
   } else {
-    // r = -x is killed when it is one of the x^2 + x: the bitset's last
-    // word (xxwords) is zero
+    // r = -x is killed when it is one of the x^2 + x, for the low primes
+    // also when r + q, r + 2q, ... is
     kill = (sbits[min(r >> 5, c.xxwords)] >> (r & 31)) & 1u;
-    // the primes up to max(x^2 + x): so are r + q, r + 2q, ...
-    if (t.q <= c.xxmax)
+    if (MODE == TEST_EULER_LOW)
       for (u32 s = r + t.q; s <= c.xxmax; s += t.q)
         kill |= (sbits[s >> 5] >> (s & 31)) & 1u;
   }
   return kill;
+}
+
+// The form an engine's tests take from prime `first` on.
+__device__ __forceinline__ u32 test_mode(const DevEngine& e, u32 first) {
+  if (e.kind == KIND_DICKSON) return TEST_DICKSON;
+  if (e.kind == KIND_AP) return e.ap_div ? TEST_AP_DIV : TEST_AP;
+  return first < e.NP && e.trec[first].q > e.xxmax ? TEST_EULER : TEST_EULER_LOW;
 }
 
 __device__ __forceinline__ TestRec load_rec(const TestRec* p) {
@@ -169,7 +177,7 @@ __device__ __forceinline__ ListFilter load_filt(const ListFilter* p) {
 }
 
 // One prime's data in registers.
-template <int KIND>
+template <int MODE>
 struct Prime {
   TestRec t;
   ListFilter f;   // Dickson only
@@ -178,23 +186,38 @@ struct Prime {
     i = p;
     t = load_rec(c.trec + p);
     k = __ldg(c.kq + p);
-    if (KIND == KIND_DICKSON) f = load_filt(c.filt + p);
-  }
-  // the same from the tables staged in shared memory, for prime first + j
-  __device__ __forceinline__ void load(const TestCtx& c, const TestRec* srec,
-                                       const u32* skq, u32 first, u32 j) {
-    i = first + j;
-    t = srec[j];
-    k = skq[j];
-    if (KIND == KIND_DICKSON) f = load_filt(c.filt + i);
-  }
-  __device__ __forceinline__ bool kills(const TestCtx& c, const u32* sbits,
-                                        u32 vl, u32 vh) const {
-    const u32 r = redc_residue(t, k, vl, vh);
-    if (KIND == KIND_DICKSON) return list_kill(f, min(r, t.q - r), c.lists);
-    return kill_test<KIND>(c, sbits, i, t, r);
+    if (MODE == TEST_DICKSON) f = load_filt(c.filt + p);
   }
 };
+
+// Does one of the lane's N primes kill the value?  Without a branch, but for
+// Dickson's lists, read behind one branch for all N.
+template <int MODE, int N>
+__device__ __forceinline__ bool any_kill(const Prime<MODE>* p, const TestCtx& c,
+                                         const u32* sbits, u32 vl, u32 vh) {
+  if (MODE == TEST_DICKSON) {
+    u32 h[N], maybe = 0;
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const u32 r = redc_residue(p[j].t, p[j].k, vl, vh);
+      h[j] = min(r, p[j].t.q - r);
+      maybe |= list_maybe(p[j].f, h[j]) << j;
+    }
+    bool kill = false;
+    if (maybe) {
+#pragma unroll
+      for (int j = 0; j < N; ++j)
+        if ((maybe >> j) & 1u) kill |= list_has(p[j].f, h[j], c.lists);
+    }
+    return kill;
+  }
+  bool kill = false;
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+    kill |= kill_test<MODE>(c, sbits, p[j].i, p[j].t,
+                            redc_residue(p[j].t, p[j].k, vl, vh));
+  return kill;
+}
 
 // ---- S1 helpers, unrolled over the compile-time pattern primes ----------
 // Padding of a variant's pattern tables: entry q + i repeats entry i, so a
@@ -330,14 +353,14 @@ struct SieveSmem {
   TestCtx ctx;            // the current item's tests
   const u32* rounds;
   u32 entry;              // the item joined
-  u32 skq[kStaged];
-  u32 sboff[kStaged];     // Dickson: the prime's first word in sbit
+  uint2 sk[kStaged];      // the base's residue; Dickson: the prime's first
+                          // word in sbit
   u32 sbit[kStagedBits];  // bit h: min(r, q - r) = h is killed
   u32 chain_w0[kBlock];
   u32 qn[kWarps], qn2[kWarps];  // queue lengths
   u32 pk[kNSMax];
   u32 sbits[kSbits + 1];
-  u32 NP, kind, deep;
+  u32 NP, mode, deep;
   u32 eng;
   u32 status;
   unsigned long long mbar;
@@ -363,21 +386,19 @@ __host__ __device__ constexpr u32 pat_bytes() {
 }
 
 // A warp's n candidates against the 32 primes its lanes hold: the survivors
-// compacted in place, their count returned.
-template <int KIND>
-__device__ __forceinline__ u32 test_group(u64* Q, u32 n, const TestCtx& c,
-                                          const u32* sbits,
-                                          const Prime<KIND>& p) {
+// compacted in place, their count returned.  kills(vl, vh): does the lane's
+// prime kill that value?
+template <typename F>
+__device__ __forceinline__ u32 test_group(u64* Q, u32 n, F kills) {
   const u32 lane = threadIdx.x & 31;
   u32 out = 0;
   for (u32 idx = 0; idx < n; idx += 2) {
     const bool two = idx + 1 < n;
     const u64 v = Q[idx], w = Q[two ? idx + 1 : idx];
-    const u32 vl = (u32)v & ((1u << kRedcSplit) - 1u);
-    const u32 vh = (u32)(v >> kRedcSplit);
-    const u32 wl = (u32)w & ((1u << kRedcSplit) - 1u);
-    const u32 wh = (u32)(w >> kRedcSplit);
-    const bool kv = p.kills(c, sbits, vl, vh), kw = p.kills(c, sbits, wl, wh);
+    const bool kv = kills((u32)v & ((1u << kRedcSplit) - 1u),
+                          (u32)(v >> kRedcSplit));
+    const bool kw = kills((u32)w & ((1u << kRedcSplit) - 1u),
+                          (u32)(w >> kRedcSplit));
     const bool dv = __any_sync(0xffffffffu, kv);
     const bool dw = __any_sync(0xffffffffu, kw) || !two;
     if (!dv) {
@@ -395,19 +416,21 @@ __device__ __forceinline__ u32 test_group(u64* Q, u32 n, const TestCtx& c,
 
 // A warp's n candidates against the primes [at, end), 32 at a time, the
 // next 32 primes' loads in flight meanwhile.  Returns the survivors' count.
-template <int KIND>
+template <int MODE>
 __device__ __forceinline__ u32 drain_groups(u64* Q, u32 n, const TestCtx& c,
                                             const u32* sbits, u32 at, u32 end,
                                             u32& ntest) {
   const u32 lane = threadIdx.x & 31;
   if (n == 0 || at >= end) return n;
-  Prime<KIND> p, next;
+  Prime<MODE> p, next;
   p.load(c, min(at + lane, end - 1));  // past the end: the last prime again
   for (;;) {
     at += 32;
     next.load(c, min(at + lane, end - 1));
     ntest += n;
-    n = test_group<KIND>(Q, n, c, sbits, p);
+    n = test_group(Q, n, [&](u32 vl, u32 vh) {
+      return any_kill<MODE, 1>(&p, c, sbits, vl, vh);
+    });
     if (at >= end || n == 0) return n;
     p = next;
   }
@@ -437,7 +460,7 @@ __device__ __forceinline__ u32 list_rest(const SieveSmem& S, const u64* Q,
 // against every prime from index `at` on, in place, and the survivors into the global list: 32 primes at a time, then, once
 // few candidates die among 128 primes (S.deep), kDeep groups of 32 at a
 // time (fewer votes, more loads in flight).
-template <int KIND>
+template <int MODE>
 __device__ __noinline__ void drain_rest(bool second, u32 skip, u32 n, u32 at,
                                         const SieveArgs& a) {
   SieveSmem& S = sieve_smem_ref();
@@ -447,8 +470,8 @@ __device__ __noinline__ void drain_rest(bool second, u32 skip, u32 n, u32 at,
   const u32 NP = S.NP;
   u32 ntest = 0;
   const u32 deep = min(max(S.deep, at), NP);
-  n = drain_groups<KIND>(Q, n, c, S.sbits, at, deep, ntest);
-  constexpr u32 kDeep = KIND == KIND_DICKSON ? 2 : 4;
+  n = drain_groups<MODE>(Q, n, c, S.sbits, at, deep, ntest);
+  constexpr int kDeep = MODE == TEST_DICKSON ? 2 : 4;
   at = deep;
   bool room = true;
   for (; n > 0 && at + 32 * kDeep <= NP; at += 32 * kDeep) {
@@ -460,17 +483,15 @@ __device__ __noinline__ void drain_rest(bool second, u32 skip, u32 n, u32 at,
       room = n == 0;
       if (n == 0) break;
     }
-    Prime<KIND> p[kDeep];
+    Prime<MODE> p[kDeep];
 #pragma unroll
-    for (u32 j = 0; j < kDeep; ++j) p[j].load(c, at + 32 * j + lane);
+    for (int j = 0; j < kDeep; ++j) p[j].load(c, at + 32 * j + lane);
     u32 out = 0;
     for (u32 idx = 0; idx < n; ++idx) {
       const u64 v = Q[idx];
       const u32 vl = (u32)v & ((1u << kRedcSplit) - 1u);
       const u32 vh = (u32)(v >> kRedcSplit);
-      bool kill = false;
-#pragma unroll
-      for (u32 j = 0; j < kDeep; ++j) kill |= p[j].kills(c, S.sbits, vl, vh);
+      const bool kill = any_kill<MODE, kDeep>(p, c, S.sbits, vl, vh);
       if (!__any_sync(0xffffffffu, kill)) {
         if (lane == 0) Q[out] = v;  // out <= idx: read already
         ++out;
@@ -480,7 +501,7 @@ __device__ __noinline__ void drain_rest(bool second, u32 skip, u32 n, u32 at,
     __syncwarp();
     n = out;
   }
-  n = drain_groups<KIND>(Q, n, c, S.sbits, at, NP, ntest);
+  n = drain_groups<MODE>(Q, n, c, S.sbits, at, NP, ntest);
   // survivors: one atomic per warp
   if (n) {
     u64 base = 0;
@@ -500,6 +521,19 @@ __device__ __noinline__ void drain_rest(bool second, u32 skip, u32 n, u32 at,
   __syncwarp();
 }
 
+// Does a staged prime kill the value?  0 or 1, without a branch.
+template <int MODE>
+__device__ __forceinline__ u32 staged_kill(const SieveSmem& S, const TestCtx& c,
+                                           u32 i, const TestRec& t,
+                                           const uint2& k, u32 vl, u32 vh) {
+  const u32 r = redc_residue(t, k.x, vl, vh);
+  if (MODE == TEST_DICKSON) {
+    const u32 h = min(r, t.q - r);
+    return (S.sbit[k.y + (h >> 5)] >> (h & 31)) & 1u;
+  }
+  return kill_test<MODE>(c, S.sbits, i, t, r) ? 1u : 0u;
+}
+
 // Drain one warp's queue.  Over the staged primes (the first past the
 // pattern, which kill most): rounds with one candidate per lane, the
 // survivors compacted in place by ballot after each, down to a.warp_queue
@@ -513,7 +547,7 @@ __device__ __noinline__ void drain_rest(bool second, u32 skip, u32 n, u32 at,
 // Warp-synchronous: every lane calls it.  Not inlined: the pattern loop
 // around it keeps its NS table indexes in registers and runs between
 // drains.
-template <int KIND>
+template <int MODE>
 __device__ __noinline__ void warp_drain(bool final, const SieveArgs& a) {
   SieveSmem& S = sieve_smem_ref();
   const u32 wq_short = a.warp_queue;
@@ -544,19 +578,14 @@ __device__ __noinline__ void warp_drain(bool final, const SieveArgs& a) {
         for (u32 i = i0; i < at && __any_sync(0xffffffffu, alive);
              i += kRoundUnroll) {
           if (alive) ntest += kRoundUnroll;
-          bool kill = false;
+          u32 hit = 0;
 #pragma unroll
           for (u32 j = 0; j < kRoundUnroll; ++j) {
             const TestRec t = S.srec[i + j];
-            const u32 q = redc_residue(t, S.skq[i + j], vl, vh);
-            if (KIND == KIND_DICKSON) {
-              const u32 h = min(q, t.q - q);
-              kill |= (S.sbit[S.sboff[i + j] + (h >> 5)] >> (h & 31)) & 1u;
-            } else {
-              kill |= kill_test<KIND>(c, S.sbits, first + i + j, t, q);
-            }
+            const uint2 k = S.sk[i + j];
+            hit |= staged_kill<MODE>(S, c, first + i + j, t, k, vl, vh);
           }
-          alive = alive && !kill;
+          alive = alive && !hit;
         }
         const u32 bal = __ballot_sync(0xffffffffu, alive);
         if (alive) Q[out + __popc(bal & lt)] = v;  // out <= base: read already
@@ -567,10 +596,13 @@ __device__ __noinline__ void warp_drain(bool final, const SieveArgs& a) {
     }
     // too few to fill the lanes: one staged prime per lane instead
     for (; n > 0 && at < nstaged; at += 32) {
-      Prime<KIND> p;
-      p.load(c, S.srec, S.skq, first, min(at + lane, nstaged - 1));
+      const u32 p = min(at + lane, nstaged - 1);
+      const TestRec t = S.srec[p];
+      const uint2 k = S.sk[p];
       ntest += n;
-      n = test_group<KIND>(Q, n, c, S.sbits, p);
+      n = test_group(Q, n, [&](u32 vl, u32 vh) {
+        return staged_kill<MODE>(S, c, first + p, t, k, vl, vh) != 0;
+      });
     }
     ntest = __reduce_add_sync(0xffffffffu, ntest);
     if (lane == 0) S.ntest[wid] += ntest;
@@ -579,16 +611,16 @@ __device__ __noinline__ void warp_drain(bool final, const SieveArgs& a) {
   if (final) {
     // the warp's last of the item: k_rest shares them out
     u32 m = list_rest(S, Q, n, done, a);
-    if (m < n) drain_rest<KIND>(false, m, n - m, done, a);
+    if (m < n) drain_rest<MODE>(false, m, n - m, done, a);
     m = list_rest(S, Q2, n2, done, a);
-    if (m < n2) drain_rest<KIND>(true, m, n2 - m, done, a);
+    if (m < n2) drain_rest<MODE>(true, m, n2 - m, done, a);
     n = n2 = 0;
   } else if (n >= kWq2 / 2) {   // enough by themselves
-    drain_rest<KIND>(false, 0, n, done, a);
+    drain_rest<MODE>(false, 0, n, done, a);
     n = 0;
   }
   if (n2 + n > kWq2) {
-    drain_rest<KIND>(true, 0, n2, done, a);
+    drain_rest<MODE>(true, 0, n2, done, a);
     n2 = 0;
   }
   if (lane < n) Q2[n2 + lane] = Q[lane];  // n < kWq2 / 2 = 32
@@ -606,10 +638,12 @@ static_assert(kWq2 / 2 <= 32, "a lane appends one candidate");
 __device__ __forceinline__ void drain_any(SieveSmem& S, bool final,
                                           const SieveArgs& a) {
   if ((S.qn[threadIdx.x >> 5] | S.qn2[threadIdx.x >> 5]) == 0) return;
-  switch (S.kind) {
-    case KIND_EULER: return warp_drain<KIND_EULER>(final, a);
-    case KIND_DICKSON: return warp_drain<KIND_DICKSON>(final, a);
-    default: return warp_drain<KIND_AP>(final, a);
+  switch (S.mode) {
+    case TEST_EULER: return warp_drain<TEST_EULER>(final, a);
+    case TEST_DICKSON: return warp_drain<TEST_DICKSON>(final, a);
+    case TEST_AP: return warp_drain<TEST_AP>(final, a);
+    case TEST_EULER_LOW: return warp_drain<TEST_EULER_LOW>(final, a);
+    default: return warp_drain<TEST_AP_DIV>(final, a);
   }
 }
 
@@ -890,9 +924,10 @@ __global__ void __launch_bounds__(kBlock, 3)
       if (tid < (u32)kStaged && first < eg.NP) {
         const u32 p = min(first + tid, eg.NP - 1);  // past the end: the last
         S.srec[tid] = eg.trec[p];
-        S.skq[tid] = a.xq[it.xq_off + p];
-        if (eg.kind == KIND_DICKSON)
-          S.sboff[tid] = eg.boff[p - kNSMin] - eg.boff[first - kNSMin];
+        S.sk[tid] = make_uint2(
+            a.xq[it.xq_off + p],
+            eg.kind == KIND_DICKSON
+                ? eg.boff[p - kNSMin] - eg.boff[first - kNSMin] : 0u);
       }
       if (eg.kind == KIND_DICKSON && first < eg.NP) {
         const u32 b0 = eg.boff[first - kNSMin];
@@ -909,7 +944,7 @@ __global__ void __launch_bounds__(kBlock, 3)
         S.rounds = eg.rounds;
         S.NP = eg.NP;
         S.deep = eg.deep;
-        S.kind = eg.kind;
+        S.mode = test_mode(eg, first);
       }
       __syncthreads();
     }

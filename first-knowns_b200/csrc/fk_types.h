@@ -8,6 +8,14 @@ namespace fk {
 
 enum Kind : uint32_t { KIND_EULER = 0, KIND_DICKSON = 1, KIND_AP = 2 };
 
+// How a prime's scaled residue is tested (fk_sieve.cuh): by kind, and for
+// Euler and AP in a plain form without a branch and one for the primes that
+// need more -- Euler's up to max(x^2 + x), and those that may divide d.
+enum TestMode : uint32_t {
+  TEST_EULER = 0, TEST_DICKSON = 1, TEST_AP = 2, TEST_EULER_LOW = 3,
+  TEST_AP_DIV = 4,
+};
+
 // What an item asks for.
 enum Mode : uint32_t {
   MODE_SIEVE = 0,   // pre-primality survivors only
@@ -119,7 +127,7 @@ struct DevEngine {
   const uint32_t* bits;
   uint32_t deep;                  // rounds: first prime past which 128 primes
                                   // kill less than a quarter
-  uint32_t ap_div;                // AP: a sieve prime divides d
+  uint32_t ap_div;                // AP: a prime past the pattern divides d
   const uint32_t* rounds;         // [nrounds + 1] prime-index cuts
   const uint32_t* sbits;          // Euler: bitset of {x^2 + x : x < n}
   // marking sieve (long lanes): the primes past the pattern are marked in a
