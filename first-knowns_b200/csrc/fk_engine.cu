@@ -112,9 +112,9 @@ static std::string u128_str(u128 x) {
 }
 
 // ---------------------------------------------------------------- engine ---
-// The sieve kernels' cost model, in instructions per post-wheel candidate
-// (one lane-period) plus per-segment and per-lane terms, for one bound of
-// the marked primes.
+// The sieve kernels' cost model, in SM cycles per post-wheel candidate (one
+// lane-period) plus per-segment and per-lane terms, for one bound of the
+// marked primes.
 struct Cost {
   double round = 0;   // compaction rounds, per lane-period
   double bit = 0;     // marking, per lane-period
@@ -228,13 +228,15 @@ static u32 pat_bytes_for(u32 P0) {
   }
 }
 
-// Both kernels run the same pattern stage (NS primes); the rounds then
-// test each pattern survivor against every remaining prime until one kills
-// it; the marking sieve pays about 1.5 instructions per byte mark plus,
-// per segment of SEG periods, one setup per work entry, an offset step per
-// marked prime and the map's zeroing and extraction, and per lane (task)
-// the shift of every marked prime; candidates that survive the marked
-// primes are tested one by one against the rest.
+// In SM cycles, as measured on a B200 over 256 mixed intervals and single
+// engines.  The rounds: the pattern loop per lane-period (1.84 cycles a
+// word), 2.2 cycles for a pattern survivor's way through column and queue,
+// 0.32 for each of its prime tests.  The marking sieve: 0.115 cycles a byte
+// mark (3.5 wavefronts for 32), per segment 0.25 for each (prime, residue),
+// 0.3 for each prime's offset step and 3500 for the pattern words and the
+// map's zeroing and extraction, per lane (task) 0.46 for each prime's first
+// offset; candidates that survive the marked primes are tested one by one
+// against the rest, a thread each.
 static Cost engine_cost(const fk_engine* e, u32 NPm, u32 ns_sieve, u32 ns,
                         u32 seg) {
   Cost c;
@@ -266,10 +268,10 @@ static Cost engine_cost(const fk_engine* e, u32 NPm, u32 ns_sieve, u32 ns,
   const std::vector<u32>& mp = e->mprefix;
   const double items = NPm > ns && !mp.empty()
                            ? (double)mp[NPm - kNSMin] - mp[ns - kNSMin] : 0;
-  c.round = 2.5 + 22.0 * s1r * tests;
-  c.bit = 2.5 + 2.0 + 1.5 * mark_bit + 22.0 * s1 * tail;
-  c.seg = 12.0 * items + 6.0 * npm + 2048.0 * seg / 32768.0;
-  c.lane = 25.0 * npm;
+  c.round = 0.029 + s1r * (2.2 + 0.32 * tests);
+  c.bit = 0.115 * mark_bit + 1.0 * s1 * tail;
+  c.seg = 0.25 * items + 0.3 * npm + 3500.0 * seg / 32768.0;
+  c.lane = 0.46 * npm;
   c.mark = NPm > ns;
   return c;
 }
