@@ -12,7 +12,7 @@
 //             the reference's definition for its engine (Euler
 //             mr_run_length, Dickson run_length / sprp_run, AP two-pass
 //             chain_depth), kept when it reaches the item's threshold.
-// k_scan / k_scatter / k_sort_seg
+// k_order_prep, k_bucket_*, k_scan, k_sort_seg
 //             order the kept entries per item ascending in x without a
 //             host sort: counting scatter by item, then a bitonic sort of
 //             each item's segment.
@@ -26,8 +26,6 @@ namespace fk {
 struct ClassArgs {
   const DevEngine* engines;
   const DevItem* items;
-  const u32* nitems_p;      // device scalar
-  const u32* xq_items;      // unused here
   const u64* cand_key;
   const u32* cand_item;
   u64 cand_cap;
@@ -433,19 +431,15 @@ __global__ void k_xq(const DevEngine* engines, const DevItem* items,
   }
 }
 
-// Exclusive scan of the per-item counts (one CTA).  With n_dev set, the
-// count is read from device memory (graph replays of varying sizes).
-__global__ void k_scan(const u32* count, u32 n, u64* off,
-                       const u32* n_dev = nullptr) {
-  if (n_dev) n = *n_dev;
-  __shared__ u64 s_carry;
+// Exclusive scan of n counts by one CTA of kBlock threads: off[0, n].
+template <typename F>
+__device__ __forceinline__ u64 cta_scan(u32 n, u64* off, F count) {
   __shared__ u64 s_warp[kBlock / 32];
-  if (threadIdx.x == 0) s_carry = 0;
-  __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  u64 carry = 0;
   for (u32 base = 0; base < n; base += kBlock) {
     const u32 i = base + threadIdx.x;
-    const u64 v = i < n ? count[i] : 0;
+    const u64 v = i < n ? count(i) : 0;
     u64 x = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -459,35 +453,38 @@ __global__ void k_scan(const u32* count, u32 n, u64* off,
       pre += (w < wid) ? s_warp[w] : 0;
       tot += s_warp[w];
     }
-    if (i < n) off[i] = s_carry + pre + x - v;
-    __syncthreads();
-    if (threadIdx.x == 0) s_carry += tot;
+    if (i < n) off[i] = carry + pre + x - v;
+    carry += tot;
     __syncthreads();
   }
-  if (threadIdx.x == 0) off[n] = s_carry;
+  if (threadIdx.x == 0) off[n] = carry;
+  return carry;
 }
 
-__global__ void k_scatter(const OutRec* out, const DevCounters* ctr,
-                          u64 out_cap, const u64* off, u32* fill,
-                          u64* sorted) {
-  u64 n = ctr->nout;
-  if (n > out_cap) n = out_cap;
-  for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (u64)gridDim.x * blockDim.x) {
-    const OutRec r = out[i];
-    const u32 p = atomicAdd(fill + r.item, 1u);
-    sorted[off[r.item] + p] = r.packed;
-  }
+// The scan of the bucket counts, their number read from device memory.
+__global__ void __launch_bounds__(kBlock) k_scan(const u32* count, u64* off,
+                                                 const u32* n_dev) {
+  cta_scan(*n_dev, off, [&](u32 i) { return (u64)count[i]; });
 }
 
 // Buckets for ordering: every item's entries are split by key range into
 // nb = ceil(count / kBucketFill) buckets (the entries of one interval are
 // spread over its span, so a bucket holds about kBucketFill of them), and
-// each bucket is then sorted on its own (k_sort_seg).  nb[i] per item:
-__global__ void k_bucket_nb(const u32* count, u32 n, u32* nb) {
-  for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += gridDim.x * blockDim.x)
-    nb[i] = count[i] ? (count[i] + kBucketFill - 1) / kBucketFill : 0;
+// each bucket is then sorted on its own (k_sort_seg).  One CTA: each item's
+// first output and first bucket, the number of buckets, and their counters
+// cleared.
+constexpr int kOrderBlock = kBlock;
+__global__ void __launch_bounds__(kOrderBlock)
+    k_order_prep(const u32* count, u32 nitems, u64* off, u32* nb, u64* bbase,
+                 u32* nbuckets, u32* bcount, u32* bfill) {
+  cta_scan(nitems, off, [&](u32 i) { return (u64)count[i]; });
+  const u64 total = cta_scan(nitems, bbase, [&](u32 i) {
+    const u32 k = (count[i] + kBucketFill - 1) / kBucketFill;
+    nb[i] = k;
+    return (u64)k;
+  });
+  for (u32 i = threadIdx.x; i < total; i += kBlock) bcount[i] = bfill[i] = 0;
+  if (threadIdx.x == 0) *nbuckets = (u32)total;
 }
 
 __device__ __forceinline__ u32 bucket_of(const OutRec& r, const DevItem* items,
@@ -530,12 +527,6 @@ __global__ void k_bucket_scatter(const OutRec* out, const DevCounters* ctr,
     const u32 b = bucket_of(r, items, engines, bucket_base, nb);
     sorted[boff[b] + atomicAdd(bfill + b, 1u)] = r.packed;
   }
-}
-
-// The bucket count, for k_sort_seg's device-side segment count.
-__global__ void k_bucket_total(const u64* bucket_base, u32 nitems,
-                               u32* nbuckets) {
-  *nbuckets = (u32)bucket_base[nitems];
 }
 
 // Bitonic sort of buf[0, npow) ascending, npow a power of two, by one CTA.

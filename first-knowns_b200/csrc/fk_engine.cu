@@ -780,6 +780,8 @@ struct PinBuf {
   }
 };
 
+constexpr u64 kSpecOut = 2048;   // outputs read back before their count is known
+
 struct SubItem {
   u32 user;       // index of the user item
   u128 X0;        // line base
@@ -790,8 +792,8 @@ struct Family {
   bool mark = false;
   std::vector<u32> idx;         // internal item indices
   std::vector<u64> prefix;      // task prefix, size idx+1
-  DevBuf<u32> d_idx;
-  DevBuf<u64> d_prefix;
+  u32* d_idx = nullptr;         // in the batch's upload buffer
+  u64* d_prefix = nullptr;
 };
 
 struct fk_batch {
@@ -809,28 +811,33 @@ struct fk_batch {
   std::vector<u32> dense_idx, sieve_idx;
   Family fam[8];
   // device buffers
-  DevBuf<DevItem> d_items;
-  DevBuf<u32> d_dense, d_sieve;
+  // what a run uploads, in one buffer and one copy: the items, every
+  // family's prefix and item list, the dense and sieve item lists
+  DevBuf<unsigned char> d_up;
+  PinBuf<unsigned char> h_up;
+  u64 up_bytes = 0;
+  DevItem* d_items = nullptr;
+  u32 *d_dense = nullptr, *d_sieve = nullptr;
   DevBuf<u32> d_xq;
   DevBuf<u64> d_cand_key;
   DevBuf<u32> d_cand_item;
   DevBuf<OutRec> d_out;
-  DevBuf<u32> d_item_count, d_item_fill;
+  // what a run starts from zero, in one buffer and one memset: the counters,
+  // the marking families' task counters, blocks claimed per rounds item,
+  // outputs per item
+  DevBuf<u64> d_zero;
+  u64 zero_words = 0;
+  DevCounters* d_ctr = nullptr;
+  unsigned long long *d_task_ctr = nullptr, *d_block_ctr = nullptr;
+  u32* d_item_count = nullptr;
   DevBuf<u64> d_rest_key;       // k_rest's list
   DevBuf<u32> d_rest_item, d_rest_start, d_rest_state;
   DevBuf<u64> d_item_off, d_sorted, d_scratch;
-  DevBuf<u32> d_nb, d_bcount, d_bfill, d_nbuckets;
+  DevBuf<u32> d_nb, d_bcount, d_nbuckets;   // d_bcount: counts, then fills
   DevBuf<u64> d_bbase, d_boff;
-  DevBuf<unsigned long long> d_task_ctr;
-  DevBuf<unsigned long long> d_block_ctr;  // rounds: blocks claimed per item
-  DevBuf<u32> d_nitems;
   DevBuf<u32> d_rounds;         // per engine: this batch's round cuts
-  DevCounters* d_ctr = nullptr;
-  PinBuf<DevItem> h_items;
   PinBuf<DevCounters> h_ctr;
   PinBuf<u64> h_off, h_sorted;
-  PinBuf<u32> h_small;
-  PinBuf<u64> h_prefix;
   u64 cand_cap = 0, out_cap = 0;
   // graph
   cudaGraph_t graph = nullptr;
@@ -906,7 +913,6 @@ static fk_status batch_init(fk_batch* b, fk_engine* const* engines,
   fk_status st0 = apply_tuning(b);
   if (st0) return st0;
   FK_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
-  FK_CUDA(cudaMalloc(&b->d_ctr, sizeof(DevCounters)));
   int dev = 0;
   FK_CUDA(cudaGetDevice(&dev));
   FK_CUDA(cudaDeviceGetAttribute(&b->nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -917,8 +923,6 @@ static fk_status batch_init(fk_batch* b, fk_engine* const* engines,
     b->fam[f].P0 = P0s[f & 3];
     b->fam[f].mark = f >= 4;
   }
-  FK_CUDA(b->d_task_ctr.ensure(8) == FK_OK ? cudaSuccess : cudaErrorMemoryAllocation);
-  FK_CUDA(b->d_nitems.ensure(4) == FK_OK ? cudaSuccess : cudaErrorMemoryAllocation);
   for (fk_status st : {b->d_rest_key.ensure(kRestCap), b->d_rest_item.ensure(kRestCap),
                        b->d_rest_start.ensure(kRestCap), b->d_rest_state.ensure(kRestCap)})
     if (st) return st;
@@ -935,19 +939,17 @@ static fk_status batch_init(fk_batch* b, fk_engine* const* engines,
 static void batch_free(fk_batch* b) {
   if (b->gexec) cudaGraphExecDestroy(b->gexec);
   if (b->graph) cudaGraphDestroy(b->graph);
-  b->d_items.release(); b->d_dense.release(); b->d_sieve.release();
+  b->d_up.release(); b->h_up.release(); b->d_zero.release();
   b->d_xq.release(); b->d_cand_key.release(); b->d_cand_item.release();
   b->d_rest_key.release(); b->d_rest_item.release(); b->d_rest_start.release();
   b->d_rest_state.release();
-  b->d_out.release(); b->d_item_count.release(); b->d_item_fill.release();
+  b->d_out.release(); 
   b->d_item_off.release(); b->d_sorted.release(); b->d_scratch.release();
-  b->d_nb.release(); b->d_bcount.release(); b->d_bfill.release();
+  b->d_nb.release(); b->d_bcount.release();
   b->d_nbuckets.release(); b->d_bbase.release(); b->d_boff.release();
-  b->d_task_ctr.release(); b->d_block_ctr.release(); b->d_nitems.release(); b->d_rounds.release();
-  for (auto& f : b->fam) { f.d_idx.release(); f.d_prefix.release(); }
-  b->h_items.release(); b->h_ctr.release(); b->h_off.release();
-  b->h_sorted.release(); b->h_small.release(); b->h_prefix.release();
-  if (b->d_ctr) cudaFree(b->d_ctr);
+  b->d_rounds.release();
+  b->h_ctr.release(); b->h_off.release();
+  b->h_sorted.release();
   if (b->d_engines) cudaFree(b->d_engines);
   for (auto& e : b->ev) if (e) cudaEventDestroy(e);
   for (auto& e : b->fev) if (e) cudaEventDestroy(e);
@@ -1126,32 +1128,58 @@ static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
     b->out_cap = need;
   }
   const u64 ni = b->items.size();
-  if ((st = b->d_items.ensure(ni + 1))) return st;
-  if ((st = b->d_block_ctr.ensure(ni + 1))) return st;
-  if ((st = b->d_item_count.ensure(ni + 1))) return st;
-  if ((st = b->d_item_fill.ensure(ni + 1))) return st;
+  // the zeroed buffer, in 8-byte words
+  constexpr u64 cw = (sizeof(DevCounters) + 7) / 8;
+  b->zero_words = cw + 8 + (ni + 1) + (ni + 2) / 2;
+  if ((st = b->d_zero.ensure(b->zero_words))) return st;
+  b->d_ctr = reinterpret_cast<DevCounters*>(b->d_zero.p);
+  b->d_task_ctr = b->d_zero.p + cw;
+  b->d_block_ctr = b->d_task_ctr + 8;
+  b->d_item_count = reinterpret_cast<u32*>(b->d_block_ctr + ni + 1);
   if ((st = b->d_item_off.ensure(ni + 2))) return st;
   if ((st = b->d_nb.ensure(ni + 1))) return st;
   if ((st = b->d_bbase.ensure(ni + 2))) return st;
   if ((st = b->d_nbuckets.ensure(4))) return st;
   {
     const u64 nbk = b->out_cap / kBucketFill + ni + 2;
-    if ((st = b->d_bcount.ensure(nbk))) return st;
-    if ((st = b->d_bfill.ensure(nbk))) return st;
+    if ((st = b->d_bcount.ensure(2 * nbk))) return st;
     if ((st = b->d_boff.ensure(nbk + 1))) return st;
   }
-  if ((st = b->h_items.ensure(ni + 1))) return st;
   if ((st = b->h_off.ensure(ni + 2))) return st;
-  if ((st = b->d_dense.ensure(b->dense_idx.size() + 1))) return st;
-  if ((st = b->d_sieve.ensure(b->sieve_idx.size() + 1))) return st;
-  u64 famsz = 0, fampre = 0;
-  for (auto& f : b->fam) { famsz += f.idx.size(); fampre += f.prefix.size(); }
-  if ((st = b->h_small.ensure(b->dense_idx.size() + b->sieve_idx.size() + famsz + 8))) return st;
-  if ((st = b->h_prefix.ensure(fampre + 8))) return st;
-  for (auto& f : b->fam) {
-    if ((st = f.d_idx.ensure(f.idx.size() + 1))) return st;
-    if ((st = f.d_prefix.ensure(f.prefix.size() + 1))) return st;
+  if ((st = b->h_sorted.ensure(kSpecOut))) return st;
+  // the upload buffer: 8-byte words first, then the 4-byte lists
+  u64 at = ni * sizeof(DevItem);
+  u64 pre[8], idx[8];
+  for (int f = 0; f < 8; ++f) {
+    pre[f] = at;
+    at += 8 * b->fam[f].prefix.size();
   }
+  for (int f = 0; f < 8; ++f) {
+    idx[f] = at;
+    at += 4 * b->fam[f].idx.size();
+  }
+  const u64 dense = at, sieve = dense + 4 * b->dense_idx.size();
+  b->up_bytes = sieve + 4 * b->sieve_idx.size();
+  if ((st = b->d_up.ensure(b->up_bytes))) return st;
+  if ((st = b->h_up.ensure(b->up_bytes))) return st;
+  unsigned char* const d = b->d_up.p;
+  b->d_items = reinterpret_cast<DevItem*>(d);
+  b->d_dense = reinterpret_cast<u32*>(d + dense);
+  b->d_sieve = reinterpret_cast<u32*>(d + sieve);
+  unsigned char* const h = b->h_up.p;
+  const auto put = [&](u64 to, const void* p, u64 bytes) {
+    if (bytes) std::memcpy(h + to, p, bytes);
+  };
+  put(0, b->items.data(), ni * sizeof(DevItem));
+  for (int f = 0; f < 8; ++f) {
+    Family& F = b->fam[f];
+    F.d_prefix = reinterpret_cast<u64*>(d + pre[f]);
+    F.d_idx = reinterpret_cast<u32*>(d + idx[f]);
+    put(pre[f], F.prefix.data(), 8 * F.prefix.size());
+    put(idx[f], F.idx.data(), 4 * F.idx.size());
+  }
+  put(dense, b->dense_idx.data(), 4 * b->dense_idx.size());
+  put(sieve, b->sieve_idx.data(), 4 * b->sieve_idx.size());
   return FK_OK;
 }
 
@@ -1165,23 +1193,18 @@ static cudaError_t record(cudaEvent_t ev, cudaStream_t s, bool capturing) {
 static fk_status enqueue(fk_batch* b, bool capturing = false) {
   cudaStream_t s = b->stream;
   const u32 ni = (u32)b->items.size();
-  FK_CUDA(cudaMemsetAsync(b->d_ctr, 0, sizeof(DevCounters), s));
-  FK_CUDA(cudaMemsetAsync(b->d_task_ctr.p, 0, 8 * sizeof(unsigned long long), s));
-  FK_CUDA(cudaMemsetAsync(b->d_item_count.p, 0, (ni + 1) * sizeof(u32), s));
-  FK_CUDA(cudaMemsetAsync(b->d_item_fill.p, 0, (ni + 1) * sizeof(u32), s));
-  FK_CUDA(cudaMemsetAsync(b->d_block_ctr.p, 0,
-                          (ni + 1) * sizeof(unsigned long long), s));
+  FK_CUDA(cudaMemsetAsync(b->d_zero.p, 0, b->zero_words * 8, s));
   FK_CUDA(record(b->ev[0], s, capturing));
   u64 nl = 1;  // k_classify
   if (!b->sieve_idx.empty()) {
     ++nl;
     dim3 g(64, (u32)std::min<size_t>(b->sieve_idx.size(), 65535));
-    k_xq<<<g, kBlock, 0, s>>>(b->d_engines, b->d_items.p, b->d_sieve.p,
+    k_xq<<<g, kBlock, 0, s>>>(b->d_engines, b->d_items, b->d_sieve,
                               (u32)b->sieve_idx.size(), b->d_xq.p);
   }
   if (!b->dense_idx.empty()) {
     ++nl;
-    k_dense<<<b->nsm * 4, kBlock, 0, s>>>(b->d_items.p, b->d_dense.p,
+    k_dense<<<b->nsm * 4, kBlock, 0, s>>>(b->d_items, b->d_dense,
                                           (u32)b->dense_idx.size(),
                                           b->d_cand_key.p, b->d_cand_item.p,
                                           b->cand_cap, b->d_ctr);
@@ -1195,9 +1218,9 @@ static fk_status enqueue(fk_batch* b, bool capturing = false) {
     FK_CUDA(record(b->fev[2 * f], s, capturing));
     SieveArgs a{};
     a.engines = b->d_engines;
-    a.items = b->d_items.p;
-    a.task_prefix = F.d_prefix.p;
-    a.item_index = F.d_idx.p;
+    a.items = b->d_items;
+    a.task_prefix = F.d_prefix;
+    a.item_index = F.d_idx;
     a.nitems = (u32)F.idx.size();
     a.ntask = F.prefix.back();
     a.xq = b->d_xq.p;
@@ -1205,8 +1228,8 @@ static fk_status enqueue(fk_batch* b, bool capturing = false) {
     a.cand_item = b->d_cand_item.p;
     a.cand_cap = b->cand_cap;
     a.ctr = b->d_ctr;
-    a.task_ctr = b->d_task_ctr.p + f;
-    a.block_ctr = b->d_block_ctr.p + blocks0;
+    a.task_ctr = b->d_task_ctr + f;
+    a.block_ctr = b->d_block_ctr + blocks0;
     if (!F.mark) blocks0 += F.idx.size();
     a.warp_queue = b->tune.warp_queue;
     a.rest_key = b->d_rest_key.p;
@@ -1240,48 +1263,52 @@ static fk_status enqueue(fk_batch* b, bool capturing = false) {
   FK_CUDA(record(b->ev[1], s, capturing));
   ClassArgs c{};
   c.engines = b->d_engines;
-  c.items = b->d_items.p;
+  c.items = b->d_items;
   c.cand_key = b->d_cand_key.p;
   c.cand_item = b->d_cand_item.p;
   c.cand_cap = b->cand_cap;
   c.ctr = b->d_ctr;
   c.out = b->d_out.p;
   c.out_cap = b->out_cap;
-  c.item_count = b->d_item_count.p;
+  c.item_count = b->d_item_count;
   // the exact list takes the ordering scratch (2 * out_cap words, and
   // cand_cap is never above out_cap), free until the sort
   c.exact = b->d_scratch.p;
   c.spec_lanes = (u64)b->nsm * kSpecLanes;
-  k_classify<<<b->nsm * b->tune.classify_ctas_per_sm, kBlock, 0, s>>>(c);
+  // both run loops over their candidates: more CTAs than fit at once would
+  // only start to find nothing left
+  const u32 cgrid = b->nsm * std::min(b->tune.classify_ctas_per_sm, kClassCtas);
+  k_classify<<<cgrid, kBlock, 0, s>>>(c);
   if (b->hunts) {   // pre-primality streams list nothing
     ++nl;
-    k_exact<<<b->nsm * b->tune.classify_ctas_per_sm, kBlock, 0, s>>>(c);
+    k_exact<<<cgrid, kBlock, 0, s>>>(c);
   }
   FK_CUDA(record(b->ev[2], s, capturing));
+  u32* const bfill = b->d_bcount.p + b->d_bcount.cap / 2;
   // order: per-item counts -> per-item buckets by key range -> bucket
   // counts -> scatter -> every bucket sorted in shared memory
-  const u64 nbk_cap = b->d_bcount.cap;
-  FK_CUDA(cudaMemsetAsync(b->d_bcount.p, 0, nbk_cap * sizeof(u32), s));
-  FK_CUDA(cudaMemsetAsync(b->d_bfill.p, 0, nbk_cap * sizeof(u32), s));
-  k_scan<<<1, kBlock, 0, s>>>(b->d_item_count.p, ni, b->d_item_off.p);
-  k_bucket_nb<<<b->nsm, kBlock, 0, s>>>(b->d_item_count.p, ni, b->d_nb.p);
-  k_scan<<<1, kBlock, 0, s>>>(b->d_nb.p, ni, b->d_bbase.p);
-  k_bucket_total<<<1, 1, 0, s>>>(b->d_bbase.p, ni, b->d_nbuckets.p);
+  k_order_prep<<<1, kOrderBlock, 0, s>>>(b->d_item_count, ni, b->d_item_off.p,
+                                         b->d_nb.p, b->d_bbase.p,
+                                         b->d_nbuckets.p, b->d_bcount.p, bfill);
   k_bucket_count<<<b->nsm * 2, kBlock, 0, s>>>(
-      b->d_out.p, b->d_ctr, b->out_cap, b->d_items.p, b->d_engines,
+      b->d_out.p, b->d_ctr, b->out_cap, b->d_items, b->d_engines,
       b->d_bbase.p, b->d_nb.p, b->d_bcount.p);
-  k_scan<<<1, kBlock, 0, s>>>(b->d_bcount.p, 0u, b->d_boff.p, b->d_nbuckets.p);
+  k_scan<<<1, kBlock, 0, s>>>(b->d_bcount.p, b->d_boff.p, b->d_nbuckets.p);
   k_bucket_scatter<<<b->nsm * 2, kBlock, 0, s>>>(
-      b->d_out.p, b->d_ctr, b->out_cap, b->d_items.p, b->d_engines,
-      b->d_bbase.p, b->d_nb.p, b->d_boff.p, b->d_bfill.p, b->d_sorted.p);
+      b->d_out.p, b->d_ctr, b->out_cap, b->d_items, b->d_engines,
+      b->d_bbase.p, b->d_nb.p, b->d_boff.p, bfill, b->d_sorted.p);
   k_sort_seg<<<b->nsm * 4, kBlock, 0, s>>>(b->d_sorted.p, b->d_boff.p,
                                            b->d_nbuckets.p, b->d_scratch.p);
-  nl += 8;     // three k_scan, k_bucket_nb/_total/_count/_scatter, k_sort_seg
+  nl += 5;     // k_order_prep, k_bucket_count, k_scan, k_bucket_scatter, k_sort_seg
   FK_CUDA(cudaGetLastError());
   FK_CUDA(record(b->ev[3], s, capturing));
   FK_CUDA(cudaMemcpyAsync(b->h_ctr.p, b->d_ctr, sizeof(DevCounters),
                           cudaMemcpyDeviceToHost, s));
   FK_CUDA(cudaMemcpyAsync(b->h_off.p, b->d_item_off.p, (ni + 1) * sizeof(u64),
+                          cudaMemcpyDeviceToHost, s));
+  // a short result comes back in the same round trip
+  FK_CUDA(cudaMemcpyAsync(b->h_sorted.p, b->d_sorted.p,
+                          std::min<u64>(kSpecOut, b->out_cap) * 8,
                           cudaMemcpyDeviceToHost, s));
   b->last_launches = nl;
   return FK_OK;
@@ -1289,40 +1316,9 @@ static fk_status enqueue(fk_batch* b, bool capturing = false) {
 
 static fk_status upload_items(fk_batch* b) {
   cudaStream_t s = b->stream;
-  const u64 ni = b->items.size();
-  b->h2d = ni * sizeof(DevItem) + 4 * (b->dense_idx.size() +
-                                       b->sieve_idx.size() + 1);
-  for (auto& f : b->fam)
-    if (!f.idx.empty()) b->h2d += 4 * f.idx.size() + 8 * f.prefix.size();
-  std::copy(b->items.begin(), b->items.end(), b->h_items.p);
-  FK_CUDA(cudaMemcpyAsync(b->d_items.p, b->h_items.p, ni * sizeof(DevItem),
+  b->h2d = b->up_bytes;
+  FK_CUDA(cudaMemcpyAsync(b->d_up.p, b->h_up.p, b->up_bytes,
                           cudaMemcpyHostToDevice, s));
-  u32* hs = b->h_small.p;
-  size_t k = 0;
-  for (u32 v : b->dense_idx) hs[k++] = v;
-  for (u32 v : b->sieve_idx) hs[k++] = v;
-  hs[k] = (u32)ni;
-  if (!b->dense_idx.empty())
-    FK_CUDA(cudaMemcpyAsync(b->d_dense.p, hs, b->dense_idx.size() * 4,
-                            cudaMemcpyHostToDevice, s));
-  if (!b->sieve_idx.empty())
-    FK_CUDA(cudaMemcpyAsync(b->d_sieve.p, hs + b->dense_idx.size(),
-                            b->sieve_idx.size() * 4, cudaMemcpyHostToDevice, s));
-  FK_CUDA(cudaMemcpyAsync(b->d_nitems.p, hs + k, 4, cudaMemcpyHostToDevice, s));
-  ++k;
-  u64* hp = b->h_prefix.p;
-  size_t kp = 0;
-  for (auto& f : b->fam) {
-    if (f.idx.empty()) continue;
-    std::copy(f.idx.begin(), f.idx.end(), hs + k);
-    FK_CUDA(cudaMemcpyAsync(f.d_idx.p, hs + k, f.idx.size() * 4,
-                            cudaMemcpyHostToDevice, s));
-    k += f.idx.size();
-    std::copy(f.prefix.begin(), f.prefix.end(), hp + kp);
-    FK_CUDA(cudaMemcpyAsync(f.d_prefix.p, hp + kp, f.prefix.size() * 8,
-                            cudaMemcpyHostToDevice, s));
-    kp += f.prefix.size();
-  }
   return FK_OK;
 }
 
@@ -1337,9 +1333,11 @@ static fk_status launch(fk_batch* b, int use_graph) {
   key.push_back(b->out_cap);
   key.push_back(b->d_xq.cap);
   for (auto& f : b->fam) { key.push_back(f.idx.size()); key.push_back(f.prefix.back()); }
-  key.push_back((u64)(uintptr_t)b->d_items.p);
+  key.push_back((u64)(uintptr_t)b->d_items);
   key.push_back((u64)(uintptr_t)b->d_cand_key.p);
-  key.push_back((u64)(uintptr_t)b->d_block_ctr.p);
+  key.push_back((u64)(uintptr_t)b->d_zero.p);
+  key.push_back((u64)(uintptr_t)b->h_sorted.p);
+  key.push_back((u64)(uintptr_t)b->d_bcount.p);
   key.push_back(((u64)b->tune.sieve_ctas_per_sm << 32) | b->tune.mark_ctas_per_sm);
   key.push_back(((u64)b->tune.warp_queue << 32) | b->tune.seg_per_task);
   key.push_back(((u64)b->tune.warp_tasks << 32) | b->tune.classify_ctas_per_sm);
@@ -1382,8 +1380,7 @@ static fk_status collect(fk_batch* b) {
     if ((st = b->d_sorted.ensure(need))) return st;
     if ((st = b->d_scratch.ensure(2 * need))) return st;
     const u64 nbk = need / kBucketFill + b->items.size() + 2;
-    if ((st = b->d_bcount.ensure(nbk))) return st;
-    if ((st = b->d_bfill.ensure(nbk))) return st;
+    if ((st = b->d_bcount.ensure(2 * nbk))) return st;
     if ((st = b->d_boff.ensure(nbk + 1))) return st;
     b->cand_cap = b->out_cap = need;
     return set_err(FK_ERR_OVERFLOW, "candidate buffer overflow (grown; rerun)");
@@ -1392,8 +1389,8 @@ static fk_status collect(fk_batch* b) {
   const u64 nout = b->h_off.p[ni];
   b->d2h = sizeof(DevCounters) + (ni + 1) * 8 + nout * 8;
   fk_status st;
-  if ((st = b->h_sorted.ensure(nout + 1))) return st;
-  if (nout) {
+  if (nout > kSpecOut) {
+    if ((st = b->h_sorted.ensure(nout))) return st;
     FK_CUDA(cudaMemcpyAsync(b->h_sorted.p, b->d_sorted.p, nout * 8,
                             cudaMemcpyDeviceToHost, s));
     FK_CUDA(cudaStreamSynchronize(s));

@@ -49,6 +49,7 @@ constexpr uint32_t kPadWide = 64, kPadNarrow = 32;  // pattern table padding
 constexpr int kMaxRounds = 64;
 constexpr int kSortSmem = 4096;   // entries a CTA sorts in shared memory
 constexpr int kClassChunk = 128;  // candidates a warp fetches at once
+constexpr uint32_t kClassCtas = 2; // SPRP: CTAs an SM holds at their registers
 constexpr int kSpecLanes = 512;   // SPRP: lanes an SM runs at no cost to each
 constexpr int kBucketFill = 1024; // expected entries per ordering bucket
 constexpr int kWarpMode = 32;     // warp queue below which a candidate
