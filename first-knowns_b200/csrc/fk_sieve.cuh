@@ -36,9 +36,9 @@
 // kernel issues instructions (65-75% of the slots), in the sparse windows
 // the pattern loads' shared-memory wavefronts, two a load.  Against 64-bit
 // Barrett tests with a queue drained at every block's end and a CTA barrier
-// after every eight blocks: 256 mixed intervals 204 -> 112 ms, the Dickson
-// window of 2^38 j 12.7 -> 6.9, the Euler n = 17 windows of 5e14 and 2e16
-// 42.2 -> 23.9 and 795 -> 483, the 13# line's quarter 19.3 -> 13.5.
+// after every eight blocks: 256 mixed intervals 204 -> 77 ms, the Dickson
+// window of 2^38 j 12.7 -> 5.5 with k_rest, the Euler n = 17 windows of 5e14
+// and 2e16 42.2 -> 23.7 and 795 -> 478, the 13# line's quarter 19.3 -> 10.4.
 #pragma once
 #include "fk_arith.cuh"
 #include "fk_types.h"
@@ -50,30 +50,6 @@ constexpr u32 kRoundUnroll = 4;  // primes per trip of the compaction rounds
 
 __device__ __forceinline__ u32 smem_u32(const void* p) {
   return (u32)__cvta_generic_to_shared(p);
-}
-
-// Block-wide exclusive scan of one u32 per thread; returns the prefix and
-// sets *total.  Two barriers.
-__device__ __forceinline__ u32 block_scan(u32 v, u32* s_warp, u32* total) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  u32 x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    u32 y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) s_warp[wid] = x;
-  __syncthreads();
-  u32 base = 0, tot = 0;
-#pragma unroll
-  for (int w = 0; w < kBlock / 32; ++w) {
-    u32 t = s_warp[w];
-    base += (w < wid) ? t : 0;
-    tot += t;
-  }
-  __syncthreads();
-  *total = tot;
-  return base + x - v;
 }
 
 // Entry i of an item's base-residue table: X0 * c1 mod q, the base folded
@@ -457,9 +433,10 @@ __device__ __forceinline__ u32 list_rest(const SieveSmem& S, const u64* Q,
 }
 
 // n candidates of a warp's first or second queue, past the first `skip`,
-// against every prime from index `at` on, in place, and the survivors into the global list: 32 primes at a time, then, once
-// few candidates die among 128 primes (S.deep), kDeep groups of 32 at a
-// time (fewer votes, more loads in flight).
+// against every prime from index `at` on, in place, and the survivors into
+// the global list: 32 primes at a time, then, once few candidates die among
+// 128 primes (S.deep), kDeep groups of 32 at a time (fewer votes, more loads
+// in flight).
 template <int MODE>
 __device__ __noinline__ void drain_rest(bool second, u32 skip, u32 n, u32 at,
                                         const SieveArgs& a) {

@@ -14,7 +14,8 @@ and three kernel-variant choices: the marking segment length in bytes
 (``mark_segment``: 16, 32 or 64 KiB of shared byte map) and the pattern
 primes each CTA stages in shared memory, per sieve kernel
 (``pattern_primes``, ``mark_pattern_primes``: 24, 32 or 40), and the
-blocks of chains per CTA task of the rounds kernel (``warp_tasks``).
+how many blocks of chains a warp of the rounds kernel claims at once
+(``warp_tasks``).
 None of them can change a result; they only move time.
 
 ``tune`` runs coordinate descent: starting from the current setting it

@@ -167,10 +167,12 @@ typedef struct fk_tuning {
   uint32_t chains_per_sm;        /* lanes are cut into chains until about this *
                                   * many chains per SM exist (64-65536)        */
   uint32_t warp_queue;           /* compaction: a warp's queue shorter than    *
-                                  * this runs one candidate per warp over all  *
-                                  * later primes (1-513; 513: always)         */
+                                  * this tests one candidate against 32 primes *
+                                  * at a time instead of 32 candidates against *
+                                  * one (1-513; 513: always)                   */
   uint32_t seg_per_task;         /* marking: segments per task (1-64)          */
-  uint32_t classify_ctas_per_sm; /* k_classify grid: CTAs per SM (1-32)        */
+  uint32_t classify_ctas_per_sm; /* k_classify and k_exact grids: CTAs per SM,  *
+                                  * at most as many as fit at once (1-32)      */
   uint32_t mark_limit;           /* sieve-prime bound of the marking sieve:    *
                                   * primes below it are marked, the rest are   *
                                   * tested per candidate (2^16 = all marked)   */
@@ -198,11 +200,10 @@ typedef struct fk_tuning {
                                   * candidate                                 */
   uint32_t mark_pattern_primes;  /* the same for the marking sieve (24, 32 or *
                                   * 40); the primes past them are marked      */
-  uint32_t warp_tasks;           /* pattern sieve + rounds: blocks of 32      *
-                                  * threads' chains per CTA task (8, 16 or    *
-                                  * 32), claimed by the CTA's warps one at a  *
-                                  * time; the CTA waits for its slowest warp  *
-                                  * once per task                             */
+  uint32_t warp_tasks;           /* pattern sieve + rounds: how many blocks   *
+                                  * of 32 threads' chains a warp claims of an *
+                                  * item at once, in eighths of the default   *
+                                  * (8, 16 or 32)                             */
 } fk_tuning;
 fk_status fk_batch_set_tuning(fk_batch* b, const fk_tuning* t);
 fk_status fk_batch_get_tuning(const fk_batch* b, fk_tuning* out);
