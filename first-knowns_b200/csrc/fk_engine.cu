@@ -1094,6 +1094,15 @@ static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
       b->sub.push_back({(u32)ui, base});
     }
   }
+  // the rounds kernel's lists by kind of test, then by engine: an SM's warps
+  // run the same code (first_item), and CTAs restage fewer tables
+  for (auto& f : b->fam)
+    if (!f.mark)
+      std::sort(f.idx.begin(), f.idx.end(), [b](u32 x, u32 y) {
+        const u32 ex = b->items[x].engine, ey = b->items[y].engine;
+        const int kx = b->engines[ex]->kind, ky = b->engines[ey]->kind;
+        return kx != ky ? kx < ky : ex != ey ? ex < ey : x < y;
+      });
   // base-residue table offsets
   u64 xo = 0;
   for (u32 i : b->sieve_idx) {
