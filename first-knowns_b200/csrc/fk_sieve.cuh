@@ -683,10 +683,15 @@ static __device__ __noinline__ void flush_columns(u32 cn, const SieveArgs& a) {
   const u32 wl = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const unsigned short* C = S.col + wid * (kColSlots * 32) + wl;
   const u32 rows = __reduce_max_sync(0xffffffffu, cn);
+  // the queue's length, the same in every lane; lane 0 stores it only after
+  // all have read it, for the drain and for the next flush
+  u32 qn = S.qn[wid];
+  __syncwarp();
   for (u32 r = 0; r < rows; ++r) {
     const u32 bal = __ballot_sync(0xffffffffu, r < cn);
-    u32 qn = S.qn[wid];
     if (qn + 32 > kWq) {
+      if (wl == 0) S.qn[wid] = qn;
+      __syncwarp();   // and the entries pushed so far are in the queue
       drain_any(S, false, a);
       qn = 0;
     }
@@ -697,9 +702,10 @@ static __device__ __noinline__ void flush_columns(u32 cn, const SieveArgs& a) {
       S.queue[wid * kWq + qn + __popc(bal & ((1u << wl) - 1u))] =
           u * S.blk.M + S.chain_R[threadIdx.x];
     }
-    if (wl == 0) S.qn[wid] = qn + __popc(bal);
-    __syncwarp();
+    qn += __popc(bal);
   }
+  if (wl == 0) S.qn[wid] = qn;
+  __syncwarp();
 }
 
 // Push the set bits of one 32-bit half word into the thread's column while
