@@ -738,21 +738,24 @@ static fk_status build_engine(fk_engine* e) {
 // old capacity): a stream of batches of slowly rising size then reallocates
 // a logarithmic number of times, since each regrowth frees the old buffer
 // (cudaFree / cudaFreeHost wait for the device) and pins new host pages.
+// `moves`, where given, counts the times the buffer's address changed: a
+// captured graph holds addresses, and must not outlive them.
 template <typename T>
 struct DevBuf {
   T* p = nullptr;
   u64 cap = 0;
+  u64* moves;
+  explicit DevBuf(u64* m = nullptr) : moves(m) {}
   fk_status ensure(u64 n) {
     if (n <= cap && p) return FK_OK;
     u64 c = std::max<u64>({n, (u64)1024, cap + cap / 2});
-    if (p) cudaFree(p);
-    p = nullptr;
-    cap = 0;
+    release();
     FK_CUDA(cudaMalloc(&p, c * sizeof(T)));
     cap = c;
     return FK_OK;
   }
   void release() {
+    if (moves) ++*moves;
     if (p) cudaFree(p);
     p = nullptr;
     cap = 0;
@@ -763,17 +766,18 @@ template <typename T>
 struct PinBuf {
   T* p = nullptr;
   u64 cap = 0;
+  u64* moves;
+  explicit PinBuf(u64* m = nullptr) : moves(m) {}
   fk_status ensure(u64 n) {
     if (n <= cap && p) return FK_OK;
     u64 c = std::max<u64>({n, (u64)1024, cap + cap / 2});
-    if (p) cudaFreeHost(p);
-    p = nullptr;
-    cap = 0;
+    release();
     FK_CUDA(cudaMallocHost(&p, c * sizeof(T)));
     cap = c;
     return FK_OK;
   }
   void release() {
+    if (moves) ++*moves;
     if (p) cudaFreeHost(p);
     p = nullptr;
     cap = 0;
@@ -810,34 +814,37 @@ struct fk_batch {
   std::vector<SubItem> sub;
   std::vector<u32> dense_idx, sieve_idx;
   Family fam[8];
-  // device buffers
+  // device buffers: those a captured graph uses count their moves
+  u64 moves = 0;
   // what a run uploads, in one buffer and one copy: the items, every
   // family's prefix and item list, the dense and sieve item lists
-  DevBuf<unsigned char> d_up;
+  DevBuf<unsigned char> d_up{&moves};
   PinBuf<unsigned char> h_up;
   u64 up_bytes = 0;
   DevItem* d_items = nullptr;
   u32 *d_dense = nullptr, *d_sieve = nullptr;
-  DevBuf<u32> d_xq;
-  DevBuf<u64> d_cand_key;
-  DevBuf<u32> d_cand_item;
-  DevBuf<OutRec> d_out;
+  DevBuf<u32> d_xq{&moves};
+  DevBuf<u64> d_cand_key{&moves};
+  DevBuf<u32> d_cand_item{&moves};
+  DevBuf<OutRec> d_out{&moves};
   // what a run starts from zero, in one buffer and one memset: the counters,
   // the marking families' task counters, blocks claimed per rounds item,
   // outputs per item
-  DevBuf<u64> d_zero;
+  DevBuf<u64> d_zero{&moves};
   u64 zero_words = 0;
   DevCounters* d_ctr = nullptr;
   unsigned long long *d_task_ctr = nullptr, *d_block_ctr = nullptr;
   u32* d_item_count = nullptr;
-  DevBuf<u64> d_rest_key;       // k_rest's list
-  DevBuf<u32> d_rest_item, d_rest_start, d_rest_state;
-  DevBuf<u64> d_item_off, d_sorted, d_scratch;
-  DevBuf<u32> d_nb, d_bcount, d_nbuckets;   // d_bcount: counts, then fills
-  DevBuf<u64> d_bbase, d_boff;
+  // k_rest's list
+  DevBuf<u64> d_rest_key{&moves};
+  DevBuf<u32> d_rest_item{&moves}, d_rest_start{&moves}, d_rest_state{&moves};
+  DevBuf<u64> d_item_off{&moves}, d_sorted{&moves}, d_scratch{&moves};
+  DevBuf<u32> d_nb{&moves}, d_nbuckets{&moves};
+  DevBuf<u32> d_bcount{&moves};   // counts, then fills
+  DevBuf<u64> d_bbase{&moves}, d_boff{&moves};
   DevBuf<u32> d_rounds;         // per engine: this batch's round cuts
-  PinBuf<DevCounters> h_ctr;
-  PinBuf<u64> h_off, h_sorted;
+  PinBuf<DevCounters> h_ctr{&moves};
+  PinBuf<u64> h_off{&moves}, h_sorted{&moves};
   u64 cand_cap = 0, out_cap = 0;
   // graph
   cudaGraph_t graph = nullptr;
@@ -1333,6 +1340,8 @@ static fk_status upload_items(fk_batch* b) {
 
 static fk_status launch(fk_batch* b, int use_graph) {
   if (!use_graph) return enqueue(b);
+  // what the captured launches hold: counts, capacities, tuning, and the
+  // buffers' addresses, by the number of times one of them moved
   std::vector<u64> key;
   key.push_back(b->items.size());
   key.push_back(b->dense_idx.size());
@@ -1340,13 +1349,8 @@ static fk_status launch(fk_batch* b, int use_graph) {
   key.push_back(b->hunts);
   key.push_back(b->cand_cap);
   key.push_back(b->out_cap);
-  key.push_back(b->d_xq.cap);
+  key.push_back(b->moves);
   for (auto& f : b->fam) { key.push_back(f.idx.size()); key.push_back(f.prefix.back()); }
-  key.push_back((u64)(uintptr_t)b->d_items);
-  key.push_back((u64)(uintptr_t)b->d_cand_key.p);
-  key.push_back((u64)(uintptr_t)b->d_zero.p);
-  key.push_back((u64)(uintptr_t)b->h_sorted.p);
-  key.push_back((u64)(uintptr_t)b->d_bcount.p);
   key.push_back(((u64)b->tune.sieve_ctas_per_sm << 32) | b->tune.mark_ctas_per_sm);
   key.push_back(((u64)b->tune.warp_queue << 32) | b->tune.seg_per_task);
   key.push_back(((u64)b->tune.warp_tasks << 32) | b->tune.classify_ctas_per_sm);

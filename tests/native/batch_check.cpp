@@ -1,0 +1,119 @@
+// Host checks of a batch's buffers and graphs (csrc/fk_engine.cu) on the fake
+// CUDA runtime.  Each check prints "<name> ok", or what went wrong.
+#include <cstdio>
+#include <cstring>
+#include <vector>
+
+#include "../../include/fk.h"
+#include "fake_cuda.h"
+
+struct CUstream_st;
+namespace fk {
+struct SieveArgs;
+int launch_sieve(unsigned, unsigned, unsigned, CUstream_st*, const SieveArgs&) {
+  fake_kernel();
+  return 0;
+}
+int launch_mark(unsigned, unsigned, unsigned, unsigned, CUstream_st*,
+                const SieveArgs&) {
+  fake_kernel();
+  return 0;
+}
+int sieve_set_smem_limits() { return 0; }
+int mark_set_smem_limits() { return 0; }
+}  // namespace fk
+
+namespace {
+
+fk_engine* engine(uint32_t kind, uint32_t n, uint32_t q2, uint32_t sieve) {
+  fk_params p;
+  std::memset(&p, 0, sizeof p);
+  p.kind = kind;
+  p.n = n;
+  p.q2 = q2;
+  p.p0 = 6;
+  p.sieve = sieve;
+  fk_engine* e = nullptr;
+  if (fk_engine_create(&p, &e)) std::printf("create: %s\n", fk_last_error());
+  return e;
+}
+
+// One run of `count` intervals of `len`; false when it fails or its result is
+// not the fake's (every output in the last interval, offsets rising by one).
+bool run(fk_batch* b, uint64_t count, int graph, uint64_t len = 1 << 16,
+         uint64_t step = 1 << 20) {
+  std::vector<fk_item> it(count);
+  std::memset(it.data(), 0, count * sizeof(fk_item));
+  for (uint64_t i = 0; i < count; ++i) {
+    it[i].mode = 1;
+    it[i].threshold = 1;
+    it[i].cap = 8;
+    it[i].lo[0] = 1000000007ull + i * step;
+    it[i].hi[0] = it[i].lo[0] + len;
+  }
+  fk_batch_result r;
+  if (fk_batch_run(b, it.data(), count, graph, &r)) return false;
+  if (r.item_start[count] != fake().outputs) return false;
+  for (uint64_t k = 0; k < fake().outputs; ++k)
+    if (r.offset[k] != r.offset[0] + k || r.depth[k] != 7) return false;
+  return true;
+}
+
+struct Batch {
+  fk_engine* e;
+  fk_batch* b = nullptr;
+  explicit Batch(uint32_t q2 = 65536) : e(engine(0, 8, q2, 1)) {
+    fk_batch_create(&e, 1, &b);
+  }
+  ~Batch() {
+    fk_batch_destroy(b);
+    fk_engine_destroy(e);
+  }
+};
+
+// Eager runs between graph runs move buffers the graph holds.
+bool growth() {
+  struct Step { uint64_t count; int graph; uint64_t len; };
+  // the first run sizes every buffer that goes by the expected output
+  const std::vector<std::vector<Step>> lists = {
+      {{684, 0, 1ull << 32}, {690, 0, 0}, {1000, 1, 0}, {1024, 0, 0}, {1000, 1, 0}},
+      {{700, 0, 1ull << 32}, {750, 0, 0}, {1000, 1, 0}, {1030, 0, 0}, {1000, 1, 0}},
+  };
+  bool ok = true;
+  for (const auto& l : lists) {
+    Batch b;
+    for (const Step& s : l) {
+      fake().outputs = 100 + s.count % 7;
+      ok &= run(b.b, s.count, s.graph, s.len ? s.len : 1 << 16);
+    }
+  }
+  // and any order of sizes, forms and results
+  uint64_t x = 88172645463325252ull;
+  for (int seq = 0; seq < 12; ++seq) {
+    Batch b(600);
+    fake().outputs = 1;
+    ok &= run(b.b, 1, 0, 1ull << 34);
+    for (int k = 0; k < 40; ++k) {
+      x ^= x << 13; x ^= x >> 7; x ^= x << 17;
+      fake().outputs = (x >> 20) % 4000;
+      fake().overflows = (x >> 50) % 8 == 0;
+      ok &= run(b.b, 1 + (x >> 40) % (40u << (seq % 6)), (x >> 10) & 1,
+                1 << (16 + (x >> 33) % 8));
+    }
+  }
+  if (fake().dead) std::printf("growth: %llu uses of freed buffers\n",
+                               (unsigned long long)fake().dead);
+  return ok && fake().dead == 0;
+}
+
+}  // namespace
+
+int main(int argc, char** argv) {
+  const struct { const char* name; bool (*check)(); } checks[] = {
+      {"growth", growth},
+  };
+  for (const auto& c : checks)
+    if (argc > 1 && std::strcmp(argv[1], c.name) == 0)
+      std::printf("%s %s\n", c.name, c.check() ? "ok" : "failed");
+  return 0;
+}

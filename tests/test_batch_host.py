@@ -1,0 +1,46 @@
+"""A batch's buffers and captured graphs, on the CPU.
+
+The host code of libfk (csrc/fk_engine.cu, as nvcc compiles it) linked with a
+runtime that runs on plain memory (native/fake_cuda.cpp): copies are made,
+captures recorded and replayed, and every use of a buffer that has been freed
+is counted.
+"""
+
+import pathlib
+import subprocess
+
+import pytest
+
+ROOT = pathlib.Path(__file__).resolve().parents[1]
+NATIVE = ROOT / "tests" / "native"
+CUDA = pathlib.Path("/usr/local/cuda")
+
+
+@pytest.fixture(scope="module")
+def batch_check(tmp_path_factory):
+    import build as fkbuild
+    tmp = tmp_path_factory.mktemp("batch")
+    obj = fkbuild.OBJ / "fk_engine.o"      # the library's own, when current
+    if not obj.exists() or any(s.stat().st_mtime > obj.stat().st_mtime
+                               for s in fkbuild.sources()):
+        obj = tmp / "fk_engine.o"
+        subprocess.run([fkbuild.NVCC, *fkbuild.FLAGS, "-c", "-o", str(obj),
+                        str(fkbuild.CSRC / "fk_engine.cu")], check=True,
+                       capture_output=True)
+    exe = tmp / "batch_check"
+    subprocess.run(["g++", "-O1", "-std=c++17", "-I", str(CUDA / "include"),
+                    "-o", str(exe), str(NATIVE / "batch_check.cpp"),
+                    str(NATIVE / "fake_cuda.cpp"), str(obj)], check=True)
+
+    def check(name):
+        out = subprocess.run([str(exe), name], capture_output=True, text=True,
+                             timeout=300)
+        assert out.returncode == 0 and out.stdout == f"{name} ok\n", \
+            out.stdout + out.stderr
+    return check
+
+
+def test_graphs_hold_no_freed_buffer(batch_check):
+    """A graph is replayed only while every buffer it was captured with is
+    still there: runs of other sizes, eager and not, between two of it."""
+    batch_check("growth")
