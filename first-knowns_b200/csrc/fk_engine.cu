@@ -844,7 +844,11 @@ struct fk_batch {
   DevBuf<u64> d_bbase{&moves}, d_boff{&moves};
   DevBuf<u32> d_rounds;         // per engine: this batch's round cuts
   PinBuf<DevCounters> h_ctr{&moves};
-  PinBuf<u64> h_off{&moves}, h_sorted{&moves};
+  PinBuf<u64> h_off{&moves};
+  // a short result is read back with the counters, into a buffer that never
+  // grows (the copy is part of a captured graph); a longer one once its length
+  // is known
+  PinBuf<u64> h_short{&moves}, h_sorted;
   u64 cand_cap = 0, out_cap = 0;
   // graph
   cudaGraph_t graph = nullptr;
@@ -956,7 +960,7 @@ static void batch_free(fk_batch* b) {
   b->d_nbuckets.release(); b->d_bbase.release(); b->d_boff.release();
   b->d_rounds.release();
   b->h_ctr.release(); b->h_off.release();
-  b->h_sorted.release();
+  b->h_short.release(); b->h_sorted.release();
   if (b->d_engines) cudaFree(b->d_engines);
   for (auto& e : b->ev) if (e) cudaEventDestroy(e);
   for (auto& e : b->fev) if (e) cudaEventDestroy(e);
@@ -1162,7 +1166,7 @@ static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
     if ((st = b->d_boff.ensure(nbk + 1))) return st;
   }
   if ((st = b->h_off.ensure(ni + 2))) return st;
-  if ((st = b->h_sorted.ensure(kSpecOut))) return st;
+  if ((st = b->h_short.ensure(kSpecOut))) return st;
   // the upload buffer: 8-byte words first, then the 4-byte lists
   u64 at = ni * sizeof(DevItem);
   u64 pre[8], idx[8];
@@ -1323,7 +1327,7 @@ static fk_status enqueue(fk_batch* b, bool capturing = false) {
   FK_CUDA(cudaMemcpyAsync(b->h_off.p, b->d_item_off.p, (ni + 1) * sizeof(u64),
                           cudaMemcpyDeviceToHost, s));
   // a short result comes back in the same round trip
-  FK_CUDA(cudaMemcpyAsync(b->h_sorted.p, b->d_sorted.p,
+  FK_CUDA(cudaMemcpyAsync(b->h_short.p, b->d_sorted.p,
                           std::min<u64>(kSpecOut, b->out_cap) * 8,
                           cudaMemcpyDeviceToHost, s));
   b->last_launches = nl;
@@ -1401,9 +1405,11 @@ static fk_status collect(fk_batch* b) {
   const u64 ni = b->items.size();
   const u64 nout = b->h_off.p[ni];
   b->d2h = sizeof(DevCounters) + (ni + 1) * 8 + nout * 8;
-  fk_status st;
+  const u64* sorted = b->h_short.p;
   if (nout > kSpecOut) {
-    if ((st = b->h_sorted.ensure(nout))) return st;
+    const fk_status st = b->h_sorted.ensure(nout);
+    if (st) return st;
+    sorted = b->h_sorted.p;
     FK_CUDA(cudaMemcpyAsync(b->h_sorted.p, b->d_sorted.p, nout * 8,
                             cudaMemcpyDeviceToHost, s));
     FK_CUDA(cudaStreamSynchronize(s));
@@ -1422,7 +1428,7 @@ static fk_status collect(fk_batch* b) {
     const u128 lo = u128_of(b->user[u].lo);
     const u64 base = (u64)(b->sub[i].X0 - lo);  // X0 >= lo - M ... may wrap
     for (u64 k = b->h_off.p[i]; k < b->h_off.p[i + 1]; ++k) {
-      const u64 pk = b->h_sorted.p[k];
+      const u64 pk = sorted[k];
       b->r_off[fill[u]] = base + (pk >> 8);
       b->r_depth[fill[u]] = (uint8_t)(pk & 255);
       ++fill[u];

@@ -106,11 +106,26 @@ bool growth() {
   return ok && fake().dead == 0;
 }
 
+// A batch's graph is captured once, whatever the number of its results, and
+// results are whole on both sides of the length that comes back at once.
+bool once() {
+  Batch b;
+  bool ok = true;
+  for (uint64_t n : {3000u, 4000u, 0u, 1u, 2047u, 2048u, 2049u, 4096u, 2048u}) {
+    fake().outputs = n;
+    ok &= run(b.b, 300, 1) && run(b.b, 300, 0);
+  }
+  if (fake().captures != 1)
+    std::printf("once: %llu captures\n", (unsigned long long)fake().captures);
+  return ok && fake().captures == 1 && fake().dead == 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
   const struct { const char* name; bool (*check)(); } checks[] = {
       {"growth", growth},
+      {"once", once},
   };
   for (const auto& c : checks)
     if (argc > 1 && std::strcmp(argv[1], c.name) == 0)

@@ -44,3 +44,9 @@ def test_graphs_hold_no_freed_buffer(batch_check):
     """A graph is replayed only while every buffer it was captured with is
     still there: runs of other sizes, eager and not, between two of it."""
     batch_check("growth")
+
+
+def test_a_graph_is_captured_once(batch_check):
+    """The result's length changes no address that the graph holds, and
+    results around the length that is read back at once are whole."""
+    batch_check("once")
