@@ -35,9 +35,11 @@ static fk_status set_err(fk_status s, const std::string& m) {
 #define FK_CUDA(call)                                                       \
   do {                                                                      \
     cudaError_t e_ = (call);                                                \
-    if (e_ != cudaSuccess)                                                  \
+    if (e_ != cudaSuccess) {                                                \
+      cudaGetLastError();  /* reported here, not by the next call too */    \
       return set_err(FK_ERR_DEVICE, std::string(#call) + ": " +            \
                                         cudaGetErrorString(e_));            \
+    }                                                                       \
   } while (0)
 
 // ------------------------------------------------------------------ math ---

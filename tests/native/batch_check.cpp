@@ -120,12 +120,22 @@ bool once() {
   return ok && fake().captures == 1 && fake().dead == 0;
 }
 
+// A failed call is reported by the run that made it and by no other.
+bool error_once() {
+  Batch b;
+  fake().outputs = 5;
+  fake_fail_allocation(0);
+  const bool first = run(b.b, 20, 0);
+  return !first && run(b.b, 20, 0) && run(b.b, 20, 1) && fake().dead == 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
   const struct { const char* name; bool (*check)(); } checks[] = {
       {"growth", growth},
       {"once", once},
+      {"error_once", error_once},
   };
   for (const auto& c : checks)
     if (argc > 1 && std::strcmp(argv[1], c.name) == 0)

@@ -50,3 +50,7 @@ def test_a_graph_is_captured_once(batch_check):
     """The result's length changes no address that the graph holds, and
     results around the length that is read back at once are whole."""
     batch_check("once")
+
+
+def test_a_failed_call_is_reported_once(batch_check):
+    batch_check("error_once")
