@@ -998,6 +998,21 @@ fk_status check_interval(const fk_engine* e, const uint64_t lo[2],
 }
 }  // namespace fk
 
+// Room for `need` candidates and outputs.  Until every buffer has it the
+// capacities are zero: a buffer that could not grow is gone, and the next run
+// asks for it again.
+static fk_status grow_outputs(fk_batch* b, u64 need) {
+  b->cand_cap = b->out_cap = 0;
+  fk_status st;
+  if ((st = b->d_cand_key.ensure(need))) return st;
+  if ((st = b->d_cand_item.ensure(need))) return st;
+  if ((st = b->d_out.ensure(need))) return st;
+  if ((st = b->d_sorted.ensure(need))) return st;
+  if ((st = b->d_scratch.ensure(2 * need))) return st;
+  b->cand_cap = b->out_cap = need;
+  return FK_OK;
+}
+
 // Expand user items into device items (launch-sized sub-ranges).
 static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
   b->user.assign(items, items + nitems);
@@ -1138,17 +1153,7 @@ static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
   }
   const u64 need = (u64)std::min<long double>(
       expect * 2 * b->tune.capacity_scale + 4096, (long double)(1ull << 28));
-  if (need > b->cand_cap) {
-    if ((st = b->d_cand_key.ensure(need))) return st;
-    if ((st = b->d_cand_item.ensure(need))) return st;
-    b->cand_cap = need;
-  }
-  if (need > b->out_cap) {
-    if ((st = b->d_out.ensure(need))) return st;
-    if ((st = b->d_sorted.ensure(need))) return st;
-    if ((st = b->d_scratch.ensure(2 * need))) return st;
-    b->out_cap = need;
-  }
+  if (need > b->out_cap && (st = grow_outputs(b, need))) return st;
   const u64 ni = b->items.size();
   // the zeroed buffer, in 8-byte words
   constexpr u64 cw = (sizeof(DevCounters) + 7) / 8;
@@ -1393,15 +1398,10 @@ static fk_status collect(fk_batch* b) {
   if (c.overflow & 3u) {
     const u64 need = std::max<u64>({c.ncand, c.nout, b->cand_cap}) * 2 + 4096;
     fk_status st;
-    if ((st = b->d_cand_key.ensure(need))) return st;
-    if ((st = b->d_cand_item.ensure(need))) return st;
-    if ((st = b->d_out.ensure(need))) return st;
-    if ((st = b->d_sorted.ensure(need))) return st;
-    if ((st = b->d_scratch.ensure(2 * need))) return st;
+    if ((st = grow_outputs(b, need))) return st;
     const u64 nbk = need / kBucketFill + b->items.size() + 2;
     if ((st = b->d_bcount.ensure(2 * nbk))) return st;
     if ((st = b->d_boff.ensure(nbk + 1))) return st;
-    b->cand_cap = b->out_cap = need;
     return set_err(FK_ERR_OVERFLOW, "candidate buffer overflow (grown; rerun)");
   }
   const u64 ni = b->items.size();

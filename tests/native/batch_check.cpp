@@ -129,6 +129,35 @@ bool error_once() {
   return !first && run(b.b, 20, 0) && run(b.b, 20, 1) && fake().dead == 0;
 }
 
+// An allocation that fails while the buffers grow fails that run alone: the
+// next one has buffers for what it does, whatever it was that was missing.
+bool failed_growth() {
+  bool ok = true;
+  for (int graph = 0; graph < 2; ++graph)
+    for (int skip = 0; skip < 40; ++skip) {
+      Batch b(600);
+      fake().outputs = 50;
+      ok &= run(b.b, 20, graph);
+      // every buffer that goes by the items or the expected output grows
+      fake_fail_allocation(skip);
+      const bool grown = run(b.b, 3000, graph, 1ull << 30, 1ull << 33);
+      fake_fail_allocation(-1);
+      // the small run again, larger ones that fit or not, and one that
+      // overflows its buffers
+      fake().overflows = skip % 3 == 0;
+      ok &= run(b.b, 20, graph) && run(b.b, 2000, graph) &&
+            run(b.b, 3000, graph, 1ull << 30, 1ull << 33);
+      if (fake().dead || !ok) {
+        std::printf("failed_growth: graph %d, allocation %d (%s): %llu uses "
+                    "of missing buffers\n", graph, skip,
+                    grown ? "passed" : "failed", (unsigned long long)fake().dead);
+        return false;
+      }
+      if (grown) break;   // no allocation left to fail
+    }
+  return ok;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -136,6 +165,7 @@ int main(int argc, char** argv) {
       {"growth", growth},
       {"once", once},
       {"error_once", error_once},
+      {"failed_growth", failed_growth},
   };
   for (const auto& c : checks)
     if (argc > 1 && std::strcmp(argv[1], c.name) == 0)

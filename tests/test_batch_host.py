@@ -54,3 +54,9 @@ def test_a_graph_is_captured_once(batch_check):
 
 def test_a_failed_call_is_reported_once(batch_check):
     batch_check("error_once")
+
+
+def test_a_failed_allocation_fails_one_run(batch_check):
+    """Whichever buffer cannot grow, that run alone fails: the next has every
+    buffer it uses."""
+    batch_check("failed_growth")
