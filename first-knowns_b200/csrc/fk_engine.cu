@@ -639,7 +639,8 @@ static fk_status build_engine(fk_engine* e) {
     std::sort(lf.begin(), lf.end());
     lf.erase(std::unique(lf.begin(), lf.end()), lf.end());
     if (lf.size() > 127) return set_err(FK_ERR_DOMAIN, "forbidden list too long");
-    if (lists.size() >= (1u << 24)) return set_err(FK_ERR_DOMAIN, "lists too large");
+    // ListFilter's offset counts groups of four in 24 bits
+    if (lists.size() / 4 >= (1u << 24)) return set_err(FK_ERR_DOMAIN, "lists too large");
     if (i < (u32)(kNSMax + kStaged)) {
       boff.push_back((u32)bits.size());
       bits.resize(bits.size() + q / 64 + 1, 0);

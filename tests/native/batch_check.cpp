@@ -158,6 +158,15 @@ bool failed_growth() {
   return ok;
 }
 
+// Dickson lists of more than 2^24 entries, filling included: their offsets
+// count groups of four.
+bool long_lists() {
+  fk_engine* e = engine(1, 3, 86000000, 1);
+  const bool ok = e != nullptr;
+  fk_engine_destroy(e);
+  return ok;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -166,6 +175,7 @@ int main(int argc, char** argv) {
       {"once", once},
       {"error_once", error_once},
       {"failed_growth", failed_growth},
+      {"long_lists", long_lists},
   };
   for (const auto& c : checks)
     if (argc > 1 && std::strcmp(argv[1], c.name) == 0)

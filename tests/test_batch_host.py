@@ -60,3 +60,9 @@ def test_a_failed_allocation_fails_one_run(batch_check):
     """Whichever buffer cannot grow, that run alone fails: the next has every
     buffer it uses."""
     batch_check("failed_growth")
+
+
+def test_dickson_lists_up_to_what_their_offset_holds(batch_check):
+    """n = 3 below 8.6e7: 4.4 million primes' residues, 1.75e7 entries when
+    each list is filled up to a multiple of four."""
+    batch_check("long_lists")
