@@ -1211,6 +1211,11 @@ static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
   return FK_OK;
 }
 
+// Outputs read back with the counters.
+static u64 short_read(const fk_batch* b) {
+  return std::min<u64>(kSpecOut, b->out_cap);
+}
+
 // Enqueue the whole pipeline on the batch stream (graph-capturable: no
 // host synchronisation, every size it needs is already on the device).
 static cudaError_t record(cudaEvent_t ev, cudaStream_t s, bool capturing) {
@@ -1335,8 +1340,7 @@ static fk_status enqueue(fk_batch* b, bool capturing = false) {
   FK_CUDA(cudaMemcpyAsync(b->h_off.p, b->d_item_off.p, (ni + 1) * sizeof(u64),
                           cudaMemcpyDeviceToHost, s));
   // a short result comes back in the same round trip
-  FK_CUDA(cudaMemcpyAsync(b->h_short.p, b->d_sorted.p,
-                          std::min<u64>(kSpecOut, b->out_cap) * 8,
+  FK_CUDA(cudaMemcpyAsync(b->h_short.p, b->d_sorted.p, short_read(b) * 8,
                           cudaMemcpyDeviceToHost, s));
   b->last_launches = nl;
   return FK_OK;
@@ -1407,12 +1411,13 @@ static fk_status collect(fk_batch* b) {
   }
   const u64 ni = b->items.size();
   const u64 nout = b->h_off.p[ni];
-  b->d2h = sizeof(DevCounters) + (ni + 1) * 8 + nout * 8;
+  b->d2h = sizeof(DevCounters) + (ni + 1) * 8 + short_read(b) * 8;
   const u64* sorted = b->h_short.p;
   if (nout > kSpecOut) {
     const fk_status st = b->h_sorted.ensure(nout);
     if (st) return st;
     sorted = b->h_sorted.p;
+    b->d2h += nout * 8;
     FK_CUDA(cudaMemcpyAsync(b->h_sorted.p, b->d_sorted.p, nout * 8,
                             cudaMemcpyDeviceToHost, s));
     FK_CUDA(cudaStreamSynchronize(s));

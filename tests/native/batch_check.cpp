@@ -167,6 +167,27 @@ bool long_lists() {
   return ok;
 }
 
+// fk_stats.d2h_bytes is what a run copies back, the entries that are read
+// before the result's length is known included.
+bool read_back() {
+  Batch b;
+  bool ok = true;
+  for (uint64_t n : {0u, 1u, 2047u, 2048u, 2049u, 4000u}) {
+    fake().outputs = n;
+    const uint64_t before = fake().d2h;
+    ok &= run(b.b, 300, 0);
+    fk_stats st;
+    ok &= fk_batch_stats(b.b, &st) == FK_OK;
+    if (st.d2h_bytes != fake().d2h - before) {
+      std::printf("read_back: %llu outputs: %llu bytes, %llu copied\n",
+                  (unsigned long long)n, (unsigned long long)st.d2h_bytes,
+                  (unsigned long long)(fake().d2h - before));
+      ok = false;
+    }
+  }
+  return ok;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -176,6 +197,7 @@ int main(int argc, char** argv) {
       {"error_once", error_once},
       {"failed_growth", failed_growth},
       {"long_lists", long_lists},
+      {"read_back", read_back},
   };
   for (const auto& c : checks)
     if (argc > 1 && std::strcmp(argv[1], c.name) == 0)

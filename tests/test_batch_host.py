@@ -66,3 +66,7 @@ def test_dickson_lists_up_to_what_their_offset_holds(batch_check):
     """n = 3 below 8.6e7: 4.4 million primes' residues, 1.75e7 entries when
     each list is filled up to a multiple of four."""
     batch_check("long_lists")
+
+
+def test_the_bytes_copied_back_are_counted(batch_check):
+    batch_check("read_back")
