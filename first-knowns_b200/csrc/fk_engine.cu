@@ -1242,8 +1242,10 @@ static fk_status enqueue(fk_batch* b, bool capturing = false) {
                                           b->d_cand_key.p, b->d_cand_item.p,
                                           b->cand_cap, b->d_ctr);
   }
-  SieveArgs rest{};  // what k_rest shares with the rounds launches
   u64 blocks0 = 0;   // the rounds families' items share one counter array
+  int last_rounds = -1;
+  for (int f = 0; f < 8; ++f)
+    if (!b->fam[f].mark && !b->fam[f].idx.empty()) last_rounds = f;
   for (int f = 0; f < 8; ++f) {
     Family& F = b->fam[f];
     b->fam_ran[f] = !F.idx.empty();
@@ -1282,15 +1284,14 @@ static fk_status enqueue(fk_batch* b, bool capturing = false) {
                           b->tune.mark_segment, (u32)grid, s, a));
     else
       FK_CUDA(launch_sieve(P0, b->tune.pattern_primes, (u32)grid, s, a));
+    if (f == last_rounds) {   // what every rounds family left, in its time
+      u32 max_np = 0;
+      for (const fk_engine* e : b->engines)
+        max_np = std::max(max_np, (u32)e->sieve.size());
+      ++nl;
+      k_rest<<<b->nsm * 3, kBlock, 0, s>>>(a, max_np);
+    }
     FK_CUDA(record(b->fev[2 * f + 1], s, capturing));
-    if (!F.mark) rest = a;
-  }
-  if (rest.items) {   // some item went through the rounds
-    u32 max_np = 0;
-    for (const fk_engine* e : b->engines)
-      max_np = std::max(max_np, (u32)e->sieve.size());
-    ++nl;
-    k_rest<<<b->nsm * 3, kBlock, 0, s>>>(rest, max_np);
   }
   FK_CUDA(cudaGetLastError());
   FK_CUDA(record(b->ev[1], s, capturing));

@@ -25,13 +25,14 @@ int mark_set_smem_limits() { return 0; }
 
 namespace {
 
-fk_engine* engine(uint32_t kind, uint32_t n, uint32_t q2, uint32_t sieve) {
+fk_engine* engine(uint32_t kind, uint32_t n, uint32_t q2, uint32_t sieve,
+                  uint32_t p0 = 6) {
   fk_params p;
   std::memset(&p, 0, sizeof p);
   p.kind = kind;
   p.n = n;
   p.q2 = q2;
-  p.p0 = 6;
+  p.p0 = p0;
   p.sieve = sieve;
   fk_engine* e = nullptr;
   if (fk_engine_create(&p, &e)) std::printf("create: %s\n", fk_last_error());
@@ -188,6 +189,44 @@ bool read_back() {
   return ok;
 }
 
+// fk_stats.rounds_ms covers the rounds launches of every wheel family and the
+// launch that finishes what they left, mark_ms the marking launches.  (An
+// event's time here is the number of kernels before it.)
+bool stage_times() {
+  fk_engine* e[3] = {engine(0, 8, 600, 1), engine(0, 8, 600, 1, 7),
+                     engine(0, 8, 600, 2)};
+  fk_batch* b = nullptr;
+  bool ok = fk_batch_create(e, 3, &b) == FK_OK;
+  for (int used = 1; used < 8; ++used)
+    for (int graph = 0; graph < 2; ++graph) {
+      std::vector<fk_item> it;
+      for (uint32_t i = 0; i < 3; ++i) {
+        if (!((used >> i) & 1)) continue;
+        fk_item x;
+        std::memset(&x, 0, sizeof x);
+        x.engine = i;
+        x.lo[0] = 1000000007ull;
+        x.hi[0] = x.lo[0] + (1 << 24);
+        it.push_back(x);
+      }
+      fake().outputs = 3;
+      fk_batch_result r;
+      fk_stats st;
+      ok &= fk_batch_run(b, it.data(), it.size(), graph, &r) == FK_OK &&
+            fk_batch_stats(b, &st) == FK_OK;
+      const int rounds = (used & 1) + (used >> 1 & 1);
+      const float want = rounds ? rounds + 1 : 0, marks = used >> 2;
+      if (st.rounds_ms != want || st.mark_ms != marks) {
+        std::printf("stage_times: engines %d graph %d: rounds %g, not %g; marks "
+                    "%g\n", used, graph, st.rounds_ms, want, st.mark_ms);
+        ok = false;
+      }
+    }
+  fk_batch_destroy(b);
+  for (fk_engine* x : e) fk_engine_destroy(x);
+  return ok;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -198,6 +237,7 @@ int main(int argc, char** argv) {
       {"failed_growth", failed_growth},
       {"long_lists", long_lists},
       {"read_back", read_back},
+      {"stage_times", stage_times},
   };
   for (const auto& c : checks)
     if (argc > 1 && std::strcmp(argv[1], c.name) == 0)

@@ -57,7 +57,8 @@ bool dead(const void* p, size_t n) {
 }
 
 struct Node {
-  std::string kernel;          // empty: a copy or a fill
+  std::string kernel;          // empty: a copy, a fill or an event
+  uint64_t* event = nullptr;
   void* dst = nullptr;
   const void* src = nullptr;
   size_t bytes = 0;
@@ -72,6 +73,10 @@ const std::pair<const char*, const char*> kKernels[] = {
 };
 
 void run(const Node& n) {
+  if (n.event) {
+    *n.event = g.kernels;
+    return;
+  }
   if (n.kernel.empty()) {
     if (dead(n.dst, n.bytes) || (n.src && dead(n.src, n.bytes))) {
       ++g.dead;
@@ -236,8 +241,9 @@ cudaError_t cudaEventCreate(cudaEvent_t* e) {
 }
 cudaError_t cudaEventDestroy(cudaEvent_t e) { delete (Event*)e; return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) {
-  ((Event*)e)->at = g.kernels;
-  return cudaSuccess;
+  Node n;
+  n.event = &((Event*)e)->at;
+  return issue(n);
 }
 cudaError_t cudaEventRecordWithFlags(cudaEvent_t e, cudaStream_t s, unsigned) {
   return cudaEventRecord(e, s);

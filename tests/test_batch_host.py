@@ -70,3 +70,7 @@ def test_dickson_lists_up_to_what_their_offset_holds(batch_check):
 
 def test_the_bytes_copied_back_are_counted(batch_check):
     batch_check("read_back")
+
+
+def test_stage_times_cover_their_launches(batch_check):
+    batch_check("stage_times")
