@@ -865,7 +865,7 @@ struct fk_batch {
   std::vector<uint8_t> r_depth;
   bool pending = false;
   int pending_graph = 0;
-  u64 last_launches = 0;
+  u64 last_launches = 0, graph_launches = 0;   // of the last run, the graph
   u64 h2d = 0, d2h = 0;
   u32 reruns = 0;               // overflow reruns of the last run
   bool hunts = false;           // the run has items to classify
@@ -1248,7 +1248,6 @@ static fk_status enqueue(fk_batch* b, bool capturing = false) {
     if (!b->fam[f].mark && !b->fam[f].idx.empty()) last_rounds = f;
   for (int f = 0; f < 8; ++f) {
     Family& F = b->fam[f];
-    b->fam_ran[f] = !F.idx.empty();
     if (F.idx.empty()) continue;
     FK_CUDA(record(b->fev[2 * f], s, capturing));
     SieveArgs a{};
@@ -1356,6 +1355,7 @@ static fk_status upload_items(fk_batch* b) {
 }
 
 static fk_status launch(fk_batch* b, int use_graph) {
+  for (int f = 0; f < 8; ++f) b->fam_ran[f] = !b->fam[f].idx.empty();
   if (!use_graph) return enqueue(b);
   // what the captured launches hold: counts, capacities, tuning, and the
   // buffers' addresses, by the number of times one of them moved
@@ -1385,7 +1385,9 @@ static fk_status launch(fk_batch* b, int use_graph) {
     b->graph = g;
     FK_CUDA(cudaGraphInstantiate(&b->gexec, g, 0));
     b->graph_key = key;
+    b->graph_launches = b->last_launches;
   }
+  b->last_launches = b->graph_launches;
   FK_CUDA(cudaGraphLaunch(b->gexec, b->stream));
   return FK_OK;
 }

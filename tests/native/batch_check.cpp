@@ -227,6 +227,33 @@ bool stage_times() {
   return ok;
 }
 
+// A replayed graph's statistics are its own, whatever ran in between.
+bool replay_stats() {
+  Batch b(600);
+  fake().outputs = 3;
+  fk_item dense;
+  std::memset(&dense, 0, sizeof dense);
+  dense.mode = 2;
+  dense.lo[0] = 2;
+  dense.hi[0] = 1000;
+  dense.cap = 8;
+  fk_stats first, eager, again;
+  fk_batch_result r;
+  bool ok = run(b.b, 20, 1) && fk_batch_stats(b.b, &first) == FK_OK;
+  ok &= fk_batch_run(b.b, &dense, 1, 0, &r) == FK_OK &&
+        fk_batch_stats(b.b, &eager) == FK_OK;
+  ok &= run(b.b, 20, 1) && fk_batch_stats(b.b, &again) == FK_OK;
+  ok &= first.launches != eager.launches && eager.rounds_ms == 0;
+  if (again.launches != first.launches || again.rounds_ms != first.rounds_ms) {
+    std::printf("replay_stats: %llu launches, not %llu; rounds %g, not %g\n",
+                (unsigned long long)again.launches,
+                (unsigned long long)first.launches, again.rounds_ms,
+                first.rounds_ms);
+    ok = false;
+  }
+  return ok;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -237,6 +264,7 @@ int main(int argc, char** argv) {
       {"failed_growth", failed_growth},
       {"long_lists", long_lists},
       {"read_back", read_back},
+      {"replay_stats", replay_stats},
       {"stage_times", stage_times},
   };
   for (const auto& c : checks)

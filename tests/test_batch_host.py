@@ -74,3 +74,7 @@ def test_the_bytes_copied_back_are_counted(batch_check):
 
 def test_stage_times_cover_their_launches(batch_check):
     batch_check("stage_times")
+
+
+def test_a_replayed_graph_has_its_own_statistics(batch_check):
+    batch_check("replay_stats")
