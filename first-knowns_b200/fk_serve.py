@@ -18,8 +18,8 @@ long: short requests that arrive behind it join the next batch, and the
 device never idles while work is queued.
 
 Admission by footprint: a chunk is charged the device bytes its run needs
--- the base-residue table of its engine (4 bytes per sieve prime) plus
-candidate and output slots for twice the survivors the engine's density
+-- the base-residue table of its engine (4 bytes per sieve prime, and for
+an engine that may mark it 4 more per marked prime's slot) plus candidate and output slots for twice the survivors the engine's density
 predicts (``fk_info.survival``, the product of 1 - f_q/q over the wheel and
 sieve primes) -- and a batch admits chunks while the sum stays under
 ``hbm_budget``.
@@ -48,6 +48,10 @@ from fk_workloads import DICKSON, Interval, line_range
 # device bytes per candidate slot: key + item, output record, ordered copy,
 # ordering scratch
 ENTRY_BYTES = 8 + 4 + 16 + 8 + 16
+# entries of a marked item's base-residue table besides one per sieve prime
+# and one per marked prime: 40 pattern primes, and the slots that fill up the
+# blocks of 32, one block of low primes and up to eleven octaves' last
+MARK_ENTRIES = 40 + 32 + 11 * 31
 
 
 class ServeLoop:
@@ -68,7 +72,10 @@ class ServeLoop:
         e = self._engine(iv)
         lo, hi = line_range(iv, e.W if iv.kind == DICKSON else 1)
         expect = (hi - lo) * e.survival + 64
-        return 4 * e.NP + int(2 * expect) * ENTRY_BYTES + 256
+        table = e.NP
+        if e.use_mark:
+            table += e.marked_primes + MARK_ENTRIES
+        return 4 * table + int(2 * expect) * ENTRY_BYTES + 256
 
     def chunk_units(self, iv):
         """Line units per chunk of this request: at most `chunk`, and at
