@@ -1211,6 +1211,11 @@ static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
   return FK_OK;
 }
 
+// CTAs per SM of the SPRP kernels: as many as fit, or as the tuning asks for.
+static u32 class_ctas(const fk_batch* b) {
+  return std::min(b->tune.classify_ctas_per_sm, kClassCtas);
+}
+
 // Outputs read back with the counters.
 static u64 short_read(const fk_batch* b) {
   return std::min<u64>(kSpecOut, b->out_cap);
@@ -1310,7 +1315,7 @@ static fk_status enqueue(fk_batch* b, bool capturing = false) {
   c.spec_lanes = (u64)b->nsm * kSpecLanes;
   // both run loops over their candidates: more CTAs than fit at once would
   // only start to find nothing left
-  const u32 cgrid = b->nsm * std::min(b->tune.classify_ctas_per_sm, kClassCtas);
+  const u32 cgrid = b->nsm * class_ctas(b);
   k_classify<<<cgrid, kBlock, 0, s>>>(c);
   if (b->hunts) {   // pre-primality streams list nothing
     ++nl;
@@ -1370,7 +1375,7 @@ static fk_status launch(fk_batch* b, int use_graph) {
   for (auto& f : b->fam) { key.push_back(f.idx.size()); key.push_back(f.prefix.back()); }
   key.push_back(((u64)b->tune.sieve_ctas_per_sm << 32) | b->tune.mark_ctas_per_sm);
   key.push_back(((u64)b->tune.warp_queue << 32) | b->tune.seg_per_task);
-  key.push_back(((u64)b->tune.warp_tasks << 32) | b->tune.classify_ctas_per_sm);
+  key.push_back(((u64)b->tune.warp_tasks << 32) | class_ctas(b));
   key.push_back(((u64)b->tune.pattern_primes << 48) |
                 ((u64)b->tune.mark_pattern_primes << 32) | b->tune.mark_segment);
   if (b->gexec == nullptr || key != b->graph_key) {

@@ -13,8 +13,8 @@ compaction round is cut (``round_cut``: lower means fewer, longer rounds),
 and three kernel-variant choices: the marking segment length in bytes
 (``mark_segment``: 16, 32 or 64 KiB of shared byte map) and the pattern
 primes each CTA stages in shared memory, per sieve kernel
-(``pattern_primes``, ``mark_pattern_primes``: 24, 32 or 40), and the
-how many blocks of chains a warp of the rounds kernel claims at once
+(``pattern_primes``, ``mark_pattern_primes``: 24, 32 or 40), and how many
+blocks of chains a warp of the rounds kernel claims at once
 (``warp_tasks``).
 None of them can change a result; they only move time.
 
@@ -39,7 +39,8 @@ SPACE = {
     "warp_queue": [8, 16, 64, 128],
     "sieve_ctas_per_sm": [2, 3],
     "mark_ctas_per_sm": [2, 3],
-    "classify_ctas_per_sm": [4, 8, 16],
+    # two fit an SM at once, and more than fit are not launched
+    "classify_ctas_per_sm": [1],
     "warp_lane_words": [64, 1024, 1 << 30],
     "round_cut": [0.3, 0.7, 0.85],
     "group_lane_words": [16, 64, 1 << 30],

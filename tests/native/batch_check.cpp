@@ -254,6 +254,27 @@ bool replay_stats() {
   return ok;
 }
 
+// Two settings of classify_ctas_per_sm that launch the same grids share a
+// graph; one that does not has its own.
+bool class_grids() {
+  Batch b(600);
+  fake().outputs = 3;
+  bool ok = run(b.b, 20, 1);
+  fk_tuning t;
+  std::memset(&t, 0, sizeof t);
+  for (uint32_t v : {2u, 4u, 16u, 32u}) {
+    t.classify_ctas_per_sm = v;
+    ok &= fk_batch_set_tuning(b.b, &t) == FK_OK && run(b.b, 20, 1);
+  }
+  const uint64_t same = fake().captures;
+  t.classify_ctas_per_sm = 1;
+  ok &= fk_batch_set_tuning(b.b, &t) == FK_OK && run(b.b, 20, 1);
+  if (same != 1 || fake().captures != 2)
+    std::printf("class_grids: %llu and %llu captures\n",
+                (unsigned long long)same, (unsigned long long)fake().captures);
+  return ok && same == 1 && fake().captures == 2;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -265,6 +286,7 @@ int main(int argc, char** argv) {
       {"long_lists", long_lists},
       {"read_back", read_back},
       {"replay_stats", replay_stats},
+      {"class_grids", class_grids},
       {"stage_times", stage_times},
   };
   for (const auto& c : checks)

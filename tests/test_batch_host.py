@@ -7,6 +7,7 @@ is counted.
 """
 
 import pathlib
+import re
 import subprocess
 
 import pytest
@@ -78,3 +79,15 @@ def test_stage_times_cover_their_launches(batch_check):
 
 def test_a_replayed_graph_has_its_own_statistics(batch_check):
     batch_check("replay_stats")
+
+
+def test_the_tuner_tries_no_grid_twice(batch_check):
+    """classify_ctas_per_sm: no value searched launches the default's grid or
+    another's, and values that launch the same grid share a graph."""
+    import fk_tune
+    types = (ROOT / "first-knowns_b200" / "csrc" / "fk_types.h").read_text()
+    most = int(re.search(r"kClassCtas = (\d+)", types).group(1))
+    grids = [min(v, most)
+             for v in fk_tune.SPACE["classify_ctas_per_sm"] + [8]]
+    assert len(set(grids)) == len(grids)
+    batch_check("class_grids")
