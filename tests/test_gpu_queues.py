@@ -46,3 +46,23 @@ def test_dense_rows(kind, span, tuning):
     for queue in (1, 32, 513):
         eng.set_tuning(warp_queue=queue, **tuning)
         assert eng.sieve(lo, lo + span).tolist() == want
+
+
+def test_a_full_rest_list_against_the_marking_sieve():
+    """256 items of five engines whose warps offer the list of shared-out
+    candidates about ten times what it holds: every stream is the marking
+    sieve's, which has no such list."""
+    kinds = [(fk_abi.EULER, 7, 65536), (fk_abi.DICKSON, 5, 1 << 18),
+             (fk_abi.AP, 6, 300), (fk_abi.AP, 5, 1 << 17),
+             (fk_abi.EULER, 3, 65536)]
+    engs = [fk_abi.Engine(k, n, q2=q2, sieve="rounds") for k, n, q2 in kinds]
+    marks = [fk_abi.Engine(k, n, q2=q2, sieve="mark") for k, n, q2 in kinds]
+    specs = []
+    for i in range(256):
+        k = i % len(kinds)
+        lo = 10 ** 12 + i * 10 ** 9
+        span = 3 * 10 ** 5 if k == 1 else 3 * 10 ** 7
+        specs.append((k, fk_abi.MODE_SIEVE, 0, 0, lo, lo + span))
+    rows = fk_abi.Batch(engs).run(specs, graph=False)
+    for (k, _m, _t, _c, lo, hi), (off, _d) in zip(specs, rows):
+        assert np.array_equal(off, marks[k].sieve(lo, hi))
