@@ -149,6 +149,7 @@ struct fk_engine {
   const uint32_t* d_mpair[kNumSeg][2] = {};
   const uint32_t* d_mwoff[kNumSeg][2] = {};
   u32 nslots = 0;
+  std::vector<u32> block_qmin;  // least prime of each block of 32 slots
   Cost cost;                  // cost model with every prime below 2^16 marked
   DevEngine dev{};
   std::vector<void*> allocs;
@@ -318,7 +319,10 @@ static void set_mark_tables(const fk_engine* e, DevEngine& d, u32 ns,
   d.NS = ns;
   d.NPm = npm;
   d.qlim = npm < (u32)e->sieve.size() ? e->sieve[npm] : 65536u;
+  // the blocks without a prime below the limit are a tail of the list: it is
+  // by octave, and the pieces of one octave differ by less than a factor of two
   d.nslots = e->nslots;
+  while (d.nslots > 0 && e->block_qmin[d.nslots / 32 - 1] >= d.qlim) d.nslots -= 32;
   d.slot0 = low ? 0 : 32;          // they fill the first block
   d.mq = e->d_mq[si];
   d.mwork = e->d_mwork[si][low];
@@ -331,6 +335,7 @@ static void set_mark_tables(const fk_engine* e, DevEngine& d, u32 ns,
 // rest by octave and within an octave by residue count.
 struct MarkTables {
   std::vector<u32> sprime, mres, prefix;   // prefix: residues before a prime
+  std::vector<u32> qmin;                   // per block
   std::vector<TestRec> mrec;
   std::vector<u32> mq[kNumSeg];
   std::vector<MarkItem> work[kNumSeg][2];
@@ -381,6 +386,7 @@ static fk_status build_marks(const fk_engine* e, u32 NPm, MarkTables& t) {
               g[p][std::min<size_t>(j, g[p].size() - 1)] << (16 * (j & 1));
       }
       blocks.push_back(b);
+      t.qmin.push_back(b.qmin);
     }
   }
   if (t.sprime.size() > (size_t)kMarkSlots)
@@ -403,7 +409,7 @@ static fk_status build_marks(const fk_engine* e, u32 NPm, MarkTables& t) {
           const bool last = k + 1 == parts;
           const u32 kk = last ? kmin - k * K : K;
           const u32 E = last ? kmax - kmin : 0;
-          pieces.push_back({{MARK_PAIRS, 0, at, k * K | kk << 16 | E << 24},
+          pieces.push_back({{MARK_PAIRS, qmin, at, k * K | kk << 16 | E << 24},
                             60.0 + 2.5 * kk + 7.0 * E});
         }
       };
@@ -670,6 +676,7 @@ static fk_status build_engine(fk_engine* e) {
   if (ms) return ms;
   e->nslots = (u32)marks.sprime.size();
   e->mprefix = marks.prefix;
+  e->block_qmin = marks.qmin;
   e->cost = engine_cost(e, NPm, kNS, kNS, kSeg);
   e->use_mark = e->cost.mark;
   if (p.sieve == 1) e->use_mark = false;

@@ -222,11 +222,14 @@ __device__ __forceinline__ u32 mark_segment(unsigned char* __restrict__ B,
   if (i >= end) return 0;
   const MarkCtx c{off16, e.mq, e.mres, e.qlim, WHOLE ? (u32)SEG : len};
   const u32* mpair = e.mpair;
+  const u32 nblock = e.nslots / 32;
   uint4 next = __ldg(work + i);
   while (i < end) {
     const uint4 w = next;
     if (++i < end) next = __ldg(work + i);   // in flight meanwhile
     const u32 kind = w.x & 0xFFu;
+    // past the marked range
+    if (w.y >= (kind == MARK_PAIRS ? e.qlim : nblock)) continue;
     if (kind == MARK_FIXED) {
       cnt += mark_fixed_any<WHOLE>(B, c, w);
       continue;

@@ -86,7 +86,7 @@ enum MarkKind : uint32_t {
 };
 struct alignas(16) MarkItem {
   uint32_t kind;            // kind | nblk << 8 | f << 16
-  uint32_t block;           // the first
+  uint32_t block;           // the first; pairs: their least prime
   uint32_t res;             // first word of the residue pairs, or of the pairs
   uint32_t hits;            // hit0 | K << 16 | E << 24
 };
@@ -137,7 +137,7 @@ struct DevEngine {
   // the marked primes sit in slots, 32 to a block: a block's primes are of
   // one octave and of (nearly) one residue count, a short list repeating its
   // last residue and a short block its last prime (a mark is idempotent)
-  uint32_t nslots, slot0;         // slot0: the first slot this batch marks
+  uint32_t nslots, slot0;         // the slots this batch marks: [slot0, nslots)
   const TestRec* mrec;            // [nslots] a = 1 / M: the scaled residue of
                                   // v = M u + R is the offset of the period u
                                   // in the prime's hits
