@@ -181,6 +181,9 @@ __device__ __forceinline__ u32 mark_fixed(unsigned char* __restrict__ B,
   return mark_blocks(c, (w.x >> 8) & 0xFFu, w.x >> 16, w.y, w.z,
                      [&](u32 a, u32 q) {
                        u32 cnt = 0;
+                       // a short segment holds few first hits: the
+                       // warp mostly leaves here
+                       if (!WHOLE && a >= c.len) return cnt;
 #pragma unroll
                        for (u32 k = 0; k < K + E; ++k, a += q) {
                          if ((WHOLE && k < K) || a < c.len) {
@@ -235,6 +238,8 @@ __device__ __forceinline__ u32 mark_segment(unsigned char* __restrict__ B,
       continue;
     }
     const u32 hit0 = w.w & 0xFFFFu, K = (w.w >> 16) & 0xFFu, E = w.w >> 24;
+    // its hits all lie past a short segment's end
+    if (!WHOLE && kind == MARK_PAIRS && hit0 * w.y >= len) continue;
     const auto many = [&](u32 h, u32 q) {
       return WHOLE ? mark_many<SEG>(B, h + hit0 * q, q, K, E)
                    : mark_short(B, h + hit0 * q, q, K, E, len);
