@@ -122,6 +122,9 @@ struct Cost {
   double bit = 0;     // marking, per lane-period
   double seg = 0;     // marking, per segment
   double lane = 0;    // marking, per task (one lane's shifts)
+  double pattern = 0; // pattern survivors of the rounds, per lane-period
+  double left = 0;    // survivors of all the primes, per lane-period
+  double tail = 0;    // primes past the marked ones
   bool mark = false;  // the marking sieve is available
 };
 
@@ -234,7 +237,9 @@ static u32 pat_bytes_for(u32 P0) {
 // In SM cycles, as measured on a B200 over 256 mixed intervals and single
 // engines.  The rounds: the pattern loop per lane-period (1.84 cycles a
 // word), 2.2 cycles for a pattern survivor's way through column and queue,
-// 0.32 for each of its prime tests.  The marking sieve: 0.115 cycles a byte
+// 0.32 for each of its prime tests, both 1.6 times that for Dickson's lists
+// (long single intervals; n = 5 to 8 took 1.6 to 2.3 times what the other
+// kinds' figures said).  The marking sieve: 0.115 cycles a byte
 // mark (3.5 wavefronts for 32), per segment 0.25 for each (prime, residue),
 // 0.3 for each prime's offset step and 3500 for the pattern words and the
 // map's zeroing and extraction, per lane (task) 0.46 for each prime's first
@@ -271,10 +276,14 @@ static Cost engine_cost(const fk_engine* e, u32 NPm, u32 ns_sieve, u32 ns,
   const std::vector<u32>& mp = e->mprefix;
   const double items = NPm > ns && !mp.empty()
                            ? (double)mp[NPm - kNSMin] - mp[ns - kNSMin] : 0;
-  c.round = 0.029 + s1r * (2.2 + 0.32 * tests);
+  c.round = 0.029 + s1r * (2.2 + 0.32 * tests) *
+                        (e->kind == KIND_DICKSON ? 1.6 : 1.0);
   c.bit = 0.115 * mark_bit + 1.0 * s1 * tail;
   c.seg = 0.25 * items + 0.3 * npm + 3500.0 * seg / 32768.0;
   c.lane = 0.46 * npm;
+  c.pattern = s1r;
+  c.left = s1 * surv_m;
+  c.tail = (double)NP - std::max(NPm, ns);
   c.mark = NPm > ns;
   return c;
 }
@@ -1021,6 +1030,106 @@ static fk_status grow_outputs(fk_batch* b, u64 need) {
   return FK_OK;
 }
 
+// Lay an item out for one of the two sieves: its tasks, and for the rounds
+// its chains.
+static void lay_out(const fk_batch* b, DevItem& di, bool mark) {
+  const u64 L = b->engines[di.engine]->lanes.size(), U = di.U;
+  di.marked = mark ? 1 : 0;
+  di.Tc = di.lane_threads = di.run = 0;
+  di.nchunk = di.nchunk_u = 0;
+  if (mark) {
+    const u64 seg_task = (u64)b->tune.mark_segment * b->tune.seg_per_task;
+    di.nchunk_u = (U + seg_task - 1) / seg_task;
+    di.ntask = L * di.nchunk_u;
+    return;
+  }
+  const u64 target_chains = (u64)b->nsm * b->tune.chains_per_sm;
+  const u64 words = (U + 63) / 64;
+  u64 tc = (words * L + target_chains - 1) / target_chains;
+  tc = std::min<u64>(std::max<u64>(tc, 1), 256);
+  // long lanes: a group of threads per lane (a warp, or eight threads for
+  // mid-length lanes), its threads on interleaved words, so a group's pattern
+  // loads are consecutive table entries
+  const u32 G = words >= (u64)b->tune.warp_lane_words ? 32u
+                : words >= (u64)b->tune.group_lane_words ? 8u : 1u;
+  di.lane_threads = G;
+  tc = std::min<u64>(tc, (words + G - 1) / G);
+  di.Tc = (u32)tc;
+  di.nchunk = (words + G * tc - 1) / (G * tc);
+  const u64 chains = di.nchunk * L;      // one per group
+  di.ntask = (chains + 32 / G - 1) / (32 / G);
+  // blocks a warp claims at once: as many as leave every warp about 16 claims
+  // (the last ones' imbalance), times warp_tasks / 8
+  const u64 warps = (u64)b->nsm * b->tune.sieve_ctas_per_sm * (kBlock / 32);
+  di.run = (u32)std::min<u64>(
+      std::max<u64>(di.ntask / (warps * 16), 1) * (b->tune.warp_tasks / 8),
+      kMaxRun);
+}
+
+// Which sieve each item takes.  An item's time is its share of the SMs'
+// cycles, all of them busy, and by that the sieves are compared (mark_bias
+// weighs them) -- but no less than its longest task takes:
+// * a warp of the rounds whose block has more candidates than its queue holds
+//   drains it alone, at about 20 times the SM cycles (what is left at the
+//   item's end, up to a full queue, goes to k_rest);
+// * a marking CTA alone takes about five times its cycles, and where primes
+//   past the marked ones are tested, a thread tests its words' survivors one
+//   after the other, some 600 cycles a test.
+// The items beside it in the batch fill that time, so an item goes to marking
+// for it only when they do not, and these figures being rough, only when
+// marking is twice as fast.  By the shares alone short intervals of weak
+// filters went to the rounds: 42,006 j of n = 1 took 0.81 ms in 16 warps,
+// marked 0.11; 4.4e6 p of n = 3 0.86 and 0.17.  Over a thousand single
+// intervals (n 1 to 12, lengths 2^12 to 2^33, primes below 4096 to 2^18) the
+// choice takes 0.4% more than the better sieve of each, the shares alone 2.8%.
+static void choose_sieves(fk_batch* b) {
+  constexpr double kWarpAlone = 20, kCtaAlone = 5, kTailTest = 600;
+  struct Times { double rounds, marking, rounds_alone, marking_alone; };
+  std::vector<Times> t(b->items.size());
+  const double bias = b->tune.mark_bias, seg = b->tune.mark_segment;
+  const double seg_words = seg / (64 * kBlock);
+  double total = 0;
+  for (size_t i = 0; i < b->items.size(); ++i) {
+    DevItem& di = b->items[i];
+    if (di.mode == MODE_DENSE) continue;
+    const fk_engine* e = b->engines[di.engine];
+    const bool ok = b->mark_ok[di.engine], forced = ok && e->force_mark;
+    lay_out(b, di, forced);
+    const Cost& c = b->cost[di.engine];
+    const double U = (double)di.U, L = (double)e->lanes.size();
+    const double tasks = std::ceil(U / (seg * b->tune.seg_per_task));
+    const double segs = std::ceil(U / seg);
+    const double marking = tasks * c.lane + segs * c.seg + U * c.bit;
+    // a thread's longest chain of tests past the marked primes in one task
+    const double word = std::min(U, 64.0) * c.left;   // survivors of a word
+    const double chain = kTailTest * c.tail * std::max(std::min(U / seg, 1.0) * seg_words, 1.0) *
+                         (segs / tasks) * std::max(word, std::min(1.0, 32 * word));
+    Times x;
+    x.rounds = L * U * c.round / b->nsm;
+    x.marking = std::max(L * marking / b->nsm, L * tasks * chain / (3 * b->nsm));
+    const bool mark = forced || (ok && x.marking < bias * x.rounds);
+    total += mark ? x.marking : x.rounds;
+    if (!ok || forced) continue;
+    if (mark) {
+      lay_out(b, di, true);
+      continue;
+    }
+    const double block = L * U / (double)di.ntask;   // lane-periods
+    x.rounds_alone = kWarpAlone * block * c.round *
+                     std::min(1.0, std::max(0.0, (block * c.pattern - 80) / 60));
+    x.marking_alone = kCtaAlone * marking / tasks +
+                      std::max(chain, kTailTest * c.tail * std::min(1.0, L * U * c.left));
+    t[i] = x;
+  }
+  for (size_t i = 0; i < b->items.size(); ++i) {
+    const Times& x = t[i];
+    const double others = total - x.rounds;
+    const double rounds = std::max(x.rounds, x.rounds_alone - others);
+    const double marking = std::max(x.marking, x.marking_alone - others);
+    if (2 * marking < bias * rounds) lay_out(b, b->items[i], true);
+  }
+}
+
 // Expand user items into device items (launch-sized sub-ranges).
 static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
   b->user.assign(items, items + nitems);
@@ -1030,9 +1139,6 @@ static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
   b->dense_idx.clear();
   b->sieve_idx.clear();
   for (auto& f : b->fam) { f.idx.clear(); f.prefix.assign(1, 0); }
-  const u64 target_chains = (u64)b->nsm * b->tune.chains_per_sm;
-  const u64 seg_len = b->tune.mark_segment;
-  const u64 seg_task = seg_len * b->tune.seg_per_task;
   for (u64 ui = 0; ui < nitems; ++ui) {
     const fk_item& it = items[ui];
     if (it.engine >= b->engines.size())
@@ -1067,7 +1173,6 @@ static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
     const u128 X0 = lo / M * M;
     const u128 periods = (hi - X0 + M - 1) / M;
     const u64 umax = item_periods_max(M);
-    const u64 L = e->lanes.size();
     for (u128 s0 = 0; s0 < periods; s0 += umax) {
       const u64 U = (u64)std::min<u128>(umax, periods - s0);
       DevItem di{};
@@ -1082,53 +1187,19 @@ static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
       di.lo_off = (s0 == 0) ? (u64)(lo - X0) : 0;
       const bool last = s0 + U >= periods;
       di.hi_last = last ? (u64)(hi - (base + (u128)(U - 1) * M)) : M;
-      bool mark = false;
-      if (b->mark_ok[it.engine]) {
-        const Cost& c = b->cost[it.engine];
-        const double Ud = (double)U;
-        const double rounds = Ud * c.round;
-        const double tasks = std::ceil(Ud / (double)seg_task);
-        const double segs = std::ceil(Ud / (double)seg_len);
-        const double marking = tasks * c.lane + segs * c.seg + Ud * c.bit;
-        mark = e->force_mark || marking < (double)b->tune.mark_bias * rounds;
-      }
-      di.marked = mark ? 1 : 0;
-      if (mark) {
-        di.nchunk_u = (U + seg_task - 1) / seg_task;
-        di.ntask = L * di.nchunk_u;
-        di.Tc = 0;
-        di.nchunk = 0;
-      } else {
-        const u64 words = (U + 63) / 64;
-        u64 tc = (words * L + target_chains - 1) / target_chains;
-        tc = std::min<u64>(std::max<u64>(tc, 1), 256);
-        di.Tc = (u32)tc;
-        // long lanes: a group of threads per lane (a warp, or eight
-        // threads for mid-length lanes), its threads on interleaved words,
-        // so a group's pattern loads are consecutive table entries
-        const u32 G = words >= (u64)b->tune.warp_lane_words ? 32u
-                      : words >= (u64)b->tune.group_lane_words ? 8u : 1u;
-        di.lane_threads = G;
-        tc = std::min<u64>(tc, (words + G - 1) / G);
-        di.Tc = (u32)tc;
-        di.nchunk = (words + G * tc - 1) / (G * tc);
-        const u64 chains = di.nchunk * L;      // one per group
-        di.ntask = (chains + 32 / G - 1) / (32 / G);
-        // blocks a warp claims at once: as many as leave every warp about
-        // 16 claims (the last ones' imbalance), times warp_tasks / 8
-        const u64 warps = (u64)b->nsm * b->tune.sieve_ctas_per_sm * (kBlock / 32);
-        di.run = (u32)std::min<u64>(
-            std::max<u64>(di.ntask / (warps * 16), 1) * (b->tune.warp_tasks / 8),
-            kMaxRun);
-      }
-      Family& f = b->fam[fam_of(e->P0, mark)];
-      di.task0 = f.prefix.back();
-      f.prefix.push_back(f.prefix.back() + di.ntask);
-      f.idx.push_back((u32)b->items.size());
-      b->sieve_idx.push_back((u32)b->items.size());
       b->items.push_back(di);
       b->sub.push_back({(u32)ui, base});
     }
+  }
+  choose_sieves(b);
+  for (u32 i = 0; i < b->items.size(); ++i) {
+    DevItem& di = b->items[i];
+    if (di.mode == MODE_DENSE) continue;
+    Family& f = b->fam[fam_of(b->engines[di.engine]->P0, di.marked)];
+    di.task0 = f.prefix.back();
+    f.prefix.push_back(f.prefix.back() + di.ntask);
+    f.idx.push_back(i);
+    b->sieve_idx.push_back(i);
   }
   // the rounds kernel's lists by kind of test, then by engine: an SM's warps
   // run the same code (first_item), and CTAs restage fewer tables

@@ -16,6 +16,7 @@ int launch_sieve(unsigned, unsigned, unsigned, CUstream_st*, const SieveArgs&) {
 }
 int launch_mark(unsigned, unsigned, unsigned, unsigned, CUstream_st*,
                 const SieveArgs&) {
+  ++fake().marks;
   fake_kernel();
   return 0;
 }
@@ -275,6 +276,58 @@ bool class_grids() {
   return ok && same == 1 && fake().captures == 2;
 }
 
+// Which sieve an interval takes alone, and beside milliseconds of other work: a
+// few blocks of a weak filter, thousands of tests each, are marked when nothing
+// else fills the time those would take -- but not where most primes lie past
+// the marked ones; strong filters and long intervals go by the SMs' cycles.
+bool lone_items() {
+  struct Case { uint32_t kind, n, q2, p0; uint64_t lo, len; bool alone, among; };
+  const Case cases[] = {
+      {0, 3, 40000, 6, 38956, 4415233, true, false},
+      {0, 2, 65536, 6, 1000000000, 1 << 20, true, false},
+      {1, 1, 4096, 7, 1758209, 42006, true, true},
+      {0, 3, 1 << 18, 6, 1000000000, 1 << 16, false, false},
+      {0, 5, 65536, 6, 300000, 1 << 20, false, false},     // about even
+      {0, 8, 65536, 6, 1000000000, 1000000000, false, false},
+      {1, 12, 65536, 6, 1000000000, 1 << 24, false, false},
+      {0, 3, 65536, 7, 1000000000, 1ull << 36, true, true},
+  };
+  bool ok = true;
+  for (const Case& c : cases) {
+    fk_engine* e[2] = {engine(c.kind, c.n, c.q2, 0, c.p0),
+                       engine(0, 12, 65536, 1, 7)};
+    fk_batch* b = nullptr;
+    ok &= fk_batch_create(e, 2, &b) == FK_OK;
+    fake().outputs = 0;
+    fk_item it[2];
+    std::memset(it, 0, sizeof it);
+    it[0].lo[0] = c.lo;
+    it[0].hi[0] = c.lo + c.len;
+    it[1].engine = 1;                  // milliseconds of rounds
+    it[1].hi[0] = 1ull << 44;
+    fk_batch_result r;
+    const uint64_t m0 = fake().marks;
+    ok &= fk_batch_run(b, it, 1, 0, &r) == FK_OK;
+    const bool marked = fake().marks != m0;
+    if (marked != c.alone) {
+      std::printf("lone_items: kind %u n %u length %llu: marked %d\n", c.kind,
+                  c.n, (unsigned long long)c.len, marked);
+      ok = false;
+    }
+    const uint64_t m1 = fake().marks;
+    ok &= fk_batch_run(b, it, 2, 0, &r) == FK_OK;
+    const bool among = fake().marks != m1;
+    if (among != c.among) {
+      std::printf("lone_items: kind %u n %u length %llu: marked %d in a batch\n",
+                  c.kind, c.n, (unsigned long long)c.len, among);
+      ok = false;
+    }
+    fk_batch_destroy(b);
+    for (fk_engine* x : e) fk_engine_destroy(x);
+  }
+  return ok;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -287,6 +340,7 @@ int main(int argc, char** argv) {
       {"read_back", read_back},
       {"replay_stats", replay_stats},
       {"class_grids", class_grids},
+      {"lone_items", lone_items},
       {"stage_times", stage_times},
   };
   for (const auto& c : checks)

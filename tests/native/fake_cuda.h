@@ -8,6 +8,7 @@ struct Fake {
   uint64_t dead = 0;       // uses of freed or null buffers so far
   uint64_t captures = 0;   // stream captures so far
   uint64_t kernels = 0;    // kernels run so far
+  uint64_t marks = 0;      // marking launches so far
   uint64_t d2h = 0;        // bytes copied back by eager runs so far
 };
 

@@ -91,3 +91,7 @@ def test_the_tuner_tries_no_grid_twice(batch_check):
              for v in fk_tune.SPACE["classify_ctas_per_sm"] + [8]]
     assert len(set(grids)) == len(grids)
     batch_check("class_grids")
+
+
+def test_which_sieve_a_lone_item_takes(batch_check):
+    batch_check("lone_items")
