@@ -814,7 +814,7 @@ struct Family {
   u32 P0;
   bool mark = false;
   std::vector<u32> idx;         // internal item indices
-  std::vector<u64> prefix;      // task prefix, size idx+1
+  std::vector<u64> prefix;      // task prefix, size idx+1 (rounds: blocks)
   u32* d_idx = nullptr;         // in the batch's upload buffer
   u64* d_prefix = nullptr;
 };
@@ -835,8 +835,9 @@ struct fk_batch {
   Family fam[8];
   // device buffers: those a captured graph uses count their moves
   u64 moves = 0;
-  // what a run uploads, in one buffer and one copy: the items, every
-  // family's prefix and item list, the dense and sieve item lists
+  // what a run uploads, in one buffer and one copy: the items, the marking
+  // families' task prefixes, every family's item list, the dense and sieve
+  // item lists
   DevBuf<unsigned char> d_up{&moves};
   PinBuf<unsigned char> h_up;
   u64 up_bytes = 0;
@@ -1196,7 +1197,6 @@ static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
     DevItem& di = b->items[i];
     if (di.mode == MODE_DENSE) continue;
     Family& f = b->fam[fam_of(b->engines[di.engine]->P0, di.marked)];
-    di.task0 = f.prefix.back();
     f.prefix.push_back(f.prefix.back() + di.ntask);
     f.idx.push_back(i);
     b->sieve_idx.push_back(i);
@@ -1256,9 +1256,9 @@ static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
   // the upload buffer: 8-byte words first, then the 4-byte lists
   u64 at = ni * sizeof(DevItem);
   u64 pre[8], idx[8];
-  for (int f = 0; f < 8; ++f) {
+  for (int f = 0; f < 8; ++f) {   // the rounds claim blocks by item instead
     pre[f] = at;
-    at += 8 * b->fam[f].prefix.size();
+    if (b->fam[f].mark) at += 8 * b->fam[f].prefix.size();
   }
   for (int f = 0; f < 8; ++f) {
     idx[f] = at;
@@ -1281,7 +1281,7 @@ static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
     Family& F = b->fam[f];
     F.d_prefix = reinterpret_cast<u64*>(d + pre[f]);
     F.d_idx = reinterpret_cast<u32*>(d + idx[f]);
-    put(pre[f], F.prefix.data(), 8 * F.prefix.size());
+    if (F.mark) put(pre[f], F.prefix.data(), 8 * F.prefix.size());
     put(idx[f], F.idx.data(), 4 * F.idx.size());
   }
   put(dense, b->dense_idx.data(), 4 * b->dense_idx.size());

@@ -266,11 +266,11 @@ __device__ __forceinline__ void shared_setup(u32* rho, const TestRec* prec,
 struct SieveArgs {
   const DevEngine* engines;
   const DevItem* items;
-  const u64* task_prefix;  // [nitems + 1] for this kernel's items
+  const u64* task_prefix;  // marking: [nitems + 1] first task of each item
   const u32* item_index;   // [nitems] global item index of each entry
   u32 nitems;
   u32 pad;
-  u64 ntask;
+  u64 ntask;               // marking: tasks
   const u32* xq;
   u64* cand_key;
   u32* cand_item;

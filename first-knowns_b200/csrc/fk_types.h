@@ -163,7 +163,7 @@ struct DevItem {
                                   // thread t of a group takes words t,
                                   // t + lane_threads, ... of its block
   uint64_t nchunk;                // chains per lane
-  uint64_t task0, ntask;          // first task, task count (rounds: blocks)
+  uint64_t ntask;                 // task count (rounds: blocks)
   uint64_t xq_off;                // this item's base-residue table
                                   // (base_residue, fk_sieve.cuh)
   uint32_t marked;                // 1: the marking kernel sweeps this item
@@ -179,7 +179,6 @@ struct OutRec {
 };
 
 struct DevCounters {
-  unsigned long long task_next;   // persistent task counter
   unsigned long long ncand;       // candidates written
   unsigned long long nout;        // outputs written
   unsigned int overflow;          // bit 0 cand, bit 1 out, bit 2 timeout,
