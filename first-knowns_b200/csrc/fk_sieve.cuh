@@ -201,7 +201,8 @@ __device__ __forceinline__ bool any_kill(const Prime<MODE>* p, const TestCtx& c,
 // base index with no wrap inside it.  (With the wrap taken per thread, a
 // run that crossed the table's end touched banks twice: 2.45 wavefronts a
 // load against 2.)  64 also covers the second word of a step; the variants
-// of more primes keep 32 and step twice, to leave room for three CTAs.
+// of more primes keep 32 and step twice, to leave room: three CTAs fit an SM
+// up to 32 primes (70 to 76 KB each), two at 40 (84 to 92 KB).
 template <int NS>
 constexpr u32 kPad = NS <= 24 ? kPadWide : kPadNarrow;
 
@@ -867,11 +868,13 @@ __device__ __forceinline__ u32 first_item(u32 nitems) {
 // item's blocks from the item's counter until none is left, each at its own
 // pace; then they drain their queues and the CTA joins the next item with
 // work.  The SMs start spread over the list, so short items run side by side
-// and long ones draw every CTA in the end.  (With CTA-wide tasks the
+// and long ones draw every CTA in the end.  The variants of 40 primes, of
+// which two CTAs fit an SM, take the registers of two: 128 mixed intervals of
+// up to 2^33, all in the rounds, 137.8 -> 126.5 ms.  (With CTA-wide tasks the
 // barrier ending each one cost a fifth to a third of the warps' time: a
 // warp in a drain held up the other seven.)
 template <int P0, int NS>
-__global__ void __launch_bounds__(kBlock, 3)
+__global__ void __launch_bounds__(kBlock, NS <= 32 ? 3 : 2)
     k_sieve(const __grid_constant__ SieveArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   SieveSmem& S = sieve_smem_ref();
