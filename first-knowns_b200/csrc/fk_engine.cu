@@ -803,6 +803,7 @@ struct PinBuf {
   }
 };
 
+constexpr u64 kFirstItems = 1024;   // items the per-item buffers hold from the start
 constexpr u64 kSpecOut = 2048;   // outputs read back before their count is known
 
 struct SubItem {
@@ -1236,8 +1237,9 @@ static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
   const u64 ni = b->items.size();
   // the zeroed buffer, in 8-byte words
   constexpr u64 cw = (sizeof(DevCounters) + 7) / 8;
-  b->zero_words = cw + 8 + (ni + 1) + (ni + 2) / 2;
-  if ((st = b->d_zero.ensure(b->zero_words))) return st;
+  const auto zeroed = [](u64 n) { return cw + 8 + (n + 1) + (n + 2) / 2; };
+  b->zero_words = zeroed(ni);
+  if ((st = b->d_zero.ensure(zeroed(std::max(ni, kFirstItems))))) return st;
   b->d_ctr = reinterpret_cast<DevCounters*>(b->d_zero.p);
   b->d_task_ctr = b->d_zero.p + cw;
   b->d_block_ctr = b->d_task_ctr + 8;
@@ -1248,7 +1250,7 @@ static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
   if ((st = b->d_nbuckets.ensure(4))) return st;
   {
     const u64 nbk = b->out_cap / kBucketFill + ni + 2;
-    if ((st = b->d_bcount.ensure(2 * nbk))) return st;
+    if ((st = b->d_bcount.ensure(2 * std::max(nbk, kFirstItems)))) return st;
     if ((st = b->d_boff.ensure(nbk + 1))) return st;
   }
   if ((st = b->h_off.ensure(ni + 2))) return st;
@@ -1266,8 +1268,11 @@ static fk_status expand(fk_batch* b, const fk_item* items, u64 nitems) {
   }
   const u64 dense = at, sieve = dense + 4 * b->dense_idx.size();
   b->up_bytes = sieve + 4 * b->sieve_idx.size();
-  if ((st = b->d_up.ensure(b->up_bytes))) return st;
-  if ((st = b->h_up.ensure(b->up_bytes))) return st;
+  // an item takes its record, a prefix and two list entries, a family one
+  // prefix more
+  constexpr u64 up_first = kFirstItems * (sizeof(DevItem) + 8 + 4 + 4) + 8 * 8;
+  if ((st = b->d_up.ensure(std::max(b->up_bytes, up_first)))) return st;
+  if ((st = b->h_up.ensure(std::max(b->up_bytes, up_first)))) return st;
   unsigned char* const d = b->d_up.p;
   b->d_items = reinterpret_cast<DevItem*>(d);
   b->d_dense = reinterpret_cast<u32*>(d + dense);

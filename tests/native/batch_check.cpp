@@ -328,6 +328,25 @@ bool lone_items() {
   return ok;
 }
 
+// Up to about a thousand items nothing grows but the residue table: growing
+// under load waits for whatever else runs on the device.
+bool steady_items() {
+  Batch b(600);
+  fake().outputs = 10;
+  bool ok = run(b.b, 1, 0, 1ull << 34);
+  for (uint64_t n : {2u, 10u, 40u, 160u, 640u, 700u}) {
+    const uint64_t before = fake().allocations;
+    ok &= run(b.b, n, 0);
+    const uint64_t grown = fake().allocations - before;
+    if (grown > 1) {
+      std::printf("steady_items: %llu items: %llu allocations\n",
+                  (unsigned long long)n, (unsigned long long)grown);
+      ok = false;
+    }
+  }
+  return ok;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -341,6 +360,7 @@ int main(int argc, char** argv) {
       {"replay_stats", replay_stats},
       {"class_grids", class_grids},
       {"lone_items", lone_items},
+      {"steady_items", steady_items},
       {"stage_times", stage_times},
   };
   for (const auto& c : checks)

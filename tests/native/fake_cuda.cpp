@@ -36,6 +36,7 @@ cudaError_t allocate(void** p, size_t n) {
     return fail(cudaErrorMemoryAllocation);
   }
   if (g_fail_at > 0) --g_fail_at;
+  ++g.allocations;
   *p = std::calloc(n ? n : 1, 1);
   g_alloc[(uintptr_t)*p] = {n ? n : 1, true};
   return cudaSuccess;

@@ -6,6 +6,7 @@ struct Fake {
   uint64_t outputs = 0;    // how many outputs the next runs "find"
   uint64_t overflows = 0;  // how many of the next runs overflow first
   uint64_t dead = 0;       // uses of freed or null buffers so far
+  uint64_t allocations = 0;
   uint64_t captures = 0;   // stream captures so far
   uint64_t kernels = 0;    // kernels run so far
   uint64_t marks = 0;      // marking launches so far

@@ -95,3 +95,7 @@ def test_the_tuner_tries_no_grid_twice(batch_check):
 
 def test_which_sieve_a_lone_item_takes(batch_check):
     batch_check("lone_items")
+
+
+def test_item_buffers_do_not_grow_up_to_a_thousand_items(batch_check):
+    batch_check("steady_items")
