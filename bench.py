@@ -705,21 +705,22 @@ def bench_fk(args):
             "measured on this GPU by fk_peak (conflict-free st.shared.u8, "
             "32 lanes)",
             "DRAM bytes do not grow with the marks (tables stay in L2 and "
-            "shared memory): ncu of the long mixed case reads 9.1 MB and "
-            "writes 95 MB (the candidate list) per launch (profiles/), so "
+            "shared memory): ncu of the long mixed case reads 4.8 MB and "
+            "writes 98 MB (the candidate list) per launch (profiles/), so "
             "a figure scaled by marks would be meaningless"),
         "k_sieve": roof(
-            "k_sieve (pattern sieve + compaction rounds)", "imad",
-            9 * st["s2_tests"], rnd_s, imad_peak, "G int-multiply-adds/s",
+            "k_sieve and k_rest (pattern sieve + compaction rounds)", "imad",
+            4 * st["s2_tests"], rnd_s, imad_peak, "G int-multiply-adds/s",
             1e9,
-            "9 IMAD per per-candidate prime test (64-bit Barrett residue: "
-            "8, residue product: 1); the pattern stage's 32 shared loads "
-            "per 64 periods ride alongside",
+            "4 multiplies per per-candidate prime test issued (one-word "
+            "Montgomery residue: two wide, a low and a high product), tests "
+            "of a group past the prime that kills included; the pattern "
+            "stage's 32 shared loads per 64 periods ride alongside",
             "measured on this GPU by fk_peak (32-bit mad.lo/mad.hi "
             "chains, 8 per thread)",
             "DRAM traffic is the lane table read once (8 B per lane) plus "
-            "the candidates written; ncu of the long mixed case: 6.7 MB "
-            "read per launch, of the Euler n = 17 window: 246 MB read for "
+            "the candidates written; ncu of the long mixed case: 6.4 MB "
+            "read per launch, of the Euler n = 17 window: 244 MB read for "
             "a 240 MB lane table (profiles/)"),
     }
     times = {"k_classify": cls_s, "k_mark": mark_s, "k_sieve": rnd_s}

@@ -21,11 +21,12 @@
 // of nearly equal step to a warp, so the lanes share their trip counts.  A
 // whole segment holds floor(SEG / q) hits of every lane at least, and those
 // are stored without a bound's test.  The host cuts the work into pieces and
-// deals them to the eight warps by cost.  What bounds it: instructions (about 25 per 32 residues
-// besides the stores) and the byte stores' bank conflicts (32 random bytes
-// take 3.5 wavefronts).  With one 8-byte work entry per (prime, residue),
-// dealt to threads at 38 instructions for the two marks of a large prime, the
-// marking of 256 mixed intervals took 86.5 ms; now 69.
+// deals them to the eight warps by cost.  What bounds it: instructions (about
+// 25 per 32 residues besides the stores) and the byte stores' bank conflicts
+// (32 random bytes take 3.5 wavefronts).  With one 8-byte work entry per
+// (prime, residue), dealt to threads at 38 instructions for the two marks of a
+// large prime, the marking of 256 mixed intervals took 86.5 ms and this form
+// 69 for the same items; the present choice of sieve leaves it fewer, 26 ms.
 // Each slot's first hit offset lives in shared memory and steps by the
 // tabulated SEG mod q from one segment to the next.
 // This is the reference AP engine's bitmap marking (primorial-ap/ap_gpu.py:
@@ -174,7 +175,7 @@ __device__ __forceinline__ u32 mark_blocks(const MarkCtx& c, u32 nblk, u32 f,
 // without a test, four with one.  (The variants stay few and their residue
 // loop rolled: the kernel's code has to stay in the instruction cache.  With
 // eight residues unrolled the warps waited for instructions, and the marking
-// of 256 mixed intervals took 131 ms instead of 69.)
+// of 256 mixed intervals took 131 ms instead of 69, items as above.)
 template <u32 K, u32 E, bool WHOLE>
 __device__ __forceinline__ u32 mark_fixed(unsigned char* __restrict__ B,
                                           const MarkCtx& c, const uint4& w) {

@@ -32,13 +32,16 @@
 // kill test on the scaled residue.  Final survivors are appended to a
 // global candidate list with warp-aggregated atomics.
 //
-// What bounds it, and what this shape measured (B200, kernel ms): the
-// kernel issues instructions (65-75% of the slots), in the sparse windows
-// the pattern loads' shared-memory wavefronts, two a load.  Against 64-bit
-// Barrett tests with a queue drained at every block's end and a CTA barrier
-// after every eight blocks: 256 mixed intervals 204 -> 77 ms, the Dickson
-// window of 2^38 j 12.7 -> 5.5 with k_rest, the Euler n = 17 windows of 5e14
-// and 2e16 42.2 -> 23.7 and 795 -> 478, the 13# line's quarter 19.3 -> 10.4.
+// What bounds it, and what this shape measured (B200, kernel ms): over
+// mixed intervals instructions (59% of the issue slots, with 2.5 warps
+// waiting for their next one at every issue), in the sparse windows the
+// pattern loads' shared-memory wavefronts (50% of the slots, the L1 pipe
+// full), two a load.  Against 64-bit Barrett tests with a queue drained at
+// every block's end and a CTA barrier after every eight blocks: 256 mixed
+// intervals 204 -> 77 ms for the same items (the present choice of sieve
+// gives the rounds more of them: 110), the Dickson window of 2^38 j 12.7 ->
+// 5.5 with k_rest, the Euler n = 17 windows of 5e14 and 2e16 42.2 -> 23.9 and
+// 795 -> 477, the 13# line's quarter 19.3 -> 10.8 with k_rest.
 #pragma once
 #include "fk_arith.cuh"
 #include "fk_types.h"

@@ -217,7 +217,9 @@ typedef struct fk_stats {
   uint64_t candidates;   /* pre-primality survivors (or dense values)       */
   uint64_t outputs;      /* ordered entries returned                        */
   uint64_t s1_words;     /* 64-candidate words the pattern sieve processed  */
-  uint64_t s2_tests;     /* per-candidate prime tests in the rounds         */
+  uint64_t s2_tests;     /* per-candidate prime tests issued: the rounds'   *
+                          * (a group's tests past the killing prime are     *
+                          * counted) and the marking sieve's past mark_limit*/
   uint64_t imad_alg;     /* algorithmic 32-bit multiply-adds of the SPRP    *
                           * stage: (bits(N)-1)*(4l^2+2l) per strong base,   *
                           * l = ceil(bits(N)/32)                            */
@@ -227,7 +229,8 @@ typedef struct fk_stats {
   uint64_t d2h_bytes;    /* device-to-host bytes the run copied             */
   float sieve_ms, classify_ms, total_ms;
   float mark_ms;         /* device time of the marking-sieve launches       */
-  float rounds_ms;       /* device time of the pattern + rounds launches    */
+  float rounds_ms;       /* device time of the pattern + rounds launches,   *
+                          * k_rest among them                               */
   uint32_t reruns;       /* pipeline reruns after a buffer overflow grew    *
                           * the buffers (the result is the rerun's)         */
 } fk_stats;
